@@ -13,6 +13,7 @@
 
 #include "pxr_sched.cuh"
 #include "pxr_chunk.cuh"
+#include "pxr_small.cuh"
 
 using namespace pxr;
 
@@ -389,6 +390,7 @@ struct pxr_handle {
     uint32_t records_n = 0;
     int xcur = 0, tcur = 0, acur = 0;
     int sweep_tab = 0;
+    uint32_t small_ctas = 0;         // largest cluster k_small_decompose can launch on this device
     cudaGraphExec_t graphs[8] = {};  // device-driven loop, one per parity combination
     cudaGraphConditionalHandle conds[8] = {};
     uint64_t body_launches[8] = {};  // kernels per replay of the loop body
@@ -996,7 +998,96 @@ __global__ void k_loop_begin(RoundCtr* c, uint32_t cap) {
     c->loop_cap = cap;
 }
 
+// CTAs of the small-graph kernel for the loaded graph, or 0 when the general
+// path takes it (the measurements are at kSmallMaxSlots).
+uint32_t small_cluster(const pxr_handle* h) {
+    if (h->sched.mode || h->sched.trace || h->n == 0 || h->slots > kSmallMaxSlots) return 0;
+    const uint32_t need = (h->n + kSmallTile - 1) / kSmallTile;
+    uint32_t ctas = 1;
+    while (ctas < need || (ctas < h->small_ctas && (h->n > ctas * kSmallVerticesPerCta ||
+                                                    h->slots > (uint64_t)ctas * kSmallSlotsPerCta)))
+        ctas <<= 1;
+    return ctas <= h->small_ctas ? ctas : 0u;
+}
+
+template <typename OffT>
+cudaError_t launch_small(pxr_handle* h, uint32_t ctas) {
+    SmallArgs<OffT> a{};
+    a.d = make_dev<OffT>(h);
+    a.d.union_sampled = 0;
+    for (int i = 0; i < 2; ++i) {
+        a.tab[i] = h->tab[i];
+        a.act[i] = h->act[i];
+        a.ids[i] = h->ids[i];
+        a.par[i] = h->par[i];
+        a.xt[i] = h->xt[i];
+        a.keys[i] = h->keys[i];
+        a.vals[i] = h->vals[i];
+    }
+    a.xcur = h->xcur;
+    a.tcur = h->tcur;
+    a.acur = h->acur;
+    a.max_rounds = h->cfg.max_rounds;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = ctas;
+    cfg.blockDim = kSmallThreads;
+    cfg.dynamicSmemBytes = sizeof(SmallShared);
+    cfg.stream = h->stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = ctas;
+    attr[0].val.clusterDim.y = 1;
+    attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, k_small_decompose<OffT>, a);
+}
+
+// Attributes of the small-graph kernel and the largest cluster the current device takes.
+template <typename OffT>
+uint32_t prepare_small() {
+    if (cudaFuncSetAttribute(k_small_decompose<OffT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)sizeof(SmallShared)) != cudaSuccess ||
+        cudaFuncSetAttribute(k_small_decompose<OffT>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) !=
+            cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    for (uint32_t ctas = kSmallMaxCtas; ctas > 0; ctas >>= 1) {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = ctas;
+        cfg.blockDim = kSmallThreads;
+        cfg.dynamicSmemBytes = sizeof(SmallShared);
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = ctas;
+        attr[0].val.clusterDim.y = 1;
+        attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        int clusters = 0;
+        if (cudaOccupancyMaxActiveClusters(&clusters, k_small_decompose<OffT>, &cfg) == cudaSuccess && clusters > 0)
+            return ctas;
+        cudaGetLastError();
+    }
+    return 0;
+}
+
+pxr_status decompose_small(pxr_handle* h, uint32_t ctas) {
+    const uint32_t before = h->h_ctr->rounds;
+    PXR_CUDA(h, h->off64 ? launch_small<uint64_t>(h, ctas) : launch_small<uint32_t>(h, ctas));
+    ++h->launches;
+    const pxr_status st = sync_ctr(h);
+    const uint32_t ran = h->h_ctr->rounds - before;
+    if (ran > 0) h->sweep_tab = h->tcur ^ (int)((ran - 1) & 1u);
+    h->xcur ^= (int)(ran & 1u);
+    h->tcur ^= (int)(ran & 1u);
+    h->acur ^= (int)(ran & 1u);
+    return st;
+}
+
 pxr_status decompose_graph(pxr_handle* h) {
+    if (const uint32_t ctas = small_cluster(h)) return decompose_small(h, ctas);
     const int key = h->xcur | (h->tcur << 1) | (h->acur << 2);
     if (!h->graphs[key]) {
         pxr_status st = build_loop_graph(h, key);
@@ -1582,13 +1673,22 @@ pxr_status pxr_create(const pxr_config* cfg, pxr_handle** out) {
     }
     std::memset(h->h_ctr, 0, sizeof(RoundCtr));
     h->stream = h->own_stream;
+    static std::mutex attrs_mu;
     static bool attrs_set[64] = {};   // function attributes are per device
-    if (h->device < 64 && !attrs_set[h->device]) {
-        radix_sort_prepare<uint64_t>();
-        radix_sort_prepare<uint32_t>();
-        cudaFuncSetAttribute(k_chunk_sort<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_sort_smem());
-        cudaFuncSetAttribute(k_chunk_sort<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)chunk_sort_smem());
-        attrs_set[h->device] = true;
+    static uint32_t small_ctas[64] = {};
+    if (h->device < 64) {
+        std::lock_guard<std::mutex> lk(attrs_mu);
+        if (!attrs_set[h->device]) {
+            radix_sort_prepare<uint64_t>();
+            radix_sort_prepare<uint32_t>();
+            cudaFuncSetAttribute(k_chunk_sort<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)chunk_sort_smem());
+            cudaFuncSetAttribute(k_chunk_sort<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)chunk_sort_smem());
+            small_ctas[h->device] = std::min(prepare_small<uint32_t>(), prepare_small<uint64_t>());
+            attrs_set[h->device] = true;
+        }
+        h->small_ctas = small_ctas[h->device];
     }
     *out = h;
     return PXR_OK;

@@ -310,6 +310,19 @@ __device__ __forceinline__ void walk_block_totals(const Dev<OffT>& d, uint32_t v
     }
 }
 
+// The end of a walk row: x' from the exact sum, x' / degree for the next step's
+// gathers; returns the bits of |x'|.
+template <typename OffT>
+__device__ __forceinline__ uint32_t walk_finish(const Dev<OffT>& d, uint32_t v, int64_t acc, double inv, float* xt_out) {
+    const double sum = __dmul_rn(__ll2double_rn(acc), inv);
+    const double val = __dadd_rn(__dmul_rn(sum, 0.9), __dmul_rn((double)d.x[v], 0.1));
+    const float xv = __double2float_rn(val);
+    d.x[v] = xv;
+    const uint32_t dg = d.ideg[v];
+    xt_out[v] = dg ? __double2float_rn(__ddiv_rn((double)xv, (double)dg)) : 0.0f;
+    return __float_as_uint(fabsf(xv));
+}
+
 template <typename OffT, int W>
 __global__ void PXR_WALK_BOUNDS k_walk(Dev<OffT> d, const uint32_t* ids, const float* xt_in,
                                                  float* xt_out) {
@@ -347,13 +360,7 @@ __global__ void PXR_WALK_BOUNDS k_walk(Dev<OffT> d, const uint32_t* ids, const f
 #pragma unroll
         for (int o = W / 2; o > 0; o >>= 1) acc += __shfl_xor_sync(0xFFFFFFFFu, acc, o, W);
         if (light && gl == 0) {
-            const double sum = __dmul_rn(__ll2double_rn(acc), inv);
-            const double val = __dadd_rn(__dmul_rn(sum, 0.9), __dmul_rn((double)d.x[v], 0.1));
-            const float xv = __double2float_rn(val);
-            d.x[v] = xv;
-            const uint32_t dg = d.ideg[v];
-            xt_out[v] = dg ? __double2float_rn(__ddiv_rn((double)xv, (double)dg)) : 0.0f;
-            const uint32_t b = __float_as_uint(fabsf(xv));
+            const uint32_t b = walk_finish(d, v, acc, inv, xt_out);
             vmax = b > vmax ? b : vmax;
         }
     }
@@ -636,30 +643,33 @@ __device__ __forceinline__ uint32_t uf_find_flat(uint32_t* parent, uint32_t v) {
 // to itself.  Only the owning thread writes parent[v] here; the vertex's
 // accumulators for the component data start from the identity.
 template <typename OffT>
+__device__ __forceinline__ void link_first_vertex(const Dev<OffT>& d, uint32_t k, uint32_t v) {
+    const int32_t lv = d.lab[v];
+    if (!in_split(d, k, lv)) return;
+    const OffT beg = d.off[v], end = d.off[v + 1];
+    uint32_t p = v;
+    for (OffT s = beg; s < end; ++s) {
+        const uint32_t nb = d.cols[s];
+        if (!slot_valid(nb)) continue;  // disabled slots keep their place in the sorted row
+        if (nb >= v) break;                // no smaller neighbour left
+        if (d.lab[nb] == lv) { p = nb; break; }
+    }
+    d.parent[v] = p;
+    d.acc_max[v] = 0u;
+    d.acc_min[v] = 0xFFFFFFFFu;
+    d.acc_sum[v] = 0;
+    d.acc_cnt[v] = 0u;
+}
+
+template <typename OffT>
 __global__ void __launch_bounds__(kBlock) k_link_first(Dev<OffT> d, const uint32_t* ids) {
     pdl_wait();
     if (d.ctr->walk_only) return;   // nothing due: the round only walks
     if (!d.ctr->any_split) return;   // no cluster split: no components to find
     const uint32_t count = d.ctr->n_active;
     const uint32_t k = d.ctr->n_clusters;
-    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x) {
-        const uint32_t v = ids[j];
-        const int32_t lv = d.lab[v];
-        if (!in_split(d, k, lv)) continue;
-        const OffT beg = d.off[v], end = d.off[v + 1];
-        uint32_t p = v;
-        for (OffT s = beg; s < end; ++s) {
-            const uint32_t nb = d.cols[s];
-            if (!slot_valid(nb)) continue;  // disabled slots keep their place in the sorted row
-            if (nb >= v) break;                // no smaller neighbour left
-            if (d.lab[nb] == lv) { p = nb; break; }
-        }
-        d.parent[v] = p;
-        d.acc_max[v] = 0u;
-        d.acc_min[v] = 0xFFFFFFFFu;
-        d.acc_sum[v] = 0;
-        d.acc_cnt[v] = 0u;
-    }
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < count; j += gridDim.x * blockDim.x)
+        link_first_vertex(d, k, ids[j]);
 }
 
 // Flatten the linked forest: every vertex of a split cluster points at its root.
@@ -759,6 +769,23 @@ __device__ __forceinline__ bool union_skip_row(const Dev<OffT>& d, uint32_t k, u
     return hint == rep;
 }
 
+// One light row of the union pass: lane gl of W joins its share of the slots.
+template <typename OffT>
+__device__ __forceinline__ void union_light_row(const Dev<OffT>& d, uint32_t k, uint32_t v, uint32_t gl, uint32_t W) {
+    const int32_t lv = d.lab[v];
+    if (!in_split(d, k, lv)) return;
+    const OffT beg = d.off[v], end = d.off[v + 1];
+    if ((uint64_t)(end - beg) > d.light_max) return;   // union_long_rows
+    uint32_t hint;
+    if (union_skip_row(d, k, v, lv, hint)) return;
+    for (OffT s = beg + gl; s < end; s += W) {
+        const uint32_t nb = d.cols[s];
+        if (!slot_valid(nb) || nb == v) continue;
+        if (!d.union_sampled && nb > v) break;   // each edge once, from its larger end
+        if (d.lab[nb] == lv) uf_join(d.parent, &d.ctr->err, v, nb, hint);
+    }
+}
+
 template <typename OffT, int W>
 __global__ void __launch_bounds__(kBlock) k_union(Dev<OffT> d, const uint32_t* ids) {
     pdl_wait();
@@ -767,21 +794,8 @@ __global__ void __launch_bounds__(kBlock) k_union(Dev<OffT> d, const uint32_t* i
     const uint32_t k = d.ctr->n_clusters;
     const uint32_t gl = threadIdx.x & (W - 1);
     const uint32_t groups = (gridDim.x * blockDim.x) / W;
-    for (uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) / W; j < count; j += groups) {
-        const uint32_t v = ids[j];
-        const int32_t lv = d.lab[v];
-        if (!in_split(d, k, lv)) continue;
-        const OffT beg = d.off[v], end = d.off[v + 1];
-        if ((uint64_t)(end - beg) > d.light_max) continue;   // k_union_long
-        uint32_t hint;
-        if (union_skip_row(d, k, v, lv, hint)) continue;
-        for (OffT s = beg + gl; s < end; s += W) {
-            const uint32_t nb = d.cols[s];
-            if (!slot_valid(nb) || nb == v) continue;
-            if (!d.union_sampled && nb > v) break;   // each edge once, from its larger end
-            if (d.lab[nb] == lv) uf_join(d.parent, &d.ctr->err, v, nb, hint);
-        }
-    }
+    for (uint32_t j = (blockIdx.x * blockDim.x + threadIdx.x) / W; j < count; j += groups)
+        union_light_row(d, k, ids[j], gl, (uint32_t)W);
 }
 
 // root registry: one bit per vertex id
@@ -1217,7 +1231,7 @@ __global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, const uint3
 // Every accumulation is order-independent, so the binning does not change
 // any result.
 
-template <typename T>
+template <int WARPS, typename T>
 __device__ __forceinline__ T block_sum(T v, T* sh) {
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
@@ -1227,7 +1241,7 @@ __device__ __forceinline__ T block_sum(T v, T* sh) {
     __syncthreads();
     T t = 0;
     if (threadIdx.x == 0)
-        for (int w = 0; w < kBlock / 32; ++w) t += sh[w];
+        for (int w = 0; w < WARPS; ++w) t += sh[w];
     return t;  // valid in thread 0
 }
 
@@ -1239,7 +1253,7 @@ __device__ __forceinline__ T group_sum(T v, T* sh) {
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
         return v;
     } else {
-        return block_sum<T>(v, sh);
+        return block_sum<G / 32, T>(v, sh);
     }
 }
 
@@ -1315,18 +1329,15 @@ __device__ __forceinline__ RowHead<OffT> row_head(const Dev<OffT>& d, const uint
     return r;
 }
 
+// A group's share of one long row (G = 32: a warp, else the whole block; sh:
+// shared scratch of G / 32 sums).
 template <typename OffT, int G>
-__global__ void PXR_WALK_BOUNDS k_walk_long(Dev<OffT> d, const float* xt_in,
-                                                                          float* xt_out) {
-    pdl_wait();
-    __shared__ int64_t sh[kBlock / 32];
-    const int e = fixed_exponent(d.ctr->xmax_bits, d.nb_bits);
-    const double scale = pow2(e), inv = pow2(-e);
+__device__ __forceinline__ void walk_long_rows(const Dev<OffT>& d, const float* xt_in, float* xt_out, double scale,
+                                               double inv, int64_t* sh, uint32_t& vmax, unsigned long long& st_v,
+                                               unsigned long long& st_s, unsigned long long& st_g) {
     uint32_t cnt;
     const uint32_t* list = row_list(d, G, &cnt);
     const RowGroups<G> rg;
-    uint32_t vmax = 0;
-    unsigned long long st_v = 0, st_s = 0, st_g = 0;
     // With PXR_WALK_PREFETCH the next row's id, label and bounds are loaded
     // before this row's slots are gathered, so a row's setup loads overlap
     // the previous row's gathers.
@@ -1358,26 +1369,27 @@ __global__ void PXR_WALK_BOUNDS k_walk_long(Dev<OffT> d, const float* xt_in,
         acc = group_sum<G, int64_t>(acc, sh);
         st_g += g;
         if (rg.lane == 0) {
-            const double sum = __dmul_rn(__ll2double_rn(acc), inv);
-            const double val = __dadd_rn(__dmul_rn(sum, 0.9), __dmul_rn((double)d.x[v], 0.1));
-            const float xv = __double2float_rn(val);
-            d.x[v] = xv;
-            const uint32_t dg = d.ideg[v];
-            xt_out[v] = dg ? __double2float_rn(__ddiv_rn((double)xv, (double)dg)) : 0.0f;
-            const uint32_t b = __float_as_uint(fabsf(xv));
+            const uint32_t b = walk_finish(d, v, acc, inv, xt_out);
             vmax = b > vmax ? b : vmax;
             st_v += 1;
             st_s += (unsigned long long)(end - beg);
         }
     }
+}
+
+template <typename OffT, int G>
+__global__ void PXR_WALK_BOUNDS k_walk_long(Dev<OffT> d, const float* xt_in, float* xt_out) {
+    pdl_wait();
+    __shared__ int64_t sh[kBlock / 32];
+    const int e = fixed_exponent(d.ctr->xmax_bits, d.nb_bits);
+    uint32_t vmax = 0;
+    unsigned long long st_v = 0, st_s = 0, st_g = 0;
+    walk_long_rows<OffT, G>(d, xt_in, xt_out, pow2(e), pow2(-e), sh, vmax, st_v, st_s, st_g);
     walk_block_totals(d, vmax, st_v, st_s, st_g);
 }
 
 template <typename OffT, int G>
-__global__ void __launch_bounds__(kBlock) k_nodediff_long(Dev<OffT> d) {
-    pdl_wait();
-    if (d.ctr->walk_only) return;   // nothing due: the round only walks
-    __shared__ int32_t sh[kBlock / 32];
+__device__ __forceinline__ void nodediff_long_rows(const Dev<OffT>& d, int32_t* sh) {
     uint32_t cnt;
     const uint32_t* list = row_list(d, G, &cnt);
     const RowGroups<G> rg;
@@ -1409,10 +1421,15 @@ __global__ void __launch_bounds__(kBlock) k_nodediff_long(Dev<OffT> d) {
 }
 
 template <typename OffT, int G>
-__global__ void __launch_bounds__(kBlock) k_union_long(Dev<OffT> d) {
+__global__ void __launch_bounds__(kBlock) k_nodediff_long(Dev<OffT> d) {
     pdl_wait();
-    if (d.ctr->walk_only || !d.ctr->any_split) return;   // nothing due, or nothing split
-    const uint32_t k = d.ctr->n_clusters;
+    if (d.ctr->walk_only) return;   // nothing due: the round only walks
+    __shared__ int32_t sh[kBlock / 32];
+    nodediff_long_rows<OffT, G>(d, sh);
+}
+
+template <typename OffT, int G>
+__device__ __forceinline__ void union_long_rows(const Dev<OffT>& d, uint32_t k) {
     uint32_t cnt;
     const uint32_t* list = row_list(d, G, &cnt);
     const RowGroups<G> rg;
@@ -1437,10 +1454,16 @@ __global__ void __launch_bounds__(kBlock) k_union_long(Dev<OffT> d) {
 }
 
 template <typename OffT, int G>
-__global__ void __launch_bounds__(kBlock) k_disable_long(Dev<OffT> d, float* xt, ClusterTables nt) {
+__global__ void __launch_bounds__(kBlock) k_union_long(Dev<OffT> d) {
     pdl_wait();
-    if (d.ctr->walk_only) return;   // nothing due: the round only walks
-    __shared__ uint32_t sh[kBlock / 32];
+    if (d.ctr->walk_only || !d.ctr->any_split) return;   // nothing due, or nothing split
+    union_long_rows<OffT, G>(d, d.ctr->n_clusters);
+}
+
+// Returns max |x| over the rows this thread finished.
+template <typename OffT, int G>
+__device__ __forceinline__ uint32_t disable_long_rows(const Dev<OffT>& d, float* xt, const ClusterTables& nt,
+                                                      uint32_t* sh) {
     uint32_t cnt;
     const uint32_t* list = row_list(d, G, &cnt);
     const RowGroups<G> rg;
@@ -1470,6 +1493,15 @@ __global__ void __launch_bounds__(kBlock) k_disable_long(Dev<OffT> d, float* xt,
             atomicAdd(&nt.vol[lv], deg);
         }
     });
+    return vmax;
+}
+
+template <typename OffT, int G>
+__global__ void __launch_bounds__(kBlock) k_disable_long(Dev<OffT> d, float* xt, ClusterTables nt) {
+    pdl_wait();
+    if (d.ctr->walk_only) return;   // nothing due: the round only walks
+    __shared__ uint32_t sh[kBlock / 32];
+    uint32_t vmax = disable_long_rows<OffT, G>(d, xt, nt, sh);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) vmax = max(vmax, __shfl_xor_sync(0xFFFFFFFFu, vmax, o));
     if ((threadIdx.x & 31u) == 0 && vmax) atomicMax(&d.ctr->xmax_bits, vmax);
