@@ -7,8 +7,9 @@
 // sort can be launched with host-side capacities only and captured in a CUDA
 // graph.  Passes whose digit is the same for every key are skipped.
 //
-// Per pass and tile (kSortTile items): each warp ranks its items with
-// __match_any_sync against a warp-private digit histogram in shared memory;
+// Per pass and tile (kSortTile items): each warp ranks its items by the
+// ballots of the digit's eight bits against a warp-private digit histogram in
+// shared memory;
 // thread d then publishes the tile's count of digit d, looks back over the
 // preceding tiles' counts of d (status words stamped with a per-pass epoch,
 // so the status area needs no clearing between sorts), and the tile is
@@ -129,6 +130,13 @@ __device__ __forceinline__ uint64_t wait_sort_status(const uint64_t* word, uint3
     return w;
 }
 
+// 8-bit digit of a key at a bit position that is a multiple of 8.
+__device__ __forceinline__ uint32_t sort_digit(uint32_t k, int shift) { return (k >> shift) & 0xFFu; }
+__device__ __forceinline__ uint32_t sort_digit(uint64_t k, int shift) {
+    const uint32_t w = shift < 32 ? (uint32_t)k : (uint32_t)(k >> 32);
+    return (w >> (shift & 31)) & 0xFFu;
+}
+
 #ifndef PXR_SORT_MIN_BLOCKS
 #define PXR_SORT_MIN_BLOCKS 2
 #endif
@@ -144,7 +152,6 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
     K* skeys = reinterpret_cast<K*>(smem_raw);
     uint32_t* svals = reinterpret_cast<uint32_t*>(skeys + kSortTile);
     uint32_t (*whist)[kRadix] = reinterpret_cast<uint32_t (*)[kRadix]>(svals + kSortTile);
-    __shared__ uint32_t tpre[kRadix];
     __shared__ uint32_t gbase[kRadix];
     __shared__ uint64_t warp_tot[kSortThreads / 32];
     __shared__ uint32_t s_tile;
@@ -152,10 +159,11 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
     const uint32_t info = s.pass_info[pass];
     if (!(info & 1u)) return;
     const int in = (info >> 1) & 1;
-    const K* kin = b.keys[in];
-    K* kout = b.keys[in ^ 1];
-    const uint32_t* vin = b.vals[in];
-    uint32_t* vout = b.vals[in ^ 1];
+    // selects, not indexing: a parameter array indexed at run time is copied to local memory
+    const K* kin = in ? b.keys[1] : b.keys[0];
+    K* kout = in ? b.keys[0] : b.keys[1];
+    const uint32_t* vin = in ? b.vals[1] : b.vals[0];
+    uint32_t* vout = in ? b.vals[0] : b.vals[1];
     const bool has_vals = vin != nullptr;
     const uint32_t count = *b.count;
     const uint32_t num_tiles = (count + kSortTile - 1) / kSortTile;
@@ -170,34 +178,63 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
 
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t base = tile * kSortTile + warp * (32 * kSortItems);
+    const uint32_t tile_items = min((uint32_t)kSortTile, count - tile * kSortTile);
+    const bool full = tile_items == (uint32_t)kSortTile;   // all but the last tile skip the bounds tests
     K key[kSortItems];
     uint32_t val[kSortItems];
-    uint32_t rank[kSortItems];
+    if (full) {
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const uint32_t idx = base + k * 32 + lane;
-        const bool valid = idx < count;
-        key[k] = valid ? kin[idx] : (K)0;
-        val[k] = (valid && has_vals) ? vin[idx] : 0u;
-    }
-    const uint32_t lt = lanemask_lt();
+        for (int k = 0; k < kSortItems; ++k) key[k] = kin[base + k * 32 + lane];
 #pragma unroll
-    for (int k = 0; k < kSortItems; ++k) {
-        const uint32_t idx = base + k * 32 + lane;
-        const bool valid = idx < count;
-        const uint32_t d = valid ? ((uint32_t)(key[k] >> shift) & 0xFFu) : 0x100u;
-        const uint32_t peers = __match_any_sync(0xFFFFFFFFu, d);
-        // the lowest lane of each digit reads and advances the warp's count,
-        // the others take the old count from it
-        const uint32_t leader = (uint32_t)__ffs(peers) - 1u;
-        uint32_t before = 0;
-        if (valid && lane == leader) {
-            before = whist[warp][d];
-            whist[warp][d] = before + __popc(peers);
+        for (int k = 0; k < kSortItems; ++k) val[k] = has_vals ? vin[base + k * 32 + lane] : 0u;
+    } else {
+#pragma unroll
+        for (int k = 0; k < kSortItems; ++k) {
+            const uint32_t idx = base + k * 32 + lane;
+            key[k] = idx < count ? kin[idx] : (K)0;
+            val[k] = (idx < count && has_vals) ? vin[idx] : 0u;
         }
-        before = __shfl_sync(0xFFFFFFFFu, before, leader);
-        rank[k] = before + __popc(peers & lt);
+    }
+    // Lanes of the same digit, for every item at once: the ballots of
+    // different items are independent, where one __match_any_sync per item,
+    // each ahead of its shared-memory count, was a serial chain.  What bounds a
+    // pass is latency (ranking about 6,000 of a tile's 27,000 cycles, the
+    // look-back 7,500, the scatter 7,500), not bandwidth.  Whole sorts under
+    // plans 0 / 1 / 2, before and after: 16.7 M pairs, four digits 958 / 892 /
+    // 949 -> 830 / 806 / 862 us; 4.2 M 296 / 282 / 282 -> 257 / 255 / 259; 67 M
+    // keys without values, six digits 4.86 / 4.49 / 5.05 -> 4.33 / 4.18 / 4.59 ms.
+    // (Measured and not taken: looking back 4 or 8 tiles at once, a warp of its
+    // own for the look-back, and counting in a kernel of its own instead of the
+    // look-back: slower below 16 M items.)
+    const uint32_t lt = lanemask_lt();
+    uint32_t rank[kSortItems];   // the item's peers, then its place in the warp's digit run
+#pragma unroll
+    for (int k = 0; k < kSortItems; ++k) {
+        const uint32_t d = sort_digit(key[k], shift);
+        uint32_t peers = 0xFFFFFFFFu;
+        if (!full) {
+            const bool valid = base + k * 32 + lane < count;
+            const uint32_t in_range = __ballot_sync(0xFFFFFFFFu, valid);
+            peers = valid ? in_range : ~in_range;
+        }
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const uint32_t set = __ballot_sync(0xFFFFFFFFu, (d >> q) & 1u);
+            peers &= (d >> q) & 1u ? set : ~set;
+        }
+        rank[k] = peers;
+    }
+#pragma unroll
+    for (int k = 0; k < kSortItems; ++k) {
+        const bool valid = full || base + k * 32 + lane < count;
+        const uint32_t d = sort_digit(key[k], shift);
+        const uint32_t peers = rank[k];
+        // every lane reads its digit's count (peers read one word), the first peer advances it
+        const uint32_t before = valid ? whist[warp][d] : 0u;
         __syncwarp();
+        if (valid && (peers & lt) == 0u) whist[warp][d] = before + __popc(peers);
+        __syncwarp();
+        rank[k] = before + __popc(peers & lt);
     }
     __syncthreads();
 
@@ -220,30 +257,32 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
         if (((w >> 32) & 3u) == 2u) break;
     }
     st_relaxed64(st, sort_status_word(epoch, 2u, excl + tile_cnt));
-    gbase[d] = s.bases[pass * kRadix + d] + excl;
     uint64_t total;
     const uint64_t incl = block_inclusive<Add64>((uint64_t)tile_cnt, warp_tot, &total);
-    tpre[d] = (uint32_t)incl - tile_cnt;
+    const uint32_t in_tile = (uint32_t)incl - tile_cnt;   // the digit's first place in the tile
+    gbase[d] = s.bases[pass * kRadix + d] + excl - in_tile;
+#pragma unroll
+    for (int w = 0; w < kSortThreads / 32; ++w) whist[w][d] += in_tile;
     __syncthreads();
 
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
-        const uint32_t idx = base + k * 32 + lane;
-        if (idx < count) {
-            const uint32_t dg = (uint32_t)(key[k] >> shift) & 0xFFu;
-            const uint32_t pos = tpre[dg] + whist[warp][dg] + rank[k];
+        if (full || base + k * 32 + lane < count) {
+            const uint32_t pos = whist[warp][sort_digit(key[k], shift)] + rank[k];
             skeys[pos] = key[k];
             svals[pos] = val[k];
         }
     }
     __syncthreads();
-    const uint32_t tile_items = min((uint32_t)kSortTile, count - tile * kSortTile);
-    for (uint32_t j = threadIdx.x; j < tile_items; j += kSortThreads) {
-        const K kk = skeys[j];
-        const uint32_t dg = (uint32_t)(kk >> shift) & 0xFFu;
-        const uint32_t out = gbase[dg] + (j - tpre[dg]);
-        kout[out] = kk;
-        if (has_vals) vout[out] = svals[j];
+#pragma unroll
+    for (int q = 0; q < kSortItems; ++q) {
+        const uint32_t j = threadIdx.x + q * kSortThreads;
+        if (full || j < tile_items) {
+            const K kk = skeys[j];
+            const uint32_t out = gbase[sort_digit(kk, shift)] + j;
+            kout[out] = kk;
+            if (has_vals) vout[out] = svals[j];
+        }
     }
 }
 
