@@ -2,14 +2,15 @@
 // on the host (readDynGraph + DynamicGraph::finalize, lib/utils/graph_io.h:49-84,
 // lib/core/graph.h:147-184: self-loops dropped, both directions of every edge,
 // duplicates merged, rows sorted by neighbour id).  Here the same CSR comes from
-// two 64-bit radix sorts with this library's onesweep sort:
+// one radix sort with this library's onesweep sort:
 //
-//   1. pack every non-loop edge as (min << 32 | max) (compaction by atomic
-//      counter: the order is irrelevant, a sort follows);
-//   2. sort, keep the first of each run of equal keys, emit both directions
-//      (src << 32 | dst);
-//   3. sort again: the low words are the columns, row starts come from a
-//      binary search for each vertex.
+//   1. both directions of every non-loop edge as src << bits | dst, bits the
+//      length of an id (compacted a block at a time: the order is irrelevant,
+//      a sort follows);
+//   2. sort (the digits of 2 bits bits);
+//   3. keep the first of each run of equal keys: its low bits are the next
+//      column, and the last column of each row marks the row's end; a running
+//      maximum over the vertices then fills the ends of empty rows.
 //
 // Also an R-MAT edge sampler with the counter-based hash of the Python
 // generator (parex_b200/graphs.py: rmat), so both produce the same graph.
@@ -54,30 +55,174 @@ __global__ void k_rmat(uint64_t samples, uint32_t scale, uint32_t ta, uint32_t t
     }
 }
 
-__global__ void k_pack_edges(const uint32_t* u, const uint32_t* v, uint64_t n_edges, uint32_t n, uint64_t* keys,
-                             uint32_t* count, uint32_t* bad) {
-    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_edges;
-         i += (uint64_t)gridDim.x * blockDim.x) {
-        const uint32_t a = u[i], b = v[i];
-        if (a >= n || b >= n) { atomicOr(bad, 1u); continue; }
-        if (a == b) continue;
-        const uint32_t lo = a < b ? a : b, hi = a < b ? b : a;
-        keys[atomicAdd(count, 1u)] = ((uint64_t)lo << 32) | hi;
+// Both directions of every non-loop edge as src << bits | dst.  A block
+// places its keys with one addition to the counter (one per warp, the
+// compiler's own aggregation, queued 10^5 additions on that word: 0.37 ms of
+// the 4.7 ms build of R-MAT 20).
+constexpr uint32_t kPackItems = 8;
+
+__global__ void __launch_bounds__(kBuildBlock) k_pack_both(const uint32_t* u, const uint32_t* v, uint64_t n_edges,
+                                                           uint32_t n, uint32_t bits, uint64_t* keys, uint32_t* count,
+                                                           uint32_t* bad) {
+    __shared__ uint64_t warp_tot[kBuildBlock / 32];
+    __shared__ uint32_t s_base;
+    constexpr uint64_t kTile = (uint64_t)kBuildBlock * kPackItems;
+    for (uint64_t t0 = blockIdx.x * kTile; t0 < n_edges; t0 += gridDim.x * kTile) {
+        uint32_t a[kPackItems], b[kPackItems], cnt = 0;
+#pragma unroll
+        for (uint32_t q = 0; q < kPackItems; ++q) {
+            const uint64_t i = t0 + q * kBuildBlock + threadIdx.x;
+            a[q] = i < n_edges ? u[i] : 0u;
+            b[q] = i < n_edges ? v[i] : 0u;
+        }
+#pragma unroll
+        for (uint32_t q = 0; q < kPackItems; ++q) {
+            if (a[q] >= n || b[q] >= n) {   // past the list both are 0: skipped as a loop below (n == 0 has no edges)
+                if (t0 + q * kBuildBlock + threadIdx.x < n_edges) atomicOr(bad, 1u);
+                a[q] = b[q] = 0u;
+            }
+            cnt += a[q] != b[q] ? 1u : 0u;
+        }
+        uint64_t total;
+        const uint64_t incl = block_inclusive<Add64>((uint64_t)cnt, warp_tot, &total);
+        if (threadIdx.x == 0) s_base = atomicAdd(count, 2u * (uint32_t)total);
+        __syncthreads();
+        uint32_t p = s_base + 2u * (uint32_t)(incl - cnt);
+        __syncthreads();
+#pragma unroll
+        for (uint32_t q = 0; q < kPackItems; ++q)
+            if (a[q] != b[q]) {
+                keys[p] = ((uint64_t)a[q] << bits) | b[q];
+                keys[p + 1] = ((uint64_t)b[q] << bits) | a[q];
+                p += 2;
+            }
     }
 }
 
-// first of each run of equal sorted keys -> both directions
-__global__ void k_unique_both(const uint64_t* sorted0, const uint64_t* sorted1, const uint32_t* sel,
-                              const uint32_t* count, uint64_t* out, uint32_t* out_count) {
+// First of each run of equal sorted keys, in order (decoupled look-back over
+// tiles): its column, and at the last column of a row the row's end.
+constexpr int kUniqueItems = 8;
+constexpr uint32_t kUniqueTile = kBuildBlock * kUniqueItems;
+
+__global__ void __launch_bounds__(kBuildBlock) k_unique_cols(const uint64_t* sorted0, const uint64_t* sorted1,
+                                                             const uint32_t* sel, const uint32_t* count,
+                                                             uint32_t bits, uint32_t* cols, uint32_t* row_end,
+                                                             uint32_t* tile_ctr, LookbackState lb,
+                                                             uint32_t* kept, uint32_t* err) {
+    __shared__ uint64_t warp_tot[kBuildBlock / 32];
+    __shared__ uint64_t s_excl;
+    __shared__ uint32_t s_tile;
     const uint64_t* k = *sel ? sorted1 : sorted0;
     const uint32_t n = *count;
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint64_t key = k[i];
-        if (i > 0 && k[i - 1] == key) continue;
-        const uint32_t lo = (uint32_t)(key >> 32), hi = (uint32_t)key;
-        const uint32_t p = atomicAdd(out_count, 2u);
-        out[p] = key;
-        out[p + 1] = ((uint64_t)hi << 32) | lo;
+    const uint32_t ntiles = (uint32_t)(((uint64_t)n + kUniqueTile - 1) / kUniqueTile);
+    if (threadIdx.x == 0) s_tile = atomicAdd(tile_ctr, 1u);
+    __syncthreads();
+    const uint32_t tile = s_tile;
+    if (tile >= ntiles) return;
+    // a warp owns 32 x kUniqueItems consecutive keys and reads 32 neighbours at a time
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    const uint64_t w0 = (uint64_t)tile * kUniqueTile + warp * (32u * kUniqueItems);
+    uint64_t key[kUniqueItems];
+    uint32_t first = 0, cnt_before[kUniqueItems], cnt = 0;
+#pragma unroll
+    for (int q = 0; q < kUniqueItems; ++q) {
+        const uint64_t i = w0 + q * 32 + lane;
+        key[q] = i < n ? k[i] : ~0ull;
+    }
+    uint64_t last = w0 > 0 && w0 - 1 < n ? k[w0 - 1] : ~0ull;   // ~0 is no key: an id is below 2^31 - 1
+    uint32_t heads[kUniqueItems];
+#pragma unroll
+    for (int q = 0; q < kUniqueItems; ++q) {
+        uint64_t prev = __shfl_up_sync(0xFFFFFFFFu, key[q], 1);
+        if (lane == 0) prev = last;
+        last = __shfl_sync(0xFFFFFFFFu, key[q], 31);
+        heads[q] = __ballot_sync(0xFFFFFFFFu, key[q] != prev && w0 + q * 32 + lane < n);
+        if ((heads[q] >> lane) & 1u) first |= 1u << q;
+        cnt_before[q] = cnt;
+        cnt += __popc(heads[q]);
+    }
+    // every lane holds the warp's count: lane 31 carries it into the block scan
+    uint64_t total;
+    const uint64_t incl = block_inclusive<Add64>(lane == 31u ? (uint64_t)cnt : 0ull, warp_tot, &total);
+    const uint32_t warp_first = (uint32_t)__shfl_sync(0xFFFFFFFFu, incl, 31) - cnt;
+    if (threadIdx.x < 32) {
+        const uint64_t ex = lookback_tile<Add64>(lb, tile, 1u, total, err);
+        if (threadIdx.x == 0) {
+            s_excl = ex;
+            if (tile == ntiles - 1) *kept = (uint32_t)(ex + total);
+        }
+    }
+    __syncthreads();
+    const uint32_t base = (uint32_t)s_excl + warp_first, lt = lanemask_lt();
+    const uint64_t id_mask = (1ull << bits) - 1ull;
+#pragma unroll
+    for (int q = 0; q < kUniqueItems; ++q) {
+        const uint64_t i = w0 + q * 32 + lane;
+        if (i >= n) continue;
+        // columns up to and including this key's run: a duplicate shares its first's place
+        const uint32_t upto = base + cnt_before[q] + __popc(heads[q] & (lt | (1u << lane)));
+        if ((first >> q) & 1u) cols[upto - 1u] = (uint32_t)(key[q] & id_mask);
+        const uint32_t src = (uint32_t)(key[q] >> bits);
+        if (i + 1 == n || (uint32_t)(k[i + 1] >> bits) != src) row_end[src] = upto;
+    }
+}
+
+// Row ends of empty rows: a running maximum over offsets[1..n], in chunks
+// (maxima of the chunks first, then every chunk scans on from the maximum of
+// those before it).
+constexpr uint32_t kFillChunks = 148 * 4;
+
+__device__ __forceinline__ void fill_range(uint32_t n, uint32_t c, uint64_t* lo, uint64_t* hi) {
+    const uint64_t per = ((uint64_t)n + kFillChunks - 1) / kFillChunks;
+    *lo = min((uint64_t)n, c * per);
+    *hi = min((uint64_t)n, *lo + per);
+}
+
+__global__ void __launch_bounds__(kBuildBlock) k_fill_max(const uint32_t* row_end, uint32_t n, uint32_t* chunk_max) {
+    __shared__ uint32_t s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    uint64_t lo, hi;
+    fill_range(n, blockIdx.x, &lo, &hi);
+    uint32_t m = 0;
+    for (uint64_t i = lo + threadIdx.x; i < hi; i += kBuildBlock) m = max(m, row_end[i]);
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    if ((threadIdx.x & 31u) == 0) atomicMax(&s_max, m);
+    __syncthreads();
+    if (threadIdx.x == 0) chunk_max[blockIdx.x] = s_max;
+}
+
+__global__ void __launch_bounds__(kBuildBlock) k_fill_rows(uint32_t* row_end, uint32_t n, const uint32_t* chunk_max) {
+    __shared__ uint32_t s_warp[kBuildBlock / 32];
+    __shared__ uint32_t s_max;
+    if (threadIdx.x == 0) s_max = 0;
+    __syncthreads();
+    uint32_t m = 0;
+    for (uint32_t c = threadIdx.x; c < blockIdx.x; c += kBuildBlock) m = max(m, chunk_max[c]);
+    m = __reduce_max_sync(0xFFFFFFFFu, m);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    if (lane == 0) atomicMax(&s_max, m);
+    __syncthreads();
+    uint32_t run = s_max;
+    uint64_t lo, hi;
+    fill_range(n, blockIdx.x, &lo, &hi);
+    for (uint64_t i0 = lo; i0 < hi; i0 += kBuildBlock) {
+        const uint64_t i = i0 + threadIdx.x;
+        uint32_t x = i < hi ? row_end[i] : 0u;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xFFFFFFFFu, x, o);
+            if (lane >= (uint32_t)o) x = max(x, y);
+        }
+        if (lane == 31u) s_warp[warp] = x;
+        __syncthreads();
+        uint32_t before = run;
+        for (uint32_t w = 0; w < kBuildBlock / 32; ++w) {
+            if (w < warp) before = max(before, s_warp[w]);
+            run = max(run, s_warp[w]);
+        }
+        if (i < hi) row_end[i] = max(x, before);
+        __syncthreads();
     }
 }
 
@@ -513,12 +658,13 @@ pxr_status pxr_build_csr(uint32_t n, uint64_t n_edges, const uint32_t* u, const 
     uint32_t *count0 = words, *count1 = words + 1, *end_bit = words + 2, *err = words + 3, *bad = words + 4;
     // sort state starts zeroed (histograms, epochs, status words)
     if (cudaMemsetAsync(base + L.hist, 0, L.total - L.hist, s) != cudaSuccess) return PXR_CUDA_ERROR;
-    uint32_t bits = 0;
+    if (cudaMemsetAsync(offsets, 0, ((size_t)n + 1) * 4, s) != cudaSuccess) return PXR_CUDA_ERROR;
+    uint32_t bits = 1;
     while (bits < 32 && (1ull << bits) < n) ++bits;
-    k_set_u32<<<1, 1, 0, s>>>(end_bit, 32u + bits);
-    const uint32_t grid = (uint32_t)std::min<uint64_t>((std::max<uint64_t>(n_edges, (uint64_t)n + 1) + kBuildBlock - 1) /
-                                                           kBuildBlock, 148u * 32u);
-    if (n_edges) k_pack_edges<<<grid, kBuildBlock, 0, s>>>(u, v, n_edges, n, k0, count0, bad);
+    k_set_u32<<<1, 1, 0, s>>>(end_bit, 2u * bits);
+    const uint32_t grid = (uint32_t)std::min<uint64_t>((n_edges + kBuildBlock * kPackItems - 1) /
+                                                           (kBuildBlock * kPackItems), 148u * 8u);
+    if (n_edges) k_pack_both<<<grid, kBuildBlock, 0, s>>>(u, v, n_edges, n, bits, k0, count0, bad);
     SortState st{};
     st.hist = reinterpret_cast<uint32_t*>(base + L.hist);
     st.bases = reinterpret_cast<uint32_t*>(base + L.bases);
@@ -533,31 +679,30 @@ pxr_status pxr_build_csr(uint32_t n, uint64_t n_edges, const uint32_t* u, const 
     b.keys[1] = k1;
     b.count = count0;
     b.end_bit = end_bit;
-    b.capacity = (uint32_t)n_edges;
-    if (radix_sort<uint64_t>(b, st, err, s, 64) != cudaSuccess) return PXR_CUDA_ERROR;
-    // the unique pass writes into the buffer the sort did not end in
-    const uint32_t* sel = st.pass_info + kMaxPasses;
-    uint32_t sel_host = 0;
-    if (cudaMemcpyAsync(&sel_host, sel, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess) return PXR_CUDA_ERROR;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return PXR_CUDA_ERROR;
-    uint64_t* uniq = sel_host ? k0 : k1;
-    if (n_edges) k_unique_both<<<grid, kBuildBlock, 0, s>>>(k0, k1, sel, count0, uniq, count1);
-    SortBuffers<uint64_t> b2{};
-    b2.keys[0] = uniq;
-    b2.keys[1] = sel_host ? k1 : k0;
-    b2.count = count1;
-    b2.end_bit = end_bit;
-    b2.capacity = (uint32_t)(2 * n_edges);
-    if (radix_sort<uint64_t>(b2, st, err, s, 64) != cudaSuccess) return PXR_CUDA_ERROR;
-    // result buffer of the second sort relative to b2: pass_info[kMaxPasses] selects keys[0] or keys[1]
-    uint32_t sel2 = 0;
-    if (cudaMemcpyAsync(&sel2, sel, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess) return PXR_CUDA_ERROR;
-    if (cudaStreamSynchronize(s) != cudaSuccess) return PXR_CUDA_ERROR;
-    k_csr_rows<<<grid, kBuildBlock, 0, s>>>(b2.keys[0], b2.keys[1], sel, count1, n, offsets, cols);
+    b.capacity = (uint32_t)(2 * n_edges);
+    if (radix_sort<uint64_t>(b, st, err, s, (int)(2u * bits)) != cudaSuccess) return PXR_CUDA_ERROR;
+    if (n_edges) {
+        // look-back state of the unique pass in the sort's status area (2 KB a
+        // sort tile, two unique tiles each: 40 bytes), after the sort
+        const uint32_t tiles = (uint32_t)((2 * n_edges + kUniqueTile - 1) / kUniqueTile);
+        LookbackState lb{};
+        unsigned char* area = base + L.status;
+        lb.agg = reinterpret_cast<uint64_t*>(area);
+        lb.inc = lb.agg + tiles;
+        lb.flags = reinterpret_cast<uint32_t*>(lb.inc + tiles);
+        uint32_t* tile_ctr = st.tile_ctr;
+        if (cudaMemsetAsync(lb.flags, 0, (size_t)tiles * 4, s) != cudaSuccess) return PXR_CUDA_ERROR;
+        if (cudaMemsetAsync(tile_ctr, 0, 4, s) != cudaSuccess) return PXR_CUDA_ERROR;
+        k_unique_cols<<<tiles, kBuildBlock, 0, s>>>(k0, k1, st.pass_info + kMaxPasses, count0, bits, cols, offsets + 1,
+                                                    tile_ctr, lb, count1, err);
+        // the chunk maxima go where the digit counts were
+        k_fill_max<<<kFillChunks, kBuildBlock, 0, s>>>(offsets + 1, n, st.hist);
+        k_fill_rows<<<kFillChunks, kBuildBlock, 0, s>>>(offsets + 1, n, st.hist);
+        if (cudaGetLastError() != cudaSuccess) return PXR_CUDA_ERROR;
+    }
     uint32_t w[5] = {0, 0, 0, 0, 0};
     if (cudaMemcpyAsync(w, words, 20, cudaMemcpyDeviceToHost, s) != cudaSuccess) return PXR_CUDA_ERROR;
     if (cudaStreamSynchronize(s) != cudaSuccess) return PXR_CUDA_ERROR;
-    (void)sel2;
     if (w[4]) return PXR_INVALID_ARG;   // a vertex id >= n
     if (w[3]) return PXR_DEVICE_FAULT;  // a sort wait ran out
     *m_out = w[1] / 2;

@@ -151,3 +151,19 @@ def test_a_shard_draws_the_same_edges_as_the_whole_batch():
         b_off, b_cols = rows(gs, int(starts_s[k]), int(starts_s[k + 1]))
         np.testing.assert_array_equal(a_off, b_off)
         np.testing.assert_array_equal(a_cols, b_cols)
+
+
+@pytest.mark.parametrize("n,edges,distinct", [(2, 1, 1), (3, 1023, 2), (1 << 20, 3, 3), (5, 1025, 7), (700000, 2048, 2048),
+                                              (129, 4096, 60), (100003, 40000, 39000)])
+def test_build_at_tile_edges_and_with_gaps(n, edges, distinct):
+    """Key counts around the unique pass's tiles, long runs of duplicates, and
+    long stretches of vertices without edges."""
+    rng = np.random.default_rng(edges)
+    pool = rng.integers(0, n, (distinct, 2))
+    pool[0] = (0, n - 1)
+    pick = pool[rng.integers(0, distinct, edges)]
+    pick[0] = pool[0]
+    off, cols, m = B.build_csr(n, _dev(pick[:, 0]), _dev(pick[:, 1]))
+    host = G.csr_from_edges(pick[:, 0], pick[:, 1], n)
+    assert m == host.m
+    _same(B.to_host(off, cols), host)
