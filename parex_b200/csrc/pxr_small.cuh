@@ -176,57 +176,23 @@ __device__ __forceinline__ uint32_t small_sort_tile(const Dev<OffT>& d, SmallSha
     return cur;
 }
 
-// Components, first pass: every vertex of a split cluster points at its
-// smallest same-label neighbour below it, or at itself (link_first_vertex,
-// with W lanes a row and kSlotUnroll slots in flight per lane: the general
-// kernel's one dependent load after another took 10 us a round here).
+// Components, hooking pass: the root of v's tree (the forest is
+// flat) goes under the smallest root among v's same-label neighbours.  Every
+// pointer still leads to a smaller vertex of the same component; an edge whose
+// hook another one overwrote is joined by the last pass, which looks at every edge.
+// A cluster's first-link trees (one per local minimum, a tenth of the
+// vertices) mostly become one here, so that pass
+// finds little left to join (joining them one by one took 24 us a round on the
+// 16,384-vertex planted partition, 11 after this pass).
+// Long rows are left out: their edges are seen from the other ends.
+// W lanes a row; every lane of the warp calls it.
 template <typename OffT>
-__device__ __forceinline__ void small_link_first(const Dev<OffT>& d, uint32_t k, uint32_t v, bool in, uint32_t gl,
-                                                 uint32_t W) {
-    const int32_t lv = in ? d.lab[v] : -1;
-    in = in && in_split(d, k, lv);
-    const OffT beg = in ? d.off[v] : 0, end = in ? d.off[v + 1] : 0;
-    uint32_t p = v;
-    for (OffT s = beg + gl; s < end; s += kSlotUnroll * W) {
-        uint32_t nb[kSlotUnroll];
-        int32_t ln[kSlotUnroll];
-#pragma unroll
-        for (int u = 0; u < kSlotUnroll; ++u) nb[u] = s + u * W < end ? d.cols[s + u * W] : kInvalidEdge;
-#pragma unroll
-        for (int u = 0; u < kSlotUnroll; ++u) ln[u] = nb[u] < v ? d.lab[nb[u]] : -1;
-        bool past = false;
-#pragma unroll
-        for (int u = kSlotUnroll - 1; u >= 0; --u) {   // rows are sorted: the first hit stays
-            if (ln[u] == lv) p = nb[u];
-            past |= slot_valid(nb[u]) && nb[u] >= v;
-        }
-        if (p != v || past) break;
-    }
-    for (uint32_t o = W >> 1; o > 0; o >>= 1) p = min(p, __shfl_xor_sync(0xFFFFFFFFu, p, o));
-    if (in && gl == 0) {
-        d.parent[v] = p;
-        d.acc_max[v] = 0u;
-        d.acc_min[v] = 0xFFFFFFFFu;
-        d.acc_sum[v] = 0;
-        d.acc_cnt[v] = 0u;
-    }
-}
-
-// Components, hooking pass: the root of v's tree (the forest is flat) goes
-// under the smallest root among v's same-label neighbours.  Every pointer
-// still leads to a smaller vertex of the same component; an edge whose hook
-// another one overwrote is joined by the last pass, which looks at every
-// edge.  A cluster's few dozen first-link trees usually become one here, so
-// that pass finds almost nothing left to join (joining them one by one took
-// 24 us a round on the 16,384-vertex planted partition).
-template <typename OffT>
-__device__ __forceinline__ void small_hook(const Dev<OffT>& d, uint32_t k, uint32_t v, bool in, uint32_t gl,
-                                           uint32_t W) {
+__device__ __forceinline__ void hook_row(const Dev<OffT>& d, uint32_t k, uint32_t v, bool in, uint32_t gl, uint32_t W) {
     const int32_t lv = in ? d.lab[v] : -1;
     in = in && in_split(d, k, lv);
     const OffT beg = in ? d.off[v] : 0;
     OffT end = in ? d.off[v + 1] : 0;
-    if ((uint64_t)(end - beg) > d.light_max) end = beg;   // a long row's end of an edge is not needed
+    if ((uint64_t)(end - beg) > d.light_max) end = beg;
     const uint32_t r = in ? ld_relaxed(&d.parent[v]) : 0u;
     uint32_t m = r;
     for (OffT s = beg + gl; s < end; s += kSlotUnroll * W) {
@@ -243,36 +209,6 @@ __device__ __forceinline__ void small_hook(const Dev<OffT>& d, uint32_t k, uint3
     }
     for (uint32_t o = W >> 1; o > 0; o >>= 1) m = min(m, __shfl_xor_sync(0xFFFFFFFFu, m, o));
     if (in && gl == 0 && m < r) atomicMin(&d.parent[r], m);
-}
-
-// Components, joining pass of a light row: union_light_row of the plain
-// schedule (each edge once, from its larger end) with a lane's labels and
-// parents loaded kSlotUnroll slots at a time.
-template <typename OffT>
-__device__ __forceinline__ void small_union_row(const Dev<OffT>& d, uint32_t k, uint32_t v, uint32_t gl, uint32_t W) {
-    const int32_t lv = d.lab[v];
-    if (!in_split(d, k, lv)) return;
-    const OffT beg = d.off[v], end = d.off[v + 1];
-    if ((uint64_t)(end - beg) > d.light_max) return;   // union_long_rows
-    uint32_t hint = ld_relaxed(&d.parent[v]);
-    for (OffT s = beg + gl; s < end; s += kSlotUnroll * W) {
-        uint32_t nb[kSlotUnroll], pr[kSlotUnroll];
-        int32_t ln[kSlotUnroll];
-#pragma unroll
-        for (int u = 0; u < kSlotUnroll; ++u) nb[u] = s + u * W < end ? d.cols[s + u * W] : kInvalidEdge;
-#pragma unroll
-        for (int u = 0; u < kSlotUnroll; ++u) {
-            ln[u] = nb[u] < v ? d.lab[nb[u]] : -1;
-            pr[u] = nb[u] < v ? ld_relaxed(&d.parent[nb[u]]) : 0u;
-        }
-        bool past = false;
-#pragma unroll
-        for (int u = 0; u < kSlotUnroll; ++u) {
-            if (ln[u] == lv && pr[u] != hint) uf_join(d.parent, &d.ctr->err, v, nb[u], hint);
-            past |= slot_valid(nb[u]) && nb[u] >= v;
-        }
-        if (past) break;
-    }
 }
 
 __device__ __forceinline__ uint32_t small_block_max(uint32_t v, uint32_t* sh) {
@@ -608,7 +544,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
 
         // ---- components of split clusters
         if (ld_relaxed(&ctr->any_split)) {
-            small_rows(ids, na, W, [&](uint32_t v, bool in, uint32_t gl) { small_link_first(d, k, v, in, gl, W); });
+            small_rows(ids, na, W, [&](uint32_t v, bool in, uint32_t gl) { link_first_row(d, k, v, in, gl, W); });
             small_sync();
             // ---- compress
             for (uint32_t j = gid; j < na; j += nt) {
@@ -617,7 +553,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
             }
             small_sync();
             // ---- hook
-            small_rows(ids, na, W, [&](uint32_t v, bool in, uint32_t gl) { small_hook(d, k, v, in, gl, W); });
+            small_rows(ids, na, W, [&](uint32_t v, bool in, uint32_t gl) { hook_row(d, k, v, in, gl, W); });
             small_sync();
             // ---- compress again
             for (uint32_t j = gid; j < na; j += nt) {
@@ -626,7 +562,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
             }
             small_sync();
             // ---- union
-            for (uint32_t j = gid / W; j < na; j += nt / W) small_union_row(d, k, ids[j], gid & (W - 1u), W);
+            for (uint32_t j = gid / W; j < na; j += nt / W) union_light_row<true>(d, k, ids[j], gid & (W - 1u), W);
             union_long_rows<OffT, 32>(d, k);
             union_long_rows<OffT, kSmallThreads>(d, k);
             small_sync();
