@@ -45,6 +45,10 @@ struct SpreadAgg {
         atomicMax(&smax[key], v.x);
         atomicMin(&smin[key], v.y);
     }
+    __device__ static void add_shared(T* slot, T v) {
+        atomicMax(&slot->x, v.x);
+        atomicMin(&slot->y, v.y);
+    }
 };
 
 template <typename OffT>
@@ -52,7 +56,11 @@ __global__ void __launch_bounds__(kBlock) k_cluster_spread(Dev<OffT> d, const ui
     pdl_wait();
     const uint32_t count = d.ctr->n_active;
     const uint32_t k = d.ctr->n_clusters;
-    SpreadAgg agg{d.smax, d.smin};
+    __shared__ uint32_t t_keys[kTableSlots];
+    __shared__ uint2 t_vals[kTableSlots];
+    const TableAgg<SpreadAgg> agg{{d.smax, d.smin}, t_keys, t_vals};
+    if (blockIdx.x * kScanTile >= count) return;
+    agg.clear();
     const uint32_t stride = gridDim.x * kScanTile;
     for (uint32_t base = blockIdx.x * kScanTile; base < count; base += stride) {
         const uint32_t first = base + threadIdx.x * kScanItems;
@@ -79,8 +87,9 @@ __global__ void __launch_bounds__(kBlock) k_cluster_spread(Dev<OffT> d, const ui
                 a_last = cur;
             }
         }
-        emit_fragments<SpreadAgg>(has, single, k_first, a_first, k_last, a_last, agg);
+        emit_fragments<TableAgg<SpreadAgg>>(has, single, k_first, a_first, k_last, a_last, agg);
     }
+    agg.flush();
 }
 
 // per cluster: due / in-sweep flags and the start tables of the sweep set
