@@ -250,18 +250,68 @@ __global__ void k_validate(const OffT* off, const uint32_t* cols, uint32_t n, ui
     }
 }
 
-// Static row bins: rows longer than light_max slots go to the wide list (up
-// to wide_max slots, a warp each) or the heavy list (a CTA each); the order
-// inside a list is irrelevant.
+// Static row bins: the rows longer than `above` slots as one list, with sort
+// keys that put the longest first; the heavy rows (a CTA each) are then a
+// prefix of it and the wide rows (a warp each) follow.
 template <typename OffT>
-__global__ void k_bin_rows(const OffT* off, uint32_t n, uint32_t light_max, uint32_t wide_max, uint32_t* wide,
-                           uint32_t* heavy, uint32_t* counts) {
+__global__ void __launch_bounds__(kBlock) k_long_rows(const OffT* off, uint32_t n, uint32_t above, uint32_t* list,
+                                                      uint32_t* keys, uint32_t* count) {
+    __shared__ uint64_t warp_tot[kBlock / 32];
+    __shared__ uint32_t s_base;
+    // one addition to the counter per kScanTile vertices (one per warp queued
+    // 131,000 additions on its word: 0.25 ms at 4.2 M vertices)
+    for (uint64_t t0 = (uint64_t)blockIdx.x * kScanTile; t0 < n; t0 += (uint64_t)gridDim.x * kScanTile) {
+        uint32_t key[kScanItems], cnt = 0;
+#pragma unroll
+        for (int q = 0; q < kScanItems; ++q) {
+            const uint64_t v = t0 + threadIdx.x * kScanItems + q;   // in id order: equal lengths stay so
+            const uint64_t len = v < n ? (uint64_t)(off[v + 1] - off[v]) : 0ull;
+            key[q] = len > above ? 0xFFFFFFFFu - (uint32_t)min(len, (uint64_t)0xFFFFFFFEu) : 0u;   // 0: not listed
+            cnt += key[q] ? 1u : 0u;
+        }
+        uint64_t total;
+        const uint64_t incl = block_inclusive<Add64>((uint64_t)cnt, warp_tot, &total);
+        if (threadIdx.x == 0 && total) s_base = atomicAdd(count, (uint32_t)total);
+        __syncthreads();
+        uint32_t p = s_base + (uint32_t)incl - cnt;
+        __syncthreads();
+#pragma unroll
+        for (int q = 0; q < kScanItems; ++q)
+            if (key[q]) {
+                list[p] = (uint32_t)t0 + threadIdx.x * kScanItems + q;
+                keys[p++] = key[q];
+            }
+    }
+}
+
+__global__ void k_take_sorted(const uint32_t* sorted1, const uint32_t* sel, const uint32_t* count, uint32_t* list) {
+    if (!*sel) return;   // the sort ended in the list's own buffer
+    const uint32_t n = *count;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) list[i] = sorted1[i];
+}
+
+// Rows longer than each of the bounds.
+constexpr int kRowBounds = 8;
+struct RowBounds { uint32_t above[kRowBounds]; };
+
+template <typename OffT>
+__global__ void __launch_bounds__(kBlock) k_count_rows(const OffT* off, uint32_t n, RowBounds b, uint32_t* counts) {
+    __shared__ uint32_t sh[kRowBounds];
+    if (threadIdx.x < kRowBounds) sh[threadIdx.x] = 0;
+    __syncthreads();
+    uint32_t c[kRowBounds] = {};
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const uint64_t len = (uint64_t)(off[v + 1] - off[v]);
-        if (len <= light_max) continue;
-        if (len <= wide_max) wide[atomicAdd(&counts[0], 1u)] = v;
-        else heavy[atomicAdd(&counts[1], 1u)] = v;
+#pragma unroll
+        for (int q = 0; q < kRowBounds; ++q) c[q] += len > b.above[q] ? 1u : 0u;
     }
+#pragma unroll
+    for (int q = 0; q < kRowBounds; ++q) {
+        const uint32_t w = __reduce_add_sync(0xFFFFFFFFu, c[q]);
+        if ((threadIdx.x & 31u) == 0 && w) atomicAdd(&sh[q], w);
+    }
+    __syncthreads();
+    if (threadIdx.x < kRowBounds && sh[threadIdx.x]) atomicAdd(&counts[threadIdx.x], sh[threadIdx.x]);
 }
 
 // rows per bit length of their size (0: empty rows, 32: 2^31 slots or more)
@@ -364,19 +414,21 @@ struct pxr_handle {
     unsigned long long* d_valid = nullptr;
     RoundCtr* h_ctr = nullptr;  // pinned mirror
 
-    uint32_t* d_check = nullptr;   // [3]: invalid-input bits, max row length, heavy rows
+    uint32_t* d_check = nullptr;   // [4]: invalid-input bits, max row length, long rows, edge out of its instance
     RoundCtr* probe_ctr = nullptr;    // scratch counters for the tuner's timed walk steps
     bool plan_forced = false;
     pxr_row_plan plan_info{};         // last plan chosen (pxr_get_row_plan)
     bool sort_forced = false;
     pxr_sort_plan sort_info{0, 16, 2, 0, 0, {0.0f, 0.0f, 0.0f}};   // sweep sort plan (pxr_get_sort_plan)
-    uint32_t light_max = kLightRow;   // row bins (see k_bin_rows)
+    uint32_t light_max = kLightRow;   // row bins (see k_long_rows)
     uint32_t wide_max = kWideRow;
-    uint32_t* wide = nullptr;
+    uint32_t* long_rows = nullptr;    // rows longer than long_above slots, longest first
+    uint32_t long_above = 0;
+    bool long_built = false;          // the list holds the loaded graph's rows
     uint32_t n_wide = 0;
     uint32_t* hist = nullptr;         // [33] rows per bit length of the row size
-    uint32_t* heavy = nullptr;
     uint32_t n_heavy = 0;
+    uint32_t* row_counts = nullptr;   // [kRowBounds]
     // learned sweep schedule
     pxr_schedule sched{};
     uint8_t* sflag = nullptr;
@@ -502,9 +554,9 @@ Dev<OffT> make_dev(pxr_handle* h) {
     d.sort = h->sort;
     d.sort_end_bit = h->sort_end_bit;
     d.light_max = h->light_max;
-    d.wide = h->wide;
+    d.wide = h->long_rows + h->n_heavy;
     d.n_wide = h->n_wide;
-    d.heavy = h->heavy;
+    d.heavy = h->long_rows;
     d.n_heavy = h->n_heavy;
     d.sched = h->sched.mode;
     d.trace = (h->sched.trace && h->records) ? 1u : 0u;
@@ -1185,8 +1237,8 @@ pxr_status allocate(pxr_handle* h, uint32_t n, uint64_t m) {
     A(&h->sort.pass_info, kMaxPasses + 1); A(&h->sort.tile_ctr, kMaxPasses); A(&h->sort.epoch, 1);
     A(&h->sort.status, (size_t)sort_tiles * kRadix);
     A(&h->sort_end_bit, 1); A(&h->fp_end_bit, 1); A(&h->d_n, 1);
-    A(&h->d_num, 1); A(&h->d_valid, 1); A(&h->d_check, 4); A(&h->heavy, N); A(&h->wide, N);
-    A(&h->probe_ctr, 1); A(&h->hist, 33);
+    A(&h->d_num, 1); A(&h->d_valid, 1); A(&h->d_check, 4); A(&h->long_rows, N);
+    A(&h->probe_ctr, 1); A(&h->hist, 33); A(&h->row_counts, kRowBounds);
 #undef A
     if (e != cudaSuccess) {
         const size_t held = h->bytes;
@@ -1236,18 +1288,66 @@ RowPlan default_row_plan(const pxr_handle* h, uint32_t n, uint64_t m) {
     return RowPlan{W, kLightRow, kWideRow};
 }
 
+// Rows longer than each of up to kRowBounds bounds.
 template <typename OffT>
-pxr_status bin_rows(pxr_handle* h, const RowPlan& p, uint32_t* counts) {
+pxr_status count_rows(pxr_handle* h, const std::vector<uint32_t>& above, std::map<uint32_t, uint32_t>* counts) {
     cudaStream_t s = h->stream;
-    PXR_CUDA(h, cudaMemsetAsync(&h->d_check[2], 0, 8, s));
-    if (h->n) {
-        k_bin_rows<OffT><<<grid_for(h->n), kBlock, 0, s>>>(static_cast<const OffT*>(h->off), h->n, p.light_max,
-                                                           p.wide_max, h->wide, h->heavy, &h->d_check[2]);
-        ++h->launches;
-    }
-    PXR_CUDA(h, cudaMemcpyAsync(counts, &h->d_check[2], 8, cudaMemcpyDeviceToHost, s));
+    RowBounds b{};
+    for (int q = 0; q < kRowBounds; ++q) b.above[q] = q < (int)above.size() ? above[q] : 0xFFFFFFFFu;
+    uint32_t c[kRowBounds] = {};
+    PXR_CUDA(h, cudaMemsetAsync(h->row_counts, 0, sizeof(c), s));
+    k_count_rows<OffT><<<std::min(grid_for(h->n), 148u * 8u), kBlock, 0, s>>>(static_cast<const OffT*>(h->off), h->n, b,
+                                                                             h->row_counts);
+    ++h->launches;
+    PXR_CUDA(h, cudaMemcpyAsync(c, h->row_counts, sizeof(c), cudaMemcpyDeviceToHost, s));
     PXR_CUDA(h, cudaStreamSynchronize(s));
+    for (int q = 0; q < (int)above.size() && q < kRowBounds; ++q) (*counts)[above[q]] = c[q];
     return PXR_OK;
+}
+
+// The list of rows longer than `above` slots, longest first: a row's length is
+// the time its warp or CTA takes, so the long ones must not start last, and
+// equally long neighbours in the list keep warps in step (walk step against
+// lists in the order the binning's atomics happened to leave, same plan: R-MAT
+// 24 2,068-2,223 -> 2,010 us, edge differences 2,000 -> 1,895; R-MAT 22
+// 546-575 -> 527-536; R-MAT 20 with rows up to 4,096 slots in the warp bin 175
+// -> 126; the list and its sort take 0.06 ms at 4.2 M vertices).
+// Scratch: the root lists and the idle parity of the active list, which hold
+// nothing between stages.
+template <typename OffT>
+pxr_status build_long_rows(pxr_handle* h, uint32_t above) {
+    if (h->long_built && h->long_above <= above) return PXR_OK;
+    cudaStream_t s = h->stream;
+    PXR_CUDA(h, cudaMemsetAsync(&h->d_check[2], 0, 4, s));
+    k_long_rows<OffT><<<std::min((h->n + kScanTile - 1) / kScanTile, 148u * 8u), kBlock, 0, s>>>(
+        static_cast<const OffT*>(h->off), h->n, above, h->long_rows, h->roots[0], &h->d_check[2]);
+    SortBuffers<uint32_t> b{};
+    b.keys[0] = h->roots[0];
+    b.keys[1] = h->roots[1];
+    b.vals[0] = h->long_rows;
+    b.vals[1] = h->act[h->acur ^ 1];
+    b.count = &h->d_check[2];
+    b.end_bit = h->fp_end_bit;
+    b.capacity = h->n;
+    SortState st = h->sort;
+    st.items_moved = nullptr;
+    PXR_CUDA(h, radix_sort<uint32_t>(b, st, &h->ctr->err, s, 32));
+    k_take_sorted<<<grid_for(h->n), kBlock, 0, s>>>(h->act[h->acur ^ 1], &h->sort.pass_info[kMaxPasses],
+                                                    &h->d_check[2], h->long_rows);
+    h->launches += 2 + 2 + 4;
+    PXR_CUDA(h, cudaGetLastError());
+    h->long_above = above;
+    h->long_built = true;
+    return PXR_OK;
+}
+
+// The plan's bins from the counts of rows above its two bounds.
+void set_bins(pxr_handle* h, const RowPlan& p, std::map<uint32_t, uint32_t>& above) {
+    h->W = p.W;
+    h->light_max = p.light_max;
+    h->wide_max = p.wide_max;
+    h->n_heavy = above[p.wide_max];
+    h->n_wide = above[p.light_max] - above[p.wide_max];
 }
 
 // ---------------------------------------------------------------------------
@@ -1301,6 +1401,14 @@ pxr_status tune_row_plan(pxr_handle* h, const std::array<uint32_t, 33>& hist, Ro
                 cands.push_back(RowPlan{W, lights[i], wides[j]});
             }
         }
+    std::map<uint32_t, uint32_t> above;
+    if (h->maxdeg > lights[0]) {
+        std::vector<uint32_t> bounds(lights, lights + 4);
+        bounds.insert(bounds.end(), wides, wides + 3);
+        pxr_status st = build_long_rows<OffT>(h, lights[0]);
+        if (st == PXR_OK) st = count_rows<OffT>(h, bounds, &above);
+        if (st != PXR_OK) return st;
+    }
     // scratch: x copy in keys[0], x / degree in keys[1], counters in probe_ctr
     float* xs = reinterpret_cast<float*>(h->keys[0]);
     float* xo = reinterpret_cast<float*>(h->keys[1]);
@@ -1310,14 +1418,7 @@ pxr_status tune_row_plan(pxr_handle* h, const std::array<uint32_t, 33>& hist, Ro
     float best_ms = 0.0f;
     bool have = false;
     for (const RowPlan& p : cands) {
-        uint32_t bins[2];
-        pxr_status st = bin_rows<OffT>(h, p, bins);
-        if (st != PXR_OK) return st;
-        h->W = p.W;
-        h->light_max = p.light_max;
-        h->wide_max = p.wide_max;
-        h->n_wide = bins[0];
-        h->n_heavy = bins[1];
+        set_bins(h, p, above);
         Dev<OffT> d = make_dev<OffT>(h);
         d.x = xs;
         d.ctr = h->probe_ctr;
@@ -1377,24 +1478,23 @@ pxr_status choose_row_plan(pxr_handle* h, bool reuse, uint32_t nb_bits) {
             g_plan_cache[key] = plan;
         }
     }
-    uint32_t bins[2] = {0, 0};
-    pxr_status bst = bin_rows<OffT>(h, plan, bins);
-    if (bst != PXR_OK) return bst;
+    std::map<uint32_t, uint32_t> above;
+    if (h->n > 0 && h->maxdeg > plan.light_max) {
+        pxr_status bst = build_long_rows<OffT>(h, plan.light_max);
+        if (bst == PXR_OK) bst = count_rows<OffT>(h, {plan.light_max, plan.wide_max}, &above);
+        if (bst != PXR_OK) return bst;
+    }
+    set_bins(h, plan, above);
     // captured round graphs bake in buffers, nb_bits and the row plan: keep them only if all are unchanged
     if (!reuse || nb_bits != old_bits || plan.W != old.W || plan.light_max != old.light_max ||
-        plan.wide_max != old.wide_max || bins[0] != old_wide || bins[1] != old_heavy)
+        plan.wide_max != old.wide_max || h->n_wide != old_wide || h->n_heavy != old_heavy)
         drop_graphs(h);
     h->nb_bits = nb_bits;
-    h->W = plan.W;
-    h->light_max = plan.light_max;
-    h->wide_max = plan.wide_max;
-    h->n_wide = bins[0];
-    h->n_heavy = bins[1];
     h->plan_info.lanes_per_row = plan.W;
     h->plan_info.light_max = plan.light_max;
     h->plan_info.wide_max = plan.wide_max;
-    h->plan_info.wide_rows = bins[0];
-    h->plan_info.heavy_rows = bins[1];
+    h->plan_info.wide_rows = h->n_wide;
+    h->plan_info.heavy_rows = h->n_heavy;
     h->plan_info.source = source;
     if (source == 1) {
         h->plan_info.candidates = tried;
@@ -1524,6 +1624,7 @@ pxr_status initialize_impl(pxr_handle* h, uint32_t n, uint64_t m, const OffT* of
     if (check[0] & 1u) return fail(h, PXR_INVALID_ARG, "offsets must be non-decreasing");
     if (check[0] & 4u) return fail(h, PXR_INVALID_ARG, "column index out of range");
     h->maxdeg = check[1];
+    h->long_built = false;
     const uint32_t nb_bits = host_bitlen(std::max<uint64_t>(n, h->maxdeg));
     // round state: one cluster, every vertex active; keep the growing epochs
     RoundCtr c;

@@ -1394,8 +1394,11 @@ template <int G, class Pred, class Body>
 __device__ __forceinline__ void for_each_row(const uint32_t* list, uint32_t cnt, const RowGroups<G>& rg, Pred pred,
                                              Body body, bool windows = true) {
     if (G == 32 && windows) {
-        for (uint32_t h0 = rg.first * 32u; h0 < cnt; h0 += rg.step * 32u) {
-            const uint32_t h = h0 + rg.lane;
+        // the window is the warp's next 32 rows of the row-by-row order, not 32
+        // neighbours of the list: neighbours are equally long, and the first
+        // warps would get nothing but the longest
+        for (uint64_t h0 = rg.first; h0 < cnt; h0 += rg.step * 32ull) {
+            const uint64_t h = h0 + rg.lane * (uint64_t)rg.step;
             const uint32_t v = h < cnt ? list[h] : 0u;
             uint32_t pass = __ballot_sync(0xFFFFFFFFu, h < cnt && pred(v));
             while (pass) {

@@ -103,9 +103,9 @@ struct Dev {
     SortState sort;
     uint32_t* sort_end_bit;   // main sort bits
     uint32_t light_max;       // rows up to this many slots: W lanes per row in the round kernels
-    const uint32_t* wide;     // vertices with light_max < row <= wide_max slots (one warp each)
+    const uint32_t* wide;     // vertices with light_max < row <= wide_max slots (one warp each), longest first
     uint32_t n_wide;
-    const uint32_t* heavy;    // vertices with longer rows (one CTA each)
+    const uint32_t* heavy;    // vertices with longer rows (one CTA each), longest first
     uint32_t n_heavy;
     // learned sweep schedule (all zero / null in the plain form)
     uint32_t sched;           // PXR_SCHEDULE_*
