@@ -290,44 +290,54 @@ __global__ void k_take_sorted(const uint32_t* sorted1, const uint32_t* sel, cons
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) list[i] = sorted1[i];
 }
 
+// One cluster with every vertex (start 0, volume 2m, root 0), every counter
+// and statistic zero; only the buffer of the last sweep's results stays.
+__global__ void k_reset_state(RoundCtr* ctr, ClusterTables t, uint32_t n, uint32_t volume) {
+    const uint32_t main_sel = ctr->main_sel;
+    *ctr = RoundCtr{};
+    ctr->n_active = n;
+    ctr->n_clusters = n ? 1u : 0u;
+    ctr->full_components = 1;
+    ctr->done = n ? 0u : 1u;
+    ctr->main_sel = main_sel;
+    ctr->max_parent = 0xFFFFFFFFu;   // the first round sorts globally (the list is in vertex order)
+    ctr->max_csize = n;
+    t.start[0] = 0;
+    t.size[0] = n;
+    t.vol[0] = volume;
+    t.vol_start[0] = 0;
+    t.root[0] = 0;
+    t.best[0] = ~0ull;
+}
+
 // Rows longer than each of the bounds.
 constexpr int kRowBounds = 8;
 struct RowBounds { uint32_t above[kRowBounds]; };
 
+// Row statistics of a graph: rows per bit length of their size (0: empty rows,
+// 32: 2^31 slots or more), then rows longer than each of the bounds.
+constexpr int kRowClasses = 33;
+
 template <typename OffT>
-__global__ void __launch_bounds__(kBlock) k_count_rows(const OffT* off, uint32_t n, RowBounds b, uint32_t* counts) {
-    __shared__ uint32_t sh[kRowBounds];
-    if (threadIdx.x < kRowBounds) sh[threadIdx.x] = 0;
+__global__ void __launch_bounds__(kBlock) k_row_stats(const OffT* off, uint32_t n, RowBounds b, uint32_t* out) {
+    __shared__ uint32_t sh[kRowClasses + kRowBounds];
+    for (int i = threadIdx.x; i < kRowClasses + kRowBounds; i += blockDim.x) sh[i] = 0;
     __syncthreads();
     uint32_t c[kRowBounds] = {};
     for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
         const uint64_t len = (uint64_t)(off[v + 1] - off[v]);
+        atomicAdd(&sh[len >= (1ull << 31) ? 32u : (len ? 32u - __clz((uint32_t)len) : 0u)], 1u);
 #pragma unroll
         for (int q = 0; q < kRowBounds; ++q) c[q] += len > b.above[q] ? 1u : 0u;
     }
 #pragma unroll
     for (int q = 0; q < kRowBounds; ++q) {
         const uint32_t w = __reduce_add_sync(0xFFFFFFFFu, c[q]);
-        if ((threadIdx.x & 31u) == 0 && w) atomicAdd(&sh[q], w);
+        if ((threadIdx.x & 31u) == 0 && w) atomicAdd(&sh[kRowClasses + q], w);
     }
     __syncthreads();
-    if (threadIdx.x < kRowBounds && sh[threadIdx.x]) atomicAdd(&counts[threadIdx.x], sh[threadIdx.x]);
-}
-
-// rows per bit length of their size (0: empty rows, 32: 2^31 slots or more)
-template <typename OffT>
-__global__ void k_degree_hist(const OffT* off, uint32_t n, uint32_t* hist) {
-    __shared__ uint32_t sh[33];
-    for (int i = threadIdx.x; i < 33; i += blockDim.x) sh[i] = 0;
-    __syncthreads();
-    for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < n; v += gridDim.x * blockDim.x) {
-        const uint64_t len = (uint64_t)(off[v + 1] - off[v]);
-        const uint32_t b = len >= (1ull << 31) ? 32u : (len ? 32u - __clz((uint32_t)len) : 0u);
-        atomicAdd(&sh[b], 1u);
-    }
-    __syncthreads();
-    for (int i = threadIdx.x; i < 33; i += blockDim.x)
-        if (sh[i]) atomicAdd(&hist[i], sh[i]);
+    for (int i = threadIdx.x; i < kRowClasses + kRowBounds; i += blockDim.x)
+        if (sh[i]) atomicAdd(&out[i], sh[i]);
 }
 
 // Profiling aid: hold the stream for a moment so the host can queue a whole
@@ -357,6 +367,9 @@ inline uint32_t host_bitlen(uint64_t v) {
 
 // ---------------------------------------------------------------------------
 
+// d_check: four words, then k_row_stats' counts
+constexpr int kCheckWords = 4 + kRowClasses + kRowBounds;
+
 struct pxr_handle {
     pxr_config cfg{};
     std::string err;
@@ -373,8 +386,9 @@ struct pxr_handle {
     uint32_t maxdeg = 0;
     uint32_t W = 8;
     uint32_t nb_bits = 0;
-    std::vector<void*> allocs;
+    std::vector<void*> allocs;       // the arena, and the trace records when traces are on
     size_t bytes = 0;
+    size_t arena_bytes = 0;
 
     void* off = nullptr;
     uint32_t* cols = nullptr;
@@ -414,7 +428,7 @@ struct pxr_handle {
     unsigned long long* d_valid = nullptr;
     RoundCtr* h_ctr = nullptr;  // pinned mirror
 
-    uint32_t* d_check = nullptr;   // [4]: invalid-input bits, max row length, long rows, edge out of its instance
+    uint32_t* d_check = nullptr;   // [4]: invalid-input bits, max row length, long rows, edge out of its instance; then row statistics
     RoundCtr* probe_ctr = nullptr;    // scratch counters for the tuner's timed walk steps
     bool plan_forced = false;
     pxr_row_plan plan_info{};         // last plan chosen (pxr_get_row_plan)
@@ -426,11 +440,12 @@ struct pxr_handle {
     uint32_t long_above = 0;
     bool long_built = false;          // the list holds the loaded graph's rows
     uint32_t n_wide = 0;
-    uint32_t* hist = nullptr;         // [33] rows per bit length of the row size
+    std::array<uint32_t, kRowClasses> row_hist{};   // the loaded graph's rows per bit length of the row size
+    std::map<uint32_t, uint32_t> rows_above;        // rows longer than each bound counted so far
     uint32_t n_heavy = 0;
-    uint32_t* row_counts = nullptr;   // [kRowBounds]
     // learned sweep schedule
     pxr_schedule sched{};
+    bool sched_stale = false;        // skip counters and history wait to be cleared (plain form: nothing reads them)
     uint8_t* sflag = nullptr;
     uint32_t* smax = nullptr;
     uint32_t* smin = nullptr;
@@ -504,6 +519,7 @@ void release(pxr_handle* h) {
     h->records = nullptr;
     h->records_n = 0;
     h->bytes = 0;
+    h->arena_bytes = 0;
     h->initialized = false;
 }
 
@@ -1177,8 +1193,12 @@ pxr_status decompose_stream(pxr_handle* h) {
 
 // ---------------------------------------------------------------------------
 
-// every cluster due, no sweep history (after any change of the partition state)
+// every cluster due, no sweep history (after any change of the partition state);
+// in the plain form without traces, which neither reads nor writes them, when
+// a schedule or traces are switched on (36 bytes a vertex)
 pxr_status reset_schedule_state(pxr_handle* h) {
+    h->sched_stale = !h->sched.mode && !h->sched.trace;
+    if (h->sched_stale) return PXR_OK;
     const size_t N = std::max<uint32_t>(h->n, 1);
     for (int i = 0; i < 2; ++i) {
         PXR_CUDA(h, cudaMemsetAsync(h->tab[i].skip, 0, N * sizeof(uint16_t), h->stream));
@@ -1187,22 +1207,13 @@ pxr_status reset_schedule_state(pxr_handle* h) {
     return PXR_OK;
 }
 
-pxr_status setup_tables_initial(pxr_handle* h) {
-    // one cluster with every vertex: start 0, size n, volume 2m, root 0
-    std::vector<uint32_t> one = {0u, h->n, (uint32_t)h->slots, 0u, 0u};
-    const ClusterTables& t = h->tab[h->tcur];
-    PXR_CUDA(h, cudaMemcpyAsync(t.start, &one[0], 4, cudaMemcpyHostToDevice, h->stream));
-    PXR_CUDA(h, cudaMemcpyAsync(t.size, &one[1], 4, cudaMemcpyHostToDevice, h->stream));
-    PXR_CUDA(h, cudaMemcpyAsync(t.vol, &one[2], 4, cudaMemcpyHostToDevice, h->stream));
-    PXR_CUDA(h, cudaMemcpyAsync(t.vol_start, &one[3], 4, cudaMemcpyHostToDevice, h->stream));
-    PXR_CUDA(h, cudaMemcpyAsync(t.root, &one[4], 4, cudaMemcpyHostToDevice, h->stream));
-    PXR_CUDA(h, cudaMemsetAsync(t.best, 0xFF, 8, h->stream));
-    return PXR_OK;
-}
+constexpr size_t kSliceAlign = 256;   // as cudaMalloc aligns
+constexpr size_t kArenaKeep = 64u << 20;
 
 template <typename OffT>
 pxr_status allocate(pxr_handle* h, uint32_t n, uint64_t m) {
-    release(h);
+    drop_graphs(h);
+    h->initialized = false;
     h->n = n;
     h->m = m;
     h->slots = 2 * m;
@@ -1211,8 +1222,14 @@ pxr_status allocate(pxr_handle* h, uint32_t n, uint64_t m) {
     // look-back state per site, sized for the smallest tile (k_relabel's)
     const uint32_t scan_tiles = (uint32_t)((N + kRelabelTile - 1) / kRelabelTile) + 1;
     const uint32_t sort_tiles = (uint32_t)((N + kSortMinTile - 1) / kSortMinTile) + 1;   // any sort plan's tiles
-    cudaError_t e = cudaSuccess;
-#define A(ptr, cnt) if (e == cudaSuccess) e = dalloc(h, ptr, cnt)
+    // every array is a slice of one allocation: 110 calls of cudaMalloc and
+    // cudaFree took most of a millisecond per handle and graph size
+    struct Slice { void** p; size_t bytes; };
+    std::vector<Slice> slices;
+    auto add = [&](auto** p, size_t count) {
+        slices.push_back({reinterpret_cast<void**>(p), std::max<size_t>(count, 1) * sizeof(**p)});
+    };
+#define A(ptr, cnt) add(ptr, cnt)
     A(reinterpret_cast<OffT**>(&h->off), (size_t)n + 1);
     A(&h->cols, std::max<uint64_t>(h->slots, 1));
     A(&h->lab, N); A(&h->ideg, N); A(&h->x, N); A(&h->xt[0], N); A(&h->xt[1], N);
@@ -1225,7 +1242,6 @@ pxr_status allocate(pxr_handle* h, uint32_t n, uint64_t m) {
     }
     A(&h->sflag, N); A(&h->nflag, N); A(&h->rootc, N); A(&h->mlp, (size_t)kMlpImage);
     A(&h->smax, N); A(&h->smin, N);
-    if (h->sched.trace) { A(&h->records, N); }
     A(&h->cut_off, N); A(&h->split, N); A(&h->allcuts, N); A(&h->rep[0], N); A(&h->rep[1], N);
     A(&h->walk_stats, 3 * kStatSlots);
     for (int i = 0; i <= kSiteRoots; ++i) {
@@ -1237,17 +1253,40 @@ pxr_status allocate(pxr_handle* h, uint32_t n, uint64_t m) {
     A(&h->sort.pass_info, kMaxPasses + 1); A(&h->sort.tile_ctr, kMaxPasses); A(&h->sort.epoch, 1);
     A(&h->sort.status, (size_t)sort_tiles * kRadix);
     A(&h->sort_end_bit, 1); A(&h->fp_end_bit, 1); A(&h->d_n, 1);
-    A(&h->d_num, 1); A(&h->d_valid, 1); A(&h->d_check, 4); A(&h->long_rows, N);
-    A(&h->probe_ctr, 1); A(&h->hist, 33); A(&h->row_counts, kRowBounds);
+    A(&h->d_num, 1); A(&h->d_valid, 1); A(&h->d_check, kCheckWords); A(&h->long_rows, N);
+    A(&h->probe_ctr, 1);
 #undef A
+    size_t total = 0;
+    for (const Slice& q : slices) total += (q.bytes + kSliceAlign - 1) / kSliceAlign * kSliceAlign;
+    // a graph that fits takes over the last one's arena, unless that would hold
+    // more than twice what it needs (or kArenaKeep)
+    const bool keep = h->arena_bytes >= total && h->arena_bytes <= std::max(2 * total, kArenaKeep) && !h->records &&
+                      !h->sched.trace && h->allocs.size() == 1;
+    unsigned char* arena = keep ? static_cast<unsigned char*>(h->allocs[0]) : nullptr;
+    cudaError_t e = cudaSuccess;
+    if (!keep) {
+        release(h);
+        e = dalloc(h, &arena, total);
+        h->arena_bytes = total;
+    }
     if (e != cudaSuccess) {
-        const size_t held = h->bytes;
         release(h);
         if (e == cudaErrorMemoryAllocation)
-            return fail(h, PXR_OUT_OF_MEMORY, "device memory exhausted after " + std::to_string(held >> 20) +
+            return fail(h, PXR_OUT_OF_MEMORY, "device memory exhausted: the graph needs " + std::to_string(total >> 20) +
                                                   " MiB" + (h->cfg.memory_cap_mib ? " (the handle's memory cap is " +
                                                   std::to_string(h->cfg.memory_cap_mib) + " MiB)" : std::string()));
         return cuda_fail(h, e, "cudaMalloc");
+    }
+    for (const Slice& q : slices) {
+        *q.p = arena;
+        arena += (q.bytes + kSliceAlign - 1) / kSliceAlign * kSliceAlign;
+    }
+    if (h->sched.trace) {
+        const cudaError_t er = dalloc(h, &h->records, N);
+        if (er != cudaSuccess) {
+            release(h);
+            return cuda_fail(h, er, "cudaMalloc");
+        }
     }
     h->sort.max_tiles = sort_tiles;
     h->sort.items_moved = &h->ctr->stat_sort_items;
@@ -1288,20 +1327,38 @@ RowPlan default_row_plan(const pxr_handle* h, uint32_t n, uint64_t m) {
     return RowPlan{W, kLightRow, kWideRow};
 }
 
-// Rows longer than each of up to kRowBounds bounds.
+// Bounds of the tuner's candidates and of the heuristic plan: counted with
+// every graph's row statistics.
+constexpr uint32_t kLightBounds[] = {16, 32, 64, 128};
+constexpr uint32_t kWideBounds[] = {1024, 4096, 16384};
+
+RowBounds standard_bounds() {
+    RowBounds b{};
+    int q = 0;
+    for (uint32_t v : kLightBounds) b.above[q++] = v;
+    for (uint32_t v : kWideBounds) b.above[q++] = v;
+    b.above[q] = 0xFFFFFFFFu;
+    return b;
+}
+
+// Count the rows longer than a forced plan's bounds.
 template <typename OffT>
-pxr_status count_rows(pxr_handle* h, const std::vector<uint32_t>& above, std::map<uint32_t, uint32_t>* counts) {
+pxr_status count_rows(pxr_handle* h, uint32_t light_max, uint32_t wide_max) {
+    if (h->rows_above.count(light_max) && h->rows_above.count(wide_max)) return PXR_OK;
     cudaStream_t s = h->stream;
     RowBounds b{};
-    for (int q = 0; q < kRowBounds; ++q) b.above[q] = q < (int)above.size() ? above[q] : 0xFFFFFFFFu;
-    uint32_t c[kRowBounds] = {};
-    PXR_CUDA(h, cudaMemsetAsync(h->row_counts, 0, sizeof(c), s));
-    k_count_rows<OffT><<<std::min(grid_for(h->n), 148u * 8u), kBlock, 0, s>>>(static_cast<const OffT*>(h->off), h->n, b,
-                                                                             h->row_counts);
+    for (uint32_t& v : b.above) v = 0xFFFFFFFFu;
+    b.above[0] = light_max;
+    b.above[1] = wide_max;
+    uint32_t c[2] = {};
+    PXR_CUDA(h, cudaMemsetAsync(h->d_check + 4, 0, (kRowClasses + kRowBounds) * 4, s));
+    k_row_stats<OffT><<<std::min(grid_for(h->n), 148u * 8u), kBlock, 0, s>>>(static_cast<const OffT*>(h->off), h->n, b,
+                                                                            h->d_check + 4);
     ++h->launches;
-    PXR_CUDA(h, cudaMemcpyAsync(c, h->row_counts, sizeof(c), cudaMemcpyDeviceToHost, s));
+    PXR_CUDA(h, cudaMemcpyAsync(c, h->d_check + 4 + kRowClasses, sizeof(c), cudaMemcpyDeviceToHost, s));
     PXR_CUDA(h, cudaStreamSynchronize(s));
-    for (int q = 0; q < (int)above.size() && q < kRowBounds; ++q) (*counts)[above[q]] = c[q];
+    h->rows_above[light_max] = c[0];
+    h->rows_above[wide_max] = c[1];
     return PXR_OK;
 }
 
@@ -1342,7 +1399,8 @@ pxr_status build_long_rows(pxr_handle* h, uint32_t above) {
 }
 
 // The plan's bins from the counts of rows above its two bounds.
-void set_bins(pxr_handle* h, const RowPlan& p, std::map<uint32_t, uint32_t>& above) {
+void set_bins(pxr_handle* h, const RowPlan& p) {
+    std::map<uint32_t, uint32_t>& above = h->rows_above;
     h->W = p.W;
     h->light_max = p.light_max;
     h->wide_max = p.wide_max;
@@ -1379,34 +1437,28 @@ cudaError_t probe_walk_w(pxr_handle* h, const Dev<OffT>& d, float* xt_out) {
 }
 
 template <typename OffT>
-pxr_status tune_row_plan(pxr_handle* h, const std::array<uint32_t, 33>& hist, RowPlan* best, uint32_t* tried,
+pxr_status tune_row_plan(pxr_handle* h, const std::array<uint32_t, kRowClasses>& hist, RowPlan* best, uint32_t* tried,
                          float* best_us) {
     cudaStream_t s = h->stream;
     const uint32_t n = h->n;
     // rows of the largest size class decide which bin bounds can differ
     int top = 0;
-    for (int b = 0; b < 33; ++b)
+    for (int b = 0; b < kRowClasses; ++b)
         if (hist[b]) top = b;
     const uint64_t maxlen = top == 0 ? 0 : (1ull << top) - 1;   // upper bound of the largest class
     std::vector<RowPlan> cands;
     const uint32_t lanes[] = {1, 4, 8, 16, 32};
-    const uint32_t lights[] = {16, 32, 64, 128};
-    const uint32_t wides[] = {1024, 4096, 16384};
     // a bound above the previous one that already holds every row gives the same bins: skip it
     for (uint32_t W : lanes)
         for (int i = 0; i < 4; ++i) {
-            if (i > 0 && (uint64_t)lights[i - 1] >= maxlen) continue;
+            if (i > 0 && (uint64_t)kLightBounds[i - 1] >= maxlen) continue;
             for (int j = 0; j < 3; ++j) {
-                if (j > 0 && (uint64_t)wides[j - 1] >= maxlen) continue;
-                cands.push_back(RowPlan{W, lights[i], wides[j]});
+                if (j > 0 && (uint64_t)kWideBounds[j - 1] >= maxlen) continue;
+                cands.push_back(RowPlan{W, kLightBounds[i], kWideBounds[j]});
             }
         }
-    std::map<uint32_t, uint32_t> above;
-    if (h->maxdeg > lights[0]) {
-        std::vector<uint32_t> bounds(lights, lights + 4);
-        bounds.insert(bounds.end(), wides, wides + 3);
-        pxr_status st = build_long_rows<OffT>(h, lights[0]);
-        if (st == PXR_OK) st = count_rows<OffT>(h, bounds, &above);
+    if (h->maxdeg > kLightBounds[0]) {
+        const pxr_status st = build_long_rows<OffT>(h, kLightBounds[0]);
         if (st != PXR_OK) return st;
     }
     // scratch: x copy in keys[0], x / degree in keys[1], counters in probe_ctr
@@ -1418,7 +1470,7 @@ pxr_status tune_row_plan(pxr_handle* h, const std::array<uint32_t, 33>& hist, Ro
     float best_ms = 0.0f;
     bool have = false;
     for (const RowPlan& p : cands) {
-        set_bins(h, p, above);
+        set_bins(h, p);
         Dev<OffT> d = make_dev<OffT>(h);
         d.x = xs;
         d.ctr = h->probe_ctr;
@@ -1452,14 +1504,7 @@ pxr_status choose_row_plan(pxr_handle* h, bool reuse, uint32_t nb_bits) {
         plan = RowPlan{h->plan_info.lanes_per_row, h->plan_info.light_max, h->plan_info.wide_max};
         source = 3;
     } else if (h->cfg.tune == PXR_TUNE_AUTO && h->n > 0) {
-        cudaStream_t s = h->stream;
-        std::array<uint32_t, 33> hist{};
-        PXR_CUDA(h, cudaMemsetAsync(h->hist, 0, 33 * 4, s));
-        k_degree_hist<OffT><<<std::min(grid_for(h->n), 148u * 4u), kBlock, 0, s>>>(static_cast<const OffT*>(h->off),
-                                                                                   h->n, h->hist);
-        ++h->launches;
-        PXR_CUDA(h, cudaMemcpyAsync(hist.data(), h->hist, 33 * 4, cudaMemcpyDeviceToHost, s));
-        PXR_CUDA(h, cudaStreamSynchronize(s));
+        const std::array<uint32_t, kRowClasses>& hist = h->row_hist;
         std::vector<uint64_t> key{h->n, h->m, sizeof(OffT)};
         key.insert(key.end(), hist.begin(), hist.end());
         bool hit = false;
@@ -1478,13 +1523,12 @@ pxr_status choose_row_plan(pxr_handle* h, bool reuse, uint32_t nb_bits) {
             g_plan_cache[key] = plan;
         }
     }
-    std::map<uint32_t, uint32_t> above;
     if (h->n > 0 && h->maxdeg > plan.light_max) {
         pxr_status bst = build_long_rows<OffT>(h, plan.light_max);
-        if (bst == PXR_OK) bst = count_rows<OffT>(h, {plan.light_max, plan.wide_max}, &above);
+        if (bst == PXR_OK) bst = count_rows<OffT>(h, plan.light_max, plan.wide_max);
         if (bst != PXR_OK) return bst;
     }
-    set_bins(h, plan, above);
+    set_bins(h, plan);
     // captured round graphs bake in buffers, nb_bits and the row plan: keep them only if all are unchanged
     if (!reuse || nb_bits != old_bits || plan.W != old.W || plan.light_max != old.light_max ||
         plan.wide_max != old.wide_max || h->n_wide != old_wide || h->n_heavy != old_heavy)
@@ -1613,33 +1657,32 @@ pxr_status initialize_impl(pxr_handle* h, uint32_t n, uint64_t m, const OffT* of
     h->xcur = h->tcur = h->acur = 0;
     PXR_CUDA(h, cudaMemcpyAsync(h->off, offsets, ((size_t)n + 1) * sizeof(OffT), kind, s));
     if (m) PXR_CUDA(h, cudaMemcpyAsync(h->cols, cols, h->slots * 4, kind, s));
-    PXR_CUDA(h, cudaMemsetAsync(h->d_check, 0, 16, s));
+    // the input checks and the row statistics come back together: one wait
+    PXR_CUDA(h, cudaMemsetAsync(h->d_check, 0, kCheckWords * 4, s));
     k_validate<OffT><<<grid_for(std::max<uint64_t>(h->slots, n)), kBlock, 0, s>>>(
         static_cast<const OffT*>(h->off), h->cols, n, h->slots, &h->d_check[0], &h->d_check[1]);
     ++h->launches;
-    uint32_t check[4] = {0, 0, 0, 0};
-    PXR_CUDA(h, cudaMemcpyAsync(check, h->d_check, 16, cudaMemcpyDeviceToHost, s));
+    const RowBounds bounds = standard_bounds();
+    if (n) {
+        k_row_stats<OffT><<<std::min(grid_for(n), 148u * 8u), kBlock, 0, s>>>(static_cast<const OffT*>(h->off), n, bounds,
+                                                                             h->d_check + 4);
+        ++h->launches;
+    }
+    uint32_t check[kCheckWords] = {};
+    PXR_CUDA(h, cudaMemcpyAsync(check, h->d_check, sizeof(check), cudaMemcpyDeviceToHost, s));
     PXR_CUDA(h, cudaStreamSynchronize(s));
     if (check[0] & 2u) return fail(h, PXR_INVALID_ARG, "offsets must start at 0 and end at 2m");
     if (check[0] & 1u) return fail(h, PXR_INVALID_ARG, "offsets must be non-decreasing");
     if (check[0] & 4u) return fail(h, PXR_INVALID_ARG, "column index out of range");
     h->maxdeg = check[1];
+    std::copy(check + 4, check + 4 + kRowClasses, h->row_hist.begin());
+    h->rows_above.clear();
+    for (int q = 0; q < kRowBounds; ++q) h->rows_above[bounds.above[q]] = check[4 + kRowClasses + q];
     h->long_built = false;
     const uint32_t nb_bits = host_bitlen(std::max<uint64_t>(n, h->maxdeg));
-    // round state: one cluster, every vertex active; keep the growing epochs
-    RoundCtr c;
-    PXR_CUDA(h, cudaMemcpyAsync(&c, h->ctr, sizeof(RoundCtr), cudaMemcpyDeviceToHost, s));
-    PXR_CUDA(h, cudaStreamSynchronize(s));
-    const RoundCtr old = c;
-    std::memset(&c, 0, sizeof(c));
-    c.n_active = n;
-    c.n_clusters = n ? 1u : 0u;
-    c.full_components = 1;
-    c.done = n ? 0u : 1u;
-    c.main_sel = old.main_sel;
-    c.max_parent = 0xFFFFFFFFu;   // the first round sorts globally (the list is in vertex order)
-    c.max_csize = n;
-    PXR_CUDA(h, cudaMemcpyAsync(h->ctr, &c, sizeof(RoundCtr), cudaMemcpyHostToDevice, s));
+    // round state: one cluster, every vertex active; the epochs keep growing
+    k_reset_state<<<1, 1, 0, s>>>(h->ctr, h->tab[h->tcur], n, (uint32_t)h->slots);
+    ++h->launches;
     PXR_CUDA(h, cudaMemsetAsync(h->cert, 0, (size_t)std::max<uint32_t>(n, 1) * 4, s));
     if (n) {
         k_degrees<OffT><<<grid_for(n), kBlock, 0, s>>>(static_cast<const OffT*>(h->off), n, h->ideg, h->lab,
@@ -1649,8 +1692,7 @@ pxr_status initialize_impl(pxr_handle* h, uint32_t n, uint64_t m, const OffT* of
         PXR_CUDA(h, cudaMemcpyAsync(&h->ctr->xmax_walk_bits, &h->ctr->xmax_bits, 4, cudaMemcpyDeviceToDevice, s));
         h->launches += 3;
     }
-    pxr_status st = setup_tables_initial(h);
-    if (st == PXR_OK) st = reset_schedule_state(h);
+    pxr_status st = reset_schedule_state(h);
     if (st == PXR_OK) st = choose_row_plan<OffT>(h, reuse, nb_bits);
     if (st == PXR_OK) st = choose_sort_plan(h);
     if (st != PXR_OK) return st;
@@ -1893,10 +1935,9 @@ pxr_status pxr_cut_clusters(pxr_handle* h) { return run_op(h, kOpCut); }
 pxr_status pxr_decompose(pxr_handle* h, uint32_t* rounds_out) {
     if (!h) return PXR_INVALID_ARG;
     if (!h->initialized) return fail(h, PXR_NOT_INITIALIZED, "no graph uploaded");
-    cudaEvent_t e0, e1;
-    PXR_CUDA(h, cudaEventCreate(&e0));
-    PXR_CUDA(h, cudaEventCreate(&e1));
-    pxr_status st = sync_ctr(h);
+    // every call that ran device work left the counters' mirror up to date
+    const cudaEvent_t e0 = take_event(h), e1 = take_event(h);
+    pxr_status st = PXR_OK;
     const uint32_t start_rounds = h->h_ctr->rounds;
     PXR_CUDA(h, cudaEventRecord(e0, h->stream));
     if (st == PXR_OK) st = h->cfg.driver == PXR_DRIVER_GRAPH ? decompose_graph(h) : decompose_stream(h);
@@ -1904,8 +1945,8 @@ pxr_status pxr_decompose(pxr_handle* h, uint32_t* rounds_out) {
     PXR_CUDA(h, cudaEventSynchronize(e1));
     float ms = 0.f;
     cudaEventElapsedTime(&ms, e0, e1);
-    cudaEventDestroy(e0);
-    cudaEventDestroy(e1);
+    h->event_pool.push_back(e0);
+    h->event_pool.push_back(e1);
     h->last_ms = ms;
     h->last_rounds = h->h_ctr->rounds - start_rounds;
     if (rounds_out) *rounds_out = h->last_rounds;
@@ -2303,6 +2344,10 @@ pxr_status pxr_set_schedule(pxr_handle* h, const pxr_schedule* cfg, const uint16
     if (mode_changed) drop_graphs(h);   // the captured round depends on the mode
     if (!h->allocs.empty()) {
         PXR_CUDA(h, cudaSetDevice(h->device));
+        if (h->sched_stale) {
+            const pxr_status rs = reset_schedule_state(h);
+            if (rs != PXR_OK) return rs;
+        }
         if (!h->mlp_img.empty())
             PXR_CUDA(h, cudaMemcpyAsync(h->mlp, h->mlp_img.data(), kMlpImage * 4, cudaMemcpyHostToDevice, h->stream));
         if (cfg->trace && !h->records) {

@@ -73,15 +73,18 @@ def build(offsets, cols, seed: int = 6582, sc_threshold: float = 0.3, rw_thresho
     off, col = offsets.to(dev), cols.to(dev)
     vol_below = None
     sc = sc_threshold
+    dm, dm_sc = None, None     # one handle for all levels: only a lowered threshold needs another
     while int(off.shape[0]) - 1 > 1 and len(levels) < max_levels:
         n = int(off.shape[0]) - 1
         m = int(col.shape[0]) // 2
-        dm = CudaDeviceManager(seed=seed, sc_threshold=sc, rw_threshold=rw_threshold, device=device)
+        if dm_sc != sc:
+            if dm is not None:
+                dm.close()
+            dm, dm_sc = CudaDeviceManager(seed=seed, sc_threshold=sc, rw_threshold=rw_threshold, device=device), sc
         dm.initialize_device(n, m, off.data_ptr(), False, col.data_ptr())
         dm.expanderDecomposition()
         fp = dm.getFinalPartition()
         cut = dm.countCutEdges()
-        dm.close()
         if m > 0 and cut > 0.95 * m:
             sc *= 0.8          # the reference's adjustment (expander_hierarchy.h:116-121)
             continue
@@ -91,4 +94,6 @@ def build(offsets, cols, seed: int = 6582, sc_threshold: float = 0.3, rw_thresho
         if fp.numClusters == n:
             break              # nothing merged (no edges left): the remaining vertices are roots
         off, col, vol_below = noff, ncol, vol
+    if dm is not None:
+        dm.close()
     return levels

@@ -93,3 +93,35 @@ def test_many_instances_from_the_start():
                   np.diff(g.offsets.astype(np.int64)).astype(np.uint32), g.cols, 2500, 0)
     dm.expanderDecomposition()
     _check(dm, orc)
+
+
+def test_one_handle_takes_graphs_of_any_size_in_turn():
+    """A smaller graph takes over the arena of the last one, a larger one replaces it."""
+    dm = P.CudaDeviceManager()
+    for n in (3000, 500, 40000, 100, 41000):
+        g = G.sbm_graph(n, max(2, n // 300), 9.0, 1.0, n)
+        dm.initialize(g)
+        orc = O.Oracle(g.offsets, g.cols, O.MODE_PXR)
+        orc.set_potentials(dm.readRandomWalkValues().astype(np.float64))
+        _check(dm, orc, dm.expanderDecomposition())
+
+
+def test_schedule_switched_on_after_plain_graphs():
+    """A handle that ran plain graphs starts the learned schedule with every cluster due, as a new one does."""
+    from parex_b200 import learn
+    model = learn.Model.load()
+    used, fresh = P.CudaDeviceManager(), P.CudaDeviceManager()
+    for n in (30000, 5000):
+        used.initialize(G.sbm_graph(n, 20, 9.0, 1.0, n))
+        used.expanderDecomposition()
+    g = G.sbm_graph(20000, 20, 9.0, 1.0, 7)
+    used.initialize(g)
+    out = []
+    for dm in (used, fresh):
+        if dm is fresh:
+            dm.initialize(g)
+        dm.set_schedule(P._lib.SCHEDULE_LEARNED, model.weights, model.norm, **learn.SHIPPED_SCHEDULE)
+        dm.expanderDecomposition()
+        out.append((dm.getFinalPartition().clusterIds, dm.downloadCertificates()))
+    np.testing.assert_array_equal(out[0][0], out[1][0])
+    np.testing.assert_array_equal(out[0][1], out[1][1])
