@@ -376,8 +376,6 @@ struct pxr_handle {
     int device = 0;
     cudaStream_t own_stream = nullptr;
     cudaStream_t side_stream = nullptr;   // captures the bodies of IF nodes
-    cudaStream_t walk_side[2] = {};       // the wide- and heavy-row walk kernels, beside the light-row one
-    cudaEvent_t walk_ev[3] = {};          // fork, and the two joins
     cudaStream_t stream = nullptr;
     bool initialized = false;
     bool off64 = false;
@@ -643,15 +641,13 @@ void collect_phases(pxr_handle* h) {
 // ---------------------------------------------------------------------------
 // stages
 
-// launches of the long-row kernels: warp per wide row, CTA per heavy row
-int long_launches(const pxr_handle* h) { return (h->n_wide ? 1 : 0) + (h->n_heavy ? 1 : 0); }
-uint32_t wide_grid(const pxr_handle* h) { return std::min((h->n_wide + kBlock / 32 - 1) / (kBlock / 32), 148u * 16u); }
-uint32_t heavy_grid(const pxr_handle* h) { return std::min(h->n_heavy, 148u * 16u); }
-#define PXR_LONG(h, kern, ...)                                                                         \
-    do {                                                                                               \
-        if ((h)->n_wide) launch_pdl(kern<OffT, 32>, wide_grid(h), kBlock, 0, s, __VA_ARGS__);          \
-        if ((h)->n_heavy) launch_pdl(kern<OffT, kBlock>, heavy_grid(h), kBlock, 0, s, __VA_ARGS__);    \
-    } while (0)
+bool has_long(const RowParts& p) { return p.heavy + p.wide > 0; }
+
+// blocks of a row launch for the handle's heavy and wide rows
+RowParts row_parts(const pxr_handle* h) {
+    return RowParts{std::min(h->n_heavy, 148u * 16u),
+                    std::min((h->n_wide + kBlock / 32 - 1) / (kBlock / 32), 148u * 16u)};
+}
 
 // Launch with programmatic stream serialization: the kernel may be scheduled
 // while its predecessor in the stream drains, and waits in pdl_wait() before
@@ -726,45 +722,13 @@ cudaError_t if_region(pxr_handle* h, cudaGraphConditionalHandle cond, F&& body) 
     return cudaStreamUpdateCaptureDependencies(h->stream, &node, 1, cudaStreamSetCaptureDependencies);
 }
 
-// A row kernel in its three parts, which work disjoint rows: light(st)
-// launches the light-row kernel(s) on s, wide(st) and heavy(st) the
-// warp- and CTA-per-row kernels on the handle's two side streams, forked
-// from s and joined back into it.  Running side by side, each part fills the
-// SMs the others leave idle in their last wave (in a captured graph the three
-// are parallel branches).  With no long rows, light(s) alone.
-template <class Light, class Wide, class Heavy>
-void launch_row_parts(pxr_handle* h, cudaStream_t s, Light light, Wide wide, Heavy heavy) {
-    if (!h->n_wide && !h->n_heavy) {
-        light(s);
-        return;
-    }
-    cudaEventRecord(h->walk_ev[0], s);
-    if (h->n_wide) {
-        cudaStreamWaitEvent(h->walk_side[0], h->walk_ev[0], 0);
-        wide(h->walk_side[0]);
-        cudaEventRecord(h->walk_ev[1], h->walk_side[0]);
-    }
-    if (h->n_heavy) {
-        cudaStreamWaitEvent(h->walk_side[1], h->walk_ev[0], 0);
-        heavy(h->walk_side[1]);
-        cudaEventRecord(h->walk_ev[2], h->walk_side[1]);
-    }
-    light(s);
-    if (h->n_wide) cudaStreamWaitEvent(s, h->walk_ev[1], 0);
-    if (h->n_heavy) cudaStreamWaitEvent(s, h->walk_ev[2], 0);
-}
-
 // One walk step: light rows of the active list (W lanes each), the wide list
 // (a warp per row) and the heavy list (a CTA per row).
 template <typename OffT, int W>
 void launch_walk(pxr_handle* h, const Dev<OffT>& d, cudaStream_t s, const float* xt_in, float* xt_out) {
-    launch_row_parts(
-        h, s,
-        [&](cudaStream_t st) {
-            k_walk<OffT, W><<<grid_for((uint64_t)h->n * W), kBlock, 0, st>>>(d, h->ids[h->acur], xt_in, xt_out);
-        },
-        [&](cudaStream_t st) { k_walk_long<OffT, 32><<<wide_grid(h), kBlock, 0, st>>>(d, xt_in, xt_out); },
-        [&](cudaStream_t st) { k_walk_long<OffT, kBlock><<<heavy_grid(h), kBlock, 0, st>>>(d, xt_in, xt_out); });
+    const RowParts p = row_parts(h);
+    launch_pdl(has_long(p) ? k_walk<OffT, W, true> : k_walk<OffT, W, false>, p.heavy + p.wide + grid_for((uint64_t)h->n * W), kBlock, 0, s, d, p, h->ids[h->acur], xt_in,
+               xt_out);
 }
 
 template <typename OffT, int W>
@@ -773,7 +737,7 @@ cudaError_t op_walk(pxr_handle* h, bool in_round = false) {
     cudaStream_t s = h->stream;
     hold_for_profiling(h);
     phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, s, d, 0, kNoCond, kNoCond); });
-    phase(h, kPhWalk, 1 + long_launches(h), [&] { launch_walk<OffT, W>(h, d, s, h->xt[h->xcur], h->xt[h->xcur ^ 1]); });
+    phase(h, kPhWalk, 1, [&] { launch_walk<OffT, W>(h, d, s, h->xt[h->xcur], h->xt[h->xcur ^ 1]); });
     // the next walk's fixed-point scale follows max |x'|; inside a plain round
     // the cut stage recomputes it over the recentred potentials anyway
     if (!in_round || h->sched.mode) phase(h, kPhBook, 1, [&] { launch_pdl(k_after_walk<OffT>, 1, 1, 0, s, d); });
@@ -799,6 +763,8 @@ cudaError_t op_sweep(pxr_handle* h) {
     }
     phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, s, d, 1, c_gsort, c_chunk); });
     const uint32_t tiles = std::max((h->n + kScanTile - 1) / kScanTile, 1u);
+    const RowParts parts = row_parts(h);
+    const uint32_t row_grid = parts.heavy + parts.wide + grid_for((uint64_t)h->n * W);
     if (h->sched.mode)
         phase(h, kPhSched, 3, [&] {
             launch_pdl(k_cluster_spread<OffT>, std::min(tiles, kMaxGrid), kBlock, 0, s, d, h->ids[h->acur]);
@@ -811,25 +777,12 @@ cudaError_t op_sweep(pxr_handle* h) {
         phase(h, kPhEmit, 1, [&] {
             launch_pdl(k_emit_sched<OffT>, tiles, kBlock, 0, s, d, h->act[h->acur], h->keys[0], h->vals[0], t.best);
         });
-        phase(h, kPhNodeDiff, 2 + long_launches(h), [&] {
-            launch_row_parts(
-                h, s,
-                [&](cudaStream_t st) {
-                    k_nodediff<OffT, W><<<grid_for((uint64_t)h->n * W), kBlock, 0, st>>>(d, h->vals[0], 1);
-                    k_nodediff<OffT, W><<<grid_for((uint64_t)h->n * W), kBlock, 0, st>>>(d, h->ids[h->acur], 0);
-                },
-                [&](cudaStream_t st) { k_nodediff_long<OffT, 32><<<wide_grid(h), kBlock, 0, st>>>(d); },
-                [&](cudaStream_t st) { k_nodediff_long<OffT, kBlock><<<heavy_grid(h), kBlock, 0, st>>>(d); });
+        phase(h, kPhNodeDiff, 1, [&] {
+            launch_pdl(has_long(parts) ? k_nodediff<OffT, W, true> : k_nodediff<OffT, W, false>, row_grid, kBlock, 0, s, d, parts, h->ids[h->acur], h->vals[0]);
         });
     } else {
-        phase(h, kPhNodeDiff, 1 + long_launches(h), [&] {
-            launch_row_parts(
-                h, s,
-                [&](cudaStream_t st) {
-                    k_nodediff<OffT, W><<<grid_for((uint64_t)h->n * W), kBlock, 0, st>>>(d, h->ids[h->acur], 0);
-                },
-                [&](cudaStream_t st) { k_nodediff_long<OffT, 32><<<wide_grid(h), kBlock, 0, st>>>(d); },
-                [&](cudaStream_t st) { k_nodediff_long<OffT, kBlock><<<heavy_grid(h), kBlock, 0, st>>>(d); });
+        phase(h, kPhNodeDiff, 1, [&] {
+            launch_pdl(has_long(parts) ? k_nodediff<OffT, W, true> : k_nodediff<OffT, W, false>, row_grid, kBlock, 0, s, d, parts, h->ids[h->acur], (const uint32_t*)nullptr);
         });
         phase(h, kPhEmit, 1, [&] {
             launch_pdl(k_emit<OffT>, grid_for(h->n), kBlock, 0, s, d, h->act[h->acur], h->keys[0], h->vals[0], t.best);
@@ -883,6 +836,7 @@ cudaError_t op_cut(pxr_handle* h) {
     const ClusterTables& t = h->tab[h->tcur];
     const ClusterTables& nt = h->tab[h->tcur ^ 1];
     const uint32_t tiles = std::max((h->n + kScanTile - 1) / kScanTile, 1u);
+    const RowParts parts = row_parts(h);
     hold_for_profiling(h);
     phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, s, d, 2, kNoCond, kNoCond); });
     if (h->sched.mode)
@@ -894,7 +848,7 @@ cudaError_t op_cut(pxr_handle* h) {
     phase(h, kPhCutInit, 1, [&] {
         launch_pdl(k_cut_init<OffT>, grid_for(h->n), kBlock, 0, s, d, t, h->vals[0], h->vals[1], h->keys[0], h->keys[1]);
     });
-    phase(h, kPhUnion, 3 + (d.union_sampled ? 3 : 0) + long_launches(h), [&] {
+    phase(h, kPhUnion, 3 + (d.union_sampled ? 3 : 0), [&] {
         launch_pdl(k_link_first<OffT>, grid_for(h->n), kBlock, 0, s, d, h->ids[h->acur]);
         launch_pdl(k_compress<OffT>, grid_for(h->n), kBlock, 0, s, d, h->ids[h->acur]);
         if (d.union_sampled) {
@@ -902,14 +856,9 @@ cudaError_t op_cut(pxr_handle* h) {
             launch_pdl(k_compress<OffT>, grid_for(h->n), kBlock, 0, s, d, h->ids[h->acur]);
             launch_pdl(k_union_reps<OffT>, grid_for(h->n), kBlock, 0, s, d, t, h->vals[0], h->vals[1]);
         }
-        // lock-free unions over disjoint rows: the three parts side by side
-        launch_row_parts(
-            h, s,
-            [&](cudaStream_t st) {
-                k_union<OffT, kUnionLanes><<<grid_for((uint64_t)h->n * kUnionLanes), kBlock, 0, st>>>(d, h->ids[h->acur]);
-            },
-            [&](cudaStream_t st) { k_union_long<OffT, 32><<<wide_grid(h), kBlock, 0, st>>>(d); },
-            [&](cudaStream_t st) { k_union_long<OffT, kBlock><<<heavy_grid(h), kBlock, 0, st>>>(d); });
+        launch_pdl(has_long(parts) ? k_union<OffT, kUnionLanes, true> : k_union<OffT, kUnionLanes, false>,
+                   parts.heavy + parts.wide + grid_for((uint64_t)h->n * kUnionLanes), kBlock, 0, s, d, parts,
+                   h->ids[h->acur]);
     });
     phase(h, kPhComponents, 1, [&] {
         launch_pdl(k_components_data<OffT>, std::min(tiles, kMaxGrid), kBlock, 0, s, d, t, h->vals[0], h->vals[1],
@@ -929,15 +878,10 @@ cudaError_t op_cut(pxr_handle* h) {
         launch_pdl(k_apply<OffT>, tiles, kBlock, 0, s, d, t, h->vals[0], h->vals[1], h->keys[0], h->keys[1],
                                                h->act[h->acur ^ 1], h->par[h->acur ^ 1]);
     });
-    phase(h, kPhDisable, 1 + long_launches(h), [&] {
-        // disjoint rows; shared results are atomics (volumes, max |x|): side by side
-        launch_row_parts(
-            h, s,
-            [&](cudaStream_t st) {
-                k_ids_disable<OffT, W><<<tiles, kBlock, 0, st>>>(d, h->ids[h->acur], h->ids[h->acur ^ 1], h->xt[h->xcur], nt);
-            },
-            [&](cudaStream_t st) { k_disable_long<OffT, 32><<<wide_grid(h), kBlock, 0, st>>>(d, h->xt[h->xcur], nt); },
-            [&](cudaStream_t st) { k_disable_long<OffT, kBlock><<<heavy_grid(h), kBlock, 0, st>>>(d, h->xt[h->xcur], nt); });
+    phase(h, kPhDisable, 1, [&] {
+        launch_pdl(has_long(parts) ? k_ids_disable<OffT, W, true> : k_ids_disable<OffT, W, false>,
+                   parts.heavy + parts.wide + tiles, kBlock, 0, s, d, parts, h->ids[h->acur], h->ids[h->acur ^ 1],
+                   h->xt[h->xcur], nt);
     });
     phase(h, kPhCvol, 1, [&] { launch_pdl(k_cvol_scan<OffT>, tiles, kBlock, 0, s, d, nt); });
     if (h->sched.mode || d.trace)
@@ -1481,7 +1425,7 @@ pxr_status tune_row_plan(pxr_handle* h, const std::array<uint32_t, kRowClasses>&
         PXR_CUDA(h, cudaEventSynchronize(e1));
         float ms = 0.0f;
         PXR_CUDA(h, cudaEventElapsedTime(&ms, e0, e1));
-        h->launches += 4ull * (1 + long_launches(h));
+        h->launches += 4;
         if (!have || ms < best_ms) { best_ms = ms; *best = p; have = true; }
     }
     h->event_pool.push_back(e0);
@@ -1805,11 +1749,6 @@ pxr_status pxr_create(const pxr_config* cfg, pxr_handle** out) {
     if (cudaSetDevice(h->device) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->own_stream, cudaStreamNonBlocking) != cudaSuccess ||
         cudaStreamCreateWithFlags(&h->side_stream, cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&h->walk_side[0], cudaStreamNonBlocking) != cudaSuccess ||
-        cudaStreamCreateWithFlags(&h->walk_side[1], cudaStreamNonBlocking) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->walk_ev[0], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->walk_ev[1], cudaEventDisableTiming) != cudaSuccess ||
-        cudaEventCreateWithFlags(&h->walk_ev[2], cudaEventDisableTiming) != cudaSuccess ||
         cudaMallocHost(&h->h_ctr, sizeof(RoundCtr)) != cudaSuccess) {
         delete h;
         return PXR_CUDA_ERROR;
@@ -1847,10 +1786,6 @@ void pxr_destroy(pxr_handle* h) {
     if (h->h_ctr) cudaFreeHost(h->h_ctr);
     if (h->own_stream) cudaStreamDestroy(h->own_stream);
     if (h->side_stream) cudaStreamDestroy(h->side_stream);
-    for (cudaStream_t st : h->walk_side)
-        if (st) cudaStreamDestroy(st);
-    for (cudaEvent_t ev : h->walk_ev)
-        if (ev) cudaEventDestroy(ev);
     delete h;
 }
 

@@ -305,6 +305,150 @@ __global__ void k_loop_cond(Dev<OffT> d, cudaGraphConditionalHandle cond) {
 }
 
 // ---------------------------------------------------------------------------
+// Long rows.  Rows longer than Dev::light_max slots are binned once per graph
+// into two static lists: "wide" rows (up to Dev::wide_max slots) get one warp
+// each, "heavy" rows one CTA each (G = 32 or kBlock lanes per row, slots
+// strided by G with kSlotUnroll independent loads per step, group reduction).
+// Every accumulation is order-independent, so the binning does not change
+// any result.
+//
+// One launch serves the three bins: its first blocks take the heavy rows, the
+// next the wide rows (both longest first), the rest the light rows, so that the
+// longest rows start first and the shorter ones fill the SMs beside them.  (As
+// three kernels on three streams the bins ran side by side only while the
+// process had few streams: the second handle's step on R-MAT 20 took 157 us
+// where the first one's took 133.)
+struct RowParts {
+    uint32_t heavy, wide;   // blocks of the launch that take the heavy and the wide rows
+
+    // this block's part (0 heavy, 1 wide, 2 light), its index there and the part's blocks
+    // LONG false: a launch without heavy or wide blocks (its kernel keeps only
+    // the light rows' code and registers).
+    template <bool LONG>
+    __device__ __forceinline__ int part(uint32_t* block, uint32_t* blocks) const {
+        if (!LONG) {
+            *block = blockIdx.x;
+            *blocks = gridDim.x;
+            return 2;
+        }
+        if (blockIdx.x < heavy) {
+            *block = blockIdx.x;
+            *blocks = heavy;
+            return 0;
+        }
+        if (blockIdx.x < heavy + wide) {
+            *block = blockIdx.x - heavy;
+            *blocks = wide;
+            return 1;
+        }
+        *block = blockIdx.x - heavy - wide;
+        *blocks = gridDim.x - heavy - wide;
+        return 2;
+    }
+};
+
+template <int WARPS, typename T>
+__device__ __forceinline__ T block_sum(T v, T* sh) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+    __syncthreads();
+    if (lane == 0) sh[warp] = v;
+    __syncthreads();
+    T t = 0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < WARPS; ++w) t += sh[w];
+    return t;  // valid in thread 0
+}
+
+// sum over the G lanes of a row group; valid in the group's first lane
+template <int G, typename T>
+__device__ __forceinline__ T group_sum(T v, T* sh) {
+    if constexpr (G == 32) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
+        return v;
+    } else {
+        return block_sum<G / 32, T>(v, sh);
+    }
+}
+
+// the rows of one list that a group visits: group index, group count, lane
+template <int G>
+struct RowGroups {
+    uint32_t first, step, lane;
+    __device__ __forceinline__ RowGroups(uint32_t block, uint32_t blocks) {
+        if constexpr (G == 32) {
+            first = (block * blockDim.x + threadIdx.x) >> 5;
+            step = (blocks * blockDim.x) >> 5;
+            lane = threadIdx.x & 31u;
+        } else {
+            first = block;
+            step = blocks;
+            lane = threadIdx.x;
+        }
+    }
+};
+
+// Rows of a long-row list that pass `pred`, each handed to `body` with the
+// whole group.  With `windows` a warp-per-row group tests a window of 32
+// rows at once, one per lane, and then works the passing rows one after
+// another: lists whose rows mostly fail (clusters not split, not swept) cost
+// one load chain per 32 rows instead of per row.  Where most rows pass, the
+// row-by-row order spreads the rows over the warps more evenly.  pred(v)
+// runs per lane; body(v) on every lane.
+template <int G, class Pred, class Body>
+__device__ __forceinline__ void for_each_row(const uint32_t* list, uint32_t cnt, const RowGroups<G>& rg, Pred pred,
+                                             Body body, bool windows = true) {
+    if (G == 32 && windows) {
+        // the window is the warp's next 32 rows of the row-by-row order, not 32
+        // neighbours of the list: neighbours are equally long, and the first
+        // warps would get nothing but the longest
+        for (uint64_t h0 = rg.first; h0 < cnt; h0 += rg.step * 32ull) {
+            const uint64_t h = h0 + rg.lane * (uint64_t)rg.step;
+            const uint32_t v = h < cnt ? list[h] : 0u;
+            uint32_t pass = __ballot_sync(0xFFFFFFFFu, h < cnt && pred(v));
+            while (pass) {
+                const int src = __ffs(pass) - 1;
+                pass &= pass - 1u;
+                body(__shfl_sync(0xFFFFFFFFu, v, src));
+            }
+        }
+    } else {
+        for (uint32_t h = rg.first; h < cnt; h += rg.step) {
+            const uint32_t v = list[h];
+            if (pred(v)) body(v);
+        }
+    }
+}
+
+template <typename OffT>
+__device__ __forceinline__ const uint32_t* row_list(const Dev<OffT>& d, int G, uint32_t* count) {
+    *count = G == 32 ? d.n_wide : d.n_heavy;
+    return G == 32 ? d.wide : d.heavy;
+}
+
+// A long row's head: vertex, label and slot bounds (label -1 past the list).
+template <typename OffT>
+struct RowHead {
+    uint32_t v;
+    int32_t lab;
+    OffT beg, end;
+};
+
+template <typename OffT>
+__device__ __forceinline__ RowHead<OffT> row_head(const Dev<OffT>& d, const uint32_t* list, uint32_t h, uint32_t cnt) {
+    RowHead<OffT> r{0u, -1, 0, 0};
+    if (h < cnt) {
+        r.v = list[h];
+        r.lab = d.lab[r.v];
+        r.beg = d.off[r.v];
+        r.end = d.off[r.v + 1];
+    }
+    return r;
+}
+
+// ---------------------------------------------------------------------------
 // walk: x'[v] = 0.9 * sum_{u ~ v, valid} x[u]/d(u) + 0.1 * x[v]
 // (fusedRandomWalk_WarpParallel, cuda/devRandomWalk.h:117-203), W lanes per
 // vertex, vertices in id order, exact fixed-point sum.
@@ -377,24 +521,21 @@ __device__ __forceinline__ uint32_t walk_finish(const Dev<OffT>& d, uint32_t v, 
 }
 
 template <typename OffT, int W>
-__global__ void PXR_WALK_BOUNDS k_walk(Dev<OffT> d, const uint32_t* ids, const float* xt_in,
-                                                 float* xt_out) {
-    pdl_wait();
+__device__ __forceinline__ void walk_light_rows(const Dev<OffT>& d, const uint32_t* ids, const float* xt_in,
+                                                float* xt_out, uint32_t block, uint32_t blocks, double scale, double inv,
+                                                uint32_t& vmax, unsigned long long& st_v, unsigned long long& st_s,
+                                                unsigned long long& st_g) {
     const uint32_t count = d.ctr->n_active;
-    const int e = fixed_exponent(d.ctr->xmax_bits, d.nb_bits);
-    const double scale = pow2(e), inv = pow2(-e);
     const uint32_t gl = threadIdx.x & (W - 1);
-    const uint32_t groups = (gridDim.x * blockDim.x) / W;
-    const uint32_t warp0 = ((blockIdx.x * blockDim.x + threadIdx.x) & ~31u) / W;
-    uint32_t vmax = 0;
-    unsigned long long st_v = 0, st_s = 0, st_g = 0;
+    const uint32_t groups = (blocks * blockDim.x) / W;
+    const uint32_t warp0 = ((block * blockDim.x + threadIdx.x) & ~31u) / W;
     for (uint32_t j0 = warp0; j0 < count; j0 += groups) {
         const uint32_t j = j0 + (threadIdx.x & 31u) / W;
         const bool valid = j < count;
         uint32_t v = valid ? ids[j] : 0u;
         OffT beg = valid ? d.off[v] : 0, end = valid ? d.off[v + 1] : 0;
         const bool light = valid && (uint64_t)(end - beg) <= d.light_max;
-        if (!light) beg = end;      // long rows: k_walk_long
+        if (!light) beg = end;      // long rows: walk_long_rows
         int64_t acc = 0;
         for (OffT s = beg + gl; s < end; s += kSlotUnroll * W) {
             uint32_t nb[kSlotUnroll];
@@ -417,6 +558,72 @@ __global__ void PXR_WALK_BOUNDS k_walk(Dev<OffT> d, const uint32_t* ids, const f
             vmax = b > vmax ? b : vmax;
         }
     }
+}
+
+// A group's share of one long row (G = 32: a warp, else the whole block; sh:
+// shared scratch of G / 32 sums).
+template <typename OffT, int G>
+__device__ __forceinline__ void walk_long_rows(const Dev<OffT>& d, const float* xt_in, float* xt_out, uint32_t block,
+                                               uint32_t blocks, double scale, double inv, int64_t* sh, uint32_t& vmax, unsigned long long& st_v,
+                                               unsigned long long& st_s, unsigned long long& st_g) {
+    uint32_t cnt;
+    const uint32_t* list = row_list(d, G, &cnt);
+    const RowGroups<G> rg(block, blocks);
+    // With PXR_WALK_PREFETCH the next row's id, label and bounds are loaded
+    // before this row's slots are gathered, so a row's setup loads overlap
+    // the previous row's gathers.
+    RowHead<OffT> nx = row_head(d, list, rg.first, cnt);
+    for (uint32_t h = rg.first; h < cnt; h += rg.step) {
+        RowHead<OffT> cur;
+        if (PXR_WALK_PREFETCH) {
+            cur = nx;
+            nx = row_head(d, list, h + rg.step, cnt);
+        } else {
+            cur = row_head(d, list, h, cnt);
+        }
+        if (cur.lab < 0) continue;
+        const uint32_t v = cur.v;
+        const OffT beg = cur.beg, end = cur.end;
+        int64_t acc = 0;
+        unsigned long long g = 0;
+        for (OffT s = beg + rg.lane; s < end; s += kSlotUnroll * G) {
+            uint32_t nb[kSlotUnroll];
+#pragma unroll
+            for (int u = 0; u < kSlotUnroll; ++u) nb[u] = s + u * G < end ? stream_col(d.cols + s + u * G) : kInvalidEdge;
+            float xv[kSlotUnroll];
+#pragma unroll
+            for (int u = 0; u < kSlotUnroll; ++u) xv[u] = slot_valid(nb[u]) ? xt_in[nb[u]] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < kSlotUnroll; ++u)
+                if (slot_valid(nb[u])) { acc += to_fixed(xv[u], scale); ++g; }
+        }
+        acc = group_sum<G, int64_t>(acc, sh);
+        st_g += g;
+        if (rg.lane == 0) {
+            const uint32_t b = walk_finish(d, v, acc, inv, xt_out);
+            vmax = b > vmax ? b : vmax;
+            st_v += 1;
+            st_s += (unsigned long long)(end - beg);
+        }
+    }
+}
+
+template <typename OffT, int W, bool LONG>
+__global__ void PXR_WALK_BOUNDS k_walk(Dev<OffT> d, RowParts parts, const uint32_t* ids, const float* xt_in,
+                                       float* xt_out) {
+    pdl_wait();
+    __shared__ int64_t sh[kBlock / 32];
+    const int e = fixed_exponent(d.ctr->xmax_bits, d.nb_bits);
+    const double scale = pow2(e), inv = pow2(-e);
+    uint32_t vmax = 0, block, blocks;
+    unsigned long long st_v = 0, st_s = 0, st_g = 0;
+    const int part = parts.part<LONG>(&block, &blocks);
+    if (part == 0)
+        walk_long_rows<OffT, kBlock>(d, xt_in, xt_out, block, blocks, scale, inv, sh, vmax, st_v, st_s, st_g);
+    else if (part == 1)
+        walk_long_rows<OffT, 32>(d, xt_in, xt_out, block, blocks, scale, inv, sh, vmax, st_v, st_s, st_g);
+    else
+        walk_light_rows<OffT, W>(d, ids, xt_in, xt_out, block, blocks, scale, inv, vmax, st_v, st_s, st_g);
     walk_block_totals(d, vmax, st_v, st_s, st_g);
 }
 
@@ -430,23 +637,12 @@ constexpr uint32_t kSweepListShare = 8;
 // ids: the active list in vertex order (count n_active), or with sweep_list
 // the sweep set as the learned schedule's emit compacted it (count n_sweep,
 // every entry swept).
-//
-// The learned schedule launches both forms; one returns at once: the sweep
-// set (in the last sort's order, so its rows are scattered) when it is a
-// small part of the active list, the vertex-order scan (coalesced) when it
-// holds a large cluster.
 template <typename OffT, int W>
-__global__ void __launch_bounds__(kBlock) k_nodediff(Dev<OffT> d, const uint32_t* ids, int sweep_list = 0) {
-    pdl_wait();
-    if (d.ctr->walk_only) return;   // nothing due: the round only walks
-    if (d.sched) {
-        const bool small = (uint64_t)d.ctr->n_sweep * kSweepListShare <= d.ctr->n_active;
-        if (sweep_list ? !small : small) return;
-    }
-    const uint32_t count = sweep_list ? d.ctr->n_sweep : d.ctr->n_active;
+__device__ __forceinline__ void nodediff_light_rows(const Dev<OffT>& d, const uint32_t* ids, uint32_t count,
+                                                    bool sweep_list, uint32_t block, uint32_t blocks) {
     const uint32_t gl = threadIdx.x & (W - 1);
-    const uint32_t groups = (gridDim.x * blockDim.x) / W;
-    const uint32_t warp0 = ((blockIdx.x * blockDim.x + threadIdx.x) & ~31u) / W;
+    const uint32_t groups = (blocks * blockDim.x) / W;
+    const uint32_t warp0 = ((block * blockDim.x + threadIdx.x) & ~31u) / W;
     for (uint32_t j0 = warp0; j0 < count; j0 += groups) {
         const uint32_t j = j0 + (threadIdx.x & 31u) / W;
         const bool valid = j < count;
@@ -456,7 +652,7 @@ __global__ void __launch_bounds__(kBlock) k_nodediff(Dev<OffT> d, const uint32_t
         const uint32_t mine = in ? ordered_bits(d.x[v]) : 0u;
         OffT beg = in ? d.off[v] : 0, end = in ? d.off[v + 1] : 0;
         const bool light = in && (uint64_t)(end - beg) <= d.light_max;
-        if (!light) beg = end;      // long rows: k_nodediff_long
+        if (!light) beg = end;      // long rows: nodediff_long_rows
         int32_t c = 0;
         for (OffT s = beg + gl; s < end; s += kSlotUnroll * W) {
             uint32_t nb[kSlotUnroll];
@@ -476,6 +672,61 @@ __global__ void __launch_bounds__(kBlock) k_nodediff(Dev<OffT> d, const uint32_t
 #pragma unroll
         for (int o = W / 2; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o, W);
         if (light && gl == 0) d.dv[v] = make_int2(c, (int)d.ideg[v]);
+    }
+}
+
+template <typename OffT, int G>
+__device__ __forceinline__ void nodediff_long_rows(const Dev<OffT>& d, uint32_t block, uint32_t blocks, int32_t* sh) {
+    uint32_t cnt;
+    const uint32_t* list = row_list(d, G, &cnt);
+    const RowGroups<G> rg(block, blocks);
+    auto swept = [&](uint32_t v) {
+        const int32_t lv = d.lab[v];
+        return lv >= 0 && (!d.sched || (d.sflag[lv] & 2u));
+    };
+    for_each_row<G>(list, cnt, rg, swept, [&](uint32_t v) {
+        const uint32_t mine = ordered_bits(d.x[v]);
+        const OffT beg = d.off[v], end = d.off[v + 1];
+        int32_t c = 0;
+        for (OffT s = beg + rg.lane; s < end; s += kSlotUnroll * G) {
+            uint32_t nb[kSlotUnroll];
+#pragma unroll
+            for (int u = 0; u < kSlotUnroll; ++u) nb[u] = s + u * G < end ? stream_col(d.cols + s + u * G) : kInvalidEdge;
+            float xn[kSlotUnroll];
+#pragma unroll
+            for (int u = 0; u < kSlotUnroll; ++u) xn[u] = slot_valid(nb[u]) ? d.x[nb[u]] : 0.0f;
+#pragma unroll
+            for (int u = 0; u < kSlotUnroll; ++u) {
+                if (!slot_valid(nb[u])) continue;
+                const uint32_t o = ordered_bits(xn[u]);
+                c += (o < mine || (o == mine && nb[u] < v)) ? -1 : 1;
+            }
+        }
+        c = group_sum<G, int32_t>(c, sh);
+        if (rg.lane == 0) d.dv[v] = make_int2(c, (int)d.ideg[v]);
+    }, d.sched != 0);   // the plain form takes the edge differences of every row
+}
+
+// sweep: the learned schedule's compacted sweep set, or null in the plain form.
+// The sweep set (in the last sort's order, so its rows are scattered) is walked
+// when it is a small part of the active list, the vertex-order list (coalesced)
+// when it holds a large cluster.
+template <typename OffT, int W, bool LONG>
+__global__ void __launch_bounds__(kBlock) k_nodediff(Dev<OffT> d, RowParts parts, const uint32_t* ids,
+                                                     const uint32_t* sweep) {
+    pdl_wait();
+    if (d.ctr->walk_only) return;   // nothing due: the round only walks
+    __shared__ int32_t sh[kBlock / 32];
+    uint32_t block, blocks;
+    const int part = parts.part<LONG>(&block, &blocks);
+    if (part == 0) {
+        nodediff_long_rows<OffT, kBlock>(d, block, blocks, sh);
+    } else if (part == 1) {
+        nodediff_long_rows<OffT, 32>(d, block, blocks, sh);
+    } else {
+        const bool listed = sweep && (uint64_t)d.ctr->n_sweep * kSweepListShare <= d.ctr->n_active;
+        nodediff_light_rows<OffT, W>(d, listed ? sweep : ids, listed ? d.ctr->n_sweep : d.ctr->n_active, listed, block,
+                                     blocks);
     }
 }
 
@@ -886,15 +1137,50 @@ __device__ __forceinline__ void union_light_row(const Dev<OffT>& d, uint32_t k, 
     }
 }
 
-template <typename OffT, int W>
-__global__ void __launch_bounds__(kBlock) k_union(Dev<OffT> d, const uint32_t* ids) {
+template <typename OffT, int G>
+__device__ __forceinline__ void union_long_rows(const Dev<OffT>& d, uint32_t k, uint32_t block, uint32_t blocks) {
+    uint32_t cnt;
+    const uint32_t* list = row_list(d, G, &cnt);
+    const RowGroups<G> rg(block, blocks);
+    auto in_split_cluster = [&](uint32_t v) {
+        const int32_t lv = d.lab[v];
+        if (lv < 0) return false;
+        const uint32_t c = (uint32_t)lv >= k ? (uint32_t)lv - k : (uint32_t)lv;   // cut labels are c or K + c
+        return c < k && d.split[c] != 0;
+    };
+    for_each_row<G>(list, cnt, rg, in_split_cluster, [&](uint32_t v) {
+        const int32_t lv = d.lab[v];
+        const OffT beg = d.off[v], end = d.off[v + 1];
+        uint32_t hint;
+        if (union_skip_row(d, k, v, lv, hint)) return;
+        for (OffT s = beg + rg.lane; s < end; s += G) {
+            const uint32_t nb = d.cols[s];
+            if (!slot_valid(nb) || nb == v) continue;
+            if (!d.union_sampled && nb > v) break;
+            if (d.lab[nb] == lv) uf_join(d.parent, &d.ctr->err, v, nb, hint);
+        }
+    });
+}
+
+template <typename OffT, int W, bool LONG>
+__global__ void __launch_bounds__(kBlock) k_union(Dev<OffT> d, RowParts parts, const uint32_t* ids) {
     pdl_wait();
     if (d.ctr->walk_only || !d.ctr->any_split) return;
     const uint32_t count = d.ctr->n_active;
     const uint32_t k = d.ctr->n_clusters;
+    uint32_t block, blocks;
+    const int part = parts.part<LONG>(&block, &blocks);
+    if (part == 0) {
+        union_long_rows<OffT, kBlock>(d, k, block, blocks);
+        return;
+    }
+    if (part == 1) {
+        union_long_rows<OffT, 32>(d, k, block, blocks);
+        return;
+    }
     const uint32_t gl = threadIdx.x & (W - 1);
-    const uint32_t groups = (gridDim.x * blockDim.x) / W;
-    const uint32_t first = (blockIdx.x * blockDim.x + threadIdx.x) / W;
+    const uint32_t groups = (blocks * blockDim.x) / W;
+    const uint32_t first = (block * blockDim.x + threadIdx.x) / W;
     if (d.union_sampled) {
         for (uint32_t j = first; j < count; j += groups) union_light_row<true>(d, k, ids[j], gl, (uint32_t)W);
     } else {
@@ -1220,13 +1506,58 @@ __global__ void __launch_bounds__(kBlock) k_apply(Dev<OffT> d, ClusterTables t, 
         }
 }
 
+// Returns max |x| over the rows this thread finished.
+template <typename OffT, int G>
+__device__ __forceinline__ uint32_t disable_long_rows(const Dev<OffT>& d, float* xt, const ClusterTables& nt,
+                                                      uint32_t block, uint32_t blocks, uint32_t* sh) {
+    uint32_t cnt;
+    const uint32_t* list = row_list(d, G, &cnt);
+    const RowGroups<G> rg(block, blocks);
+    uint32_t vmax = 0;
+    // rows of clusters born from a split only: k_ids_disable refreshed x / degree of the others
+    auto rescanned = [&](uint32_t v) {
+        const int32_t lv = d.lab[v];
+        return lv >= 0 && d.nflag[lv] == kRowsScan;
+    };
+    for_each_row<G>(list, cnt, rg, rescanned, [&](uint32_t v) {
+        const int32_t lv = d.lab[v];
+        const OffT beg = d.off[v], end = d.off[v + 1];
+        uint32_t deg = 0;
+        for (OffT s = beg + rg.lane; s < end; s += G) {
+            const uint32_t nb = d.cols[s];
+            if (!slot_valid(nb)) continue;
+            if (d.lab[nb] != lv) d.cols[s] = nb | kDisabledBit;
+            else ++deg;
+        }
+        deg = group_sum<G, uint32_t>(deg, sh);
+        if (rg.lane == 0) {
+            d.ideg[v] = deg;
+            const float xv = d.x[v];
+            xt[v] = deg ? __double2float_rn(__ddiv_rn((double)xv, (double)deg)) : 0.0f;
+            const uint32_t b = __float_as_uint(fabsf(xv));
+            vmax = b > vmax ? b : vmax;
+            atomicAdd(&nt.vol[lv], deg);
+        }
+    });
+    return vmax;
+}
+
 // next round's vertex-order list, edge disabling (disableEdgesKernel_node,
 // cuda/devPartition.h:80-146), internal degrees, x/d, cluster volumes.
-template <typename OffT, int W>
-__global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, const uint32_t* ids, uint32_t* ids_next,
-                                                        float* xt, ClusterTables nt) {
+template <typename OffT, int W, bool LONG>
+__global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, RowParts parts, const uint32_t* ids,
+                                                        uint32_t* ids_next, float* xt, ClusterTables nt) {
     pdl_wait();
     if (d.ctr->walk_only) return;   // nothing due: the round only walks
+    uint32_t block, blocks;
+    const int part = parts.part<LONG>(&block, &blocks);
+    if (part != 2) {   // disjoint rows; the shared results (volumes, max |x|) are atomics
+        __shared__ uint32_t sh[kBlock / 32];
+        const uint32_t m = part == 0 ? disable_long_rows<OffT, kBlock>(d, xt, nt, block, blocks, sh)
+                                     : disable_long_rows<OffT, 32>(d, xt, nt, block, blocks, sh);
+        block_atomic_max(&d.ctr->xmax_bits, m);
+        return;
+    }
     __shared__ uint64_t warp_tot[kBlock / 32];
     __shared__ uint64_t s_excl;
     __shared__ uint32_t s_list[kScanTile];
@@ -1286,7 +1617,7 @@ __global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, const uint3
         const bool noscan = rows != kRowsScan;   // not split: no slot can have become inter-cluster
         OffT beg = valid ? d.off[v] : 0, end = valid ? d.off[v + 1] : 0;
         const bool light = valid && (uint64_t)(end - beg) <= d.light_max;
-        if (!light || noscan) beg = end;      // long rows: k_disable_long
+        if (!light || noscan) beg = end;      // long rows: disable_long_rows
         uint32_t deg = 0;
         for (OffT s = beg + gl; s < end; s += kSlotUnroll * W) {
             uint32_t nb[kSlotUnroll];
@@ -1330,293 +1661,6 @@ __global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, const uint3
     block_atomic_max(&d.ctr->xmax_bits, vmax);
     for (uint32_t q = threadIdx.x; q < kScanTile; q += kBlock)
         if (s_hkey[q] != 0xFFFFFFFFu && s_hval[q]) atomicAdd(&nt.vol[s_hkey[q]], s_hval[q]);
-}
-
-// ---------------------------------------------------------------------------
-// Long rows.  Rows longer than Dev::light_max slots are binned once per graph
-// into two static lists: "wide" rows (up to Dev::wide_max slots) get one warp
-// each, "heavy" rows one CTA each (G = 32 or kBlock lanes per row, slots
-// strided by G with kSlotUnroll independent loads per step, group reduction).
-// Every accumulation is order-independent, so the binning does not change
-// any result.
-
-template <int WARPS, typename T>
-__device__ __forceinline__ T block_sum(T v, T* sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    __syncthreads();
-    if (lane == 0) sh[warp] = v;
-    __syncthreads();
-    T t = 0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < WARPS; ++w) t += sh[w];
-    return t;  // valid in thread 0
-}
-
-// sum over the G lanes of a row group; valid in the group's first lane
-template <int G, typename T>
-__device__ __forceinline__ T group_sum(T v, T* sh) {
-    if constexpr (G == 32) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-        return v;
-    } else {
-        return block_sum<G / 32, T>(v, sh);
-    }
-}
-
-// the rows of one list that a group visits: group index, group count, lane
-template <int G>
-struct RowGroups {
-    uint32_t first, step, lane;
-    __device__ __forceinline__ RowGroups() {
-        if constexpr (G == 32) {
-            first = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-            step = (gridDim.x * blockDim.x) >> 5;
-            lane = threadIdx.x & 31u;
-        } else {
-            first = blockIdx.x;
-            step = gridDim.x;
-            lane = threadIdx.x;
-        }
-    }
-};
-
-// Rows of a long-row list that pass `pred`, each handed to `body` with the
-// whole group.  With `windows` a warp-per-row group tests a window of 32
-// rows at once, one per lane, and then works the passing rows one after
-// another: lists whose rows mostly fail (clusters not split, not swept) cost
-// one load chain per 32 rows instead of per row.  Where most rows pass, the
-// row-by-row order spreads the rows over the warps more evenly.  pred(v)
-// runs per lane; body(v) on every lane.
-template <int G, class Pred, class Body>
-__device__ __forceinline__ void for_each_row(const uint32_t* list, uint32_t cnt, const RowGroups<G>& rg, Pred pred,
-                                             Body body, bool windows = true) {
-    if (G == 32 && windows) {
-        // the window is the warp's next 32 rows of the row-by-row order, not 32
-        // neighbours of the list: neighbours are equally long, and the first
-        // warps would get nothing but the longest
-        for (uint64_t h0 = rg.first; h0 < cnt; h0 += rg.step * 32ull) {
-            const uint64_t h = h0 + rg.lane * (uint64_t)rg.step;
-            const uint32_t v = h < cnt ? list[h] : 0u;
-            uint32_t pass = __ballot_sync(0xFFFFFFFFu, h < cnt && pred(v));
-            while (pass) {
-                const int src = __ffs(pass) - 1;
-                pass &= pass - 1u;
-                body(__shfl_sync(0xFFFFFFFFu, v, src));
-            }
-        }
-    } else {
-        for (uint32_t h = rg.first; h < cnt; h += rg.step) {
-            const uint32_t v = list[h];
-            if (pred(v)) body(v);
-        }
-    }
-}
-
-template <typename OffT>
-__device__ __forceinline__ const uint32_t* row_list(const Dev<OffT>& d, int G, uint32_t* count) {
-    *count = G == 32 ? d.n_wide : d.n_heavy;
-    return G == 32 ? d.wide : d.heavy;
-}
-
-// A long row's head: vertex, label and slot bounds (label -1 past the list).
-template <typename OffT>
-struct RowHead {
-    uint32_t v;
-    int32_t lab;
-    OffT beg, end;
-};
-
-template <typename OffT>
-__device__ __forceinline__ RowHead<OffT> row_head(const Dev<OffT>& d, const uint32_t* list, uint32_t h, uint32_t cnt) {
-    RowHead<OffT> r{0u, -1, 0, 0};
-    if (h < cnt) {
-        r.v = list[h];
-        r.lab = d.lab[r.v];
-        r.beg = d.off[r.v];
-        r.end = d.off[r.v + 1];
-    }
-    return r;
-}
-
-// A group's share of one long row (G = 32: a warp, else the whole block; sh:
-// shared scratch of G / 32 sums).
-template <typename OffT, int G>
-__device__ __forceinline__ void walk_long_rows(const Dev<OffT>& d, const float* xt_in, float* xt_out, double scale,
-                                               double inv, int64_t* sh, uint32_t& vmax, unsigned long long& st_v,
-                                               unsigned long long& st_s, unsigned long long& st_g) {
-    uint32_t cnt;
-    const uint32_t* list = row_list(d, G, &cnt);
-    const RowGroups<G> rg;
-    // With PXR_WALK_PREFETCH the next row's id, label and bounds are loaded
-    // before this row's slots are gathered, so a row's setup loads overlap
-    // the previous row's gathers.
-    RowHead<OffT> nx = row_head(d, list, rg.first, cnt);
-    for (uint32_t h = rg.first; h < cnt; h += rg.step) {
-        RowHead<OffT> cur;
-        if (PXR_WALK_PREFETCH) {
-            cur = nx;
-            nx = row_head(d, list, h + rg.step, cnt);
-        } else {
-            cur = row_head(d, list, h, cnt);
-        }
-        if (cur.lab < 0) continue;
-        const uint32_t v = cur.v;
-        const OffT beg = cur.beg, end = cur.end;
-        int64_t acc = 0;
-        unsigned long long g = 0;
-        for (OffT s = beg + rg.lane; s < end; s += kSlotUnroll * G) {
-            uint32_t nb[kSlotUnroll];
-#pragma unroll
-            for (int u = 0; u < kSlotUnroll; ++u) nb[u] = s + u * G < end ? stream_col(d.cols + s + u * G) : kInvalidEdge;
-            float xv[kSlotUnroll];
-#pragma unroll
-            for (int u = 0; u < kSlotUnroll; ++u) xv[u] = slot_valid(nb[u]) ? xt_in[nb[u]] : 0.0f;
-#pragma unroll
-            for (int u = 0; u < kSlotUnroll; ++u)
-                if (slot_valid(nb[u])) { acc += to_fixed(xv[u], scale); ++g; }
-        }
-        acc = group_sum<G, int64_t>(acc, sh);
-        st_g += g;
-        if (rg.lane == 0) {
-            const uint32_t b = walk_finish(d, v, acc, inv, xt_out);
-            vmax = b > vmax ? b : vmax;
-            st_v += 1;
-            st_s += (unsigned long long)(end - beg);
-        }
-    }
-}
-
-template <typename OffT, int G>
-__global__ void PXR_WALK_BOUNDS k_walk_long(Dev<OffT> d, const float* xt_in, float* xt_out) {
-    pdl_wait();
-    __shared__ int64_t sh[kBlock / 32];
-    const int e = fixed_exponent(d.ctr->xmax_bits, d.nb_bits);
-    uint32_t vmax = 0;
-    unsigned long long st_v = 0, st_s = 0, st_g = 0;
-    walk_long_rows<OffT, G>(d, xt_in, xt_out, pow2(e), pow2(-e), sh, vmax, st_v, st_s, st_g);
-    walk_block_totals(d, vmax, st_v, st_s, st_g);
-}
-
-template <typename OffT, int G>
-__device__ __forceinline__ void nodediff_long_rows(const Dev<OffT>& d, int32_t* sh) {
-    uint32_t cnt;
-    const uint32_t* list = row_list(d, G, &cnt);
-    const RowGroups<G> rg;
-    auto swept = [&](uint32_t v) {
-        const int32_t lv = d.lab[v];
-        return lv >= 0 && (!d.sched || (d.sflag[lv] & 2u));
-    };
-    for_each_row<G>(list, cnt, rg, swept, [&](uint32_t v) {
-        const uint32_t mine = ordered_bits(d.x[v]);
-        const OffT beg = d.off[v], end = d.off[v + 1];
-        int32_t c = 0;
-        for (OffT s = beg + rg.lane; s < end; s += kSlotUnroll * G) {
-            uint32_t nb[kSlotUnroll];
-#pragma unroll
-            for (int u = 0; u < kSlotUnroll; ++u) nb[u] = s + u * G < end ? stream_col(d.cols + s + u * G) : kInvalidEdge;
-            float xn[kSlotUnroll];
-#pragma unroll
-            for (int u = 0; u < kSlotUnroll; ++u) xn[u] = slot_valid(nb[u]) ? d.x[nb[u]] : 0.0f;
-#pragma unroll
-            for (int u = 0; u < kSlotUnroll; ++u) {
-                if (!slot_valid(nb[u])) continue;
-                const uint32_t o = ordered_bits(xn[u]);
-                c += (o < mine || (o == mine && nb[u] < v)) ? -1 : 1;
-            }
-        }
-        c = group_sum<G, int32_t>(c, sh);
-        if (rg.lane == 0) d.dv[v] = make_int2(c, (int)d.ideg[v]);
-    }, d.sched != 0);   // the plain form takes the edge differences of every row
-}
-
-template <typename OffT, int G>
-__global__ void __launch_bounds__(kBlock) k_nodediff_long(Dev<OffT> d) {
-    pdl_wait();
-    if (d.ctr->walk_only) return;   // nothing due: the round only walks
-    __shared__ int32_t sh[kBlock / 32];
-    nodediff_long_rows<OffT, G>(d, sh);
-}
-
-template <typename OffT, int G>
-__device__ __forceinline__ void union_long_rows(const Dev<OffT>& d, uint32_t k) {
-    uint32_t cnt;
-    const uint32_t* list = row_list(d, G, &cnt);
-    const RowGroups<G> rg;
-    auto in_split_cluster = [&](uint32_t v) {
-        const int32_t lv = d.lab[v];
-        if (lv < 0) return false;
-        const uint32_t c = (uint32_t)lv >= k ? (uint32_t)lv - k : (uint32_t)lv;   // cut labels are c or K + c
-        return c < k && d.split[c] != 0;
-    };
-    for_each_row<G>(list, cnt, rg, in_split_cluster, [&](uint32_t v) {
-        const int32_t lv = d.lab[v];
-        const OffT beg = d.off[v], end = d.off[v + 1];
-        uint32_t hint;
-        if (union_skip_row(d, k, v, lv, hint)) return;
-        for (OffT s = beg + rg.lane; s < end; s += G) {
-            const uint32_t nb = d.cols[s];
-            if (!slot_valid(nb) || nb == v) continue;
-            if (!d.union_sampled && nb > v) break;
-            if (d.lab[nb] == lv) uf_join(d.parent, &d.ctr->err, v, nb, hint);
-        }
-    });
-}
-
-template <typename OffT, int G>
-__global__ void __launch_bounds__(kBlock) k_union_long(Dev<OffT> d) {
-    pdl_wait();
-    if (d.ctr->walk_only || !d.ctr->any_split) return;   // nothing due, or nothing split
-    union_long_rows<OffT, G>(d, d.ctr->n_clusters);
-}
-
-// Returns max |x| over the rows this thread finished.
-template <typename OffT, int G>
-__device__ __forceinline__ uint32_t disable_long_rows(const Dev<OffT>& d, float* xt, const ClusterTables& nt,
-                                                      uint32_t* sh) {
-    uint32_t cnt;
-    const uint32_t* list = row_list(d, G, &cnt);
-    const RowGroups<G> rg;
-    uint32_t vmax = 0;
-    // rows of clusters born from a split only: k_ids_disable refreshed x / degree of the others
-    auto rescanned = [&](uint32_t v) {
-        const int32_t lv = d.lab[v];
-        return lv >= 0 && d.nflag[lv] == kRowsScan;
-    };
-    for_each_row<G>(list, cnt, rg, rescanned, [&](uint32_t v) {
-        const int32_t lv = d.lab[v];
-        const OffT beg = d.off[v], end = d.off[v + 1];
-        uint32_t deg = 0;
-        for (OffT s = beg + rg.lane; s < end; s += G) {
-            const uint32_t nb = d.cols[s];
-            if (!slot_valid(nb)) continue;
-            if (d.lab[nb] != lv) d.cols[s] = nb | kDisabledBit;
-            else ++deg;
-        }
-        deg = group_sum<G, uint32_t>(deg, sh);
-        if (rg.lane == 0) {
-            d.ideg[v] = deg;
-            const float xv = d.x[v];
-            xt[v] = deg ? __double2float_rn(__ddiv_rn((double)xv, (double)deg)) : 0.0f;
-            const uint32_t b = __float_as_uint(fabsf(xv));
-            vmax = b > vmax ? b : vmax;
-            atomicAdd(&nt.vol[lv], deg);
-        }
-    });
-    return vmax;
-}
-
-template <typename OffT, int G>
-__global__ void __launch_bounds__(kBlock) k_disable_long(Dev<OffT> d, float* xt, ClusterTables nt) {
-    pdl_wait();
-    if (d.ctr->walk_only) return;   // nothing due: the round only walks
-    __shared__ uint32_t sh[kBlock / 32];
-    uint32_t vmax = disable_long_rows<OffT, G>(d, xt, nt, sh);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) vmax = max(vmax, __shfl_xor_sync(0xFFFFFFFFu, vmax, o));
-    if ((threadIdx.x & 31u) == 0 && vmax) atomicMax(&d.ctr->xmax_bits, vmax);
 }
 
 // exclusive prefix of cluster volumes over labels

@@ -310,8 +310,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
                     ++st_v;
                 }
             });
-            walk_long_rows<OffT, 32>(d, xt_in, xt_out, scale, inv, sm.row_sum, vmax, st_v, st_s, st_g);
-            walk_long_rows<OffT, kSmallThreads>(d, xt_in, xt_out, scale, inv, sm.row_sum, vmax, st_v, st_s, st_g);
+            walk_long_rows<OffT, 32>(d, xt_in, xt_out, blockIdx.x, gridDim.x, scale, inv, sm.row_sum, vmax, st_v, st_s, st_g);
+            walk_long_rows<OffT, kSmallThreads>(d, xt_in, xt_out, blockIdx.x, gridDim.x, scale, inv, sm.row_sum, vmax, st_v, st_s, st_g);
             vmax = small_block_max(vmax, sm.red);
             if (threadIdx.x == 0 && vmax) atomicMax(&ctr->xmax_walk_bits, vmax);
         }
@@ -365,8 +365,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
             for (uint32_t o = W >> 1; o > 0; o >>= 1) c += __shfl_xor_sync(0xFFFFFFFFu, c, o);
             if (light && gl == 0) d.dv[v] = make_int2(c, (int)d.ideg[v]);
         });
-        nodediff_long_rows<OffT, 32>(d, reinterpret_cast<int32_t*>(sm.row_cnt));
-        nodediff_long_rows<OffT, kSmallThreads>(d, reinterpret_cast<int32_t*>(sm.row_cnt));
+        nodediff_long_rows<OffT, 32>(d, blockIdx.x, gridDim.x, reinterpret_cast<int32_t*>(sm.row_cnt));
+        nodediff_long_rows<OffT, kSmallThreads>(d, blockIdx.x, gridDim.x, reinterpret_cast<int32_t*>(sm.row_cnt));
         // ---- the sort's tiles, one a CTA
         // While no previous cluster (a contiguous
         // run of the active list) is longer than a tile, a cluster's items lie in
@@ -563,8 +563,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
             small_sync();
             // ---- union
             for (uint32_t j = gid / W; j < na; j += nt / W) union_light_row<true>(d, k, ids[j], gid & (W - 1u), W);
-            union_long_rows<OffT, 32>(d, k);
-            union_long_rows<OffT, kSmallThreads>(d, k);
+            union_long_rows<OffT, 32>(d, k, blockIdx.x, gridDim.x);
+            union_long_rows<OffT, kSmallThreads>(d, k, blockIdx.x, gridDim.x);
             small_sync();
         }
         // ---- per-cluster data
@@ -770,8 +770,8 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
                     h = (h + 1u) & (kSmallHash - 1u);
                 }
             });
-            vmax = max(vmax, disable_long_rows<OffT, 32>(d, xt_out, nt_tab, sm.row_cnt));
-            vmax = max(vmax, disable_long_rows<OffT, kSmallThreads>(d, xt_out, nt_tab, sm.row_cnt));
+            vmax = max(vmax, disable_long_rows<OffT, 32>(d, xt_out, nt_tab, blockIdx.x, gridDim.x, sm.row_cnt));
+            vmax = max(vmax, disable_long_rows<OffT, kSmallThreads>(d, xt_out, nt_tab, blockIdx.x, gridDim.x, sm.row_cnt));
             vmax = small_block_max(vmax, sm.red);
             if (threadIdx.x == 0 && vmax) atomicMax(&ctr->xmax_bits, vmax);
             for (uint32_t q = threadIdx.x; q < kSmallHash; q += kSmallThreads)
