@@ -822,7 +822,7 @@ cudaError_t op_sweep(pxr_handle* h) {
     });
     if (e != cudaSuccess) return e;
     phase(h, kPhScan, 1, [&] {
-        k_sweep_scan<OffT><<<tiles, kBlock, 0, s>>>(d, t, h->keys[0], h->keys[1], h->vals[0], h->vals[1]);
+        k_sweep_scan<OffT><<<scan_blocks(h->n), kBlock, 0, s>>>(d, t, h->keys[0], h->keys[1], h->vals[0], h->vals[1]);
     });
     phase(h, kPhClusterCut, 1, [&] { launch_pdl(k_cluster_cut<OffT>, grid_for(h->n), kBlock, 0, s, d, t); });
     h->sweep_tab = h->tcur;
@@ -861,7 +861,7 @@ cudaError_t op_cut(pxr_handle* h) {
                    h->ids[h->acur]);
     });
     phase(h, kPhComponents, 1, [&] {
-        launch_pdl(k_components_data<OffT>, std::min(tiles, kMaxGrid), kBlock, 0, s, d, t, h->vals[0], h->vals[1],
+        launch_pdl(k_components_data<OffT>, std::min(scan_blocks(h->n), kMaxGrid), kBlock, 0, s, d, t, h->vals[0], h->vals[1],
                                                                               h->keys[0], h->keys[1]);
     });
     // roots in vertex-id order (the order of the reference's root sort)
@@ -875,12 +875,12 @@ cudaError_t op_cut(pxr_handle* h) {
         });
     phase(h, kPhApply, 2, [&] {
         launch_pdl(k_newlab<OffT>, grid_for(h->n), kBlock, 0, s, d, t, h->ids[h->acur]);
-        launch_pdl(k_apply<OffT>, tiles, kBlock, 0, s, d, t, h->vals[0], h->vals[1], h->keys[0], h->keys[1],
+        launch_pdl(k_apply<OffT>, scan_blocks(h->n), kBlock, 0, s, d, t, h->vals[0], h->vals[1], h->keys[0], h->keys[1],
                                                h->act[h->acur ^ 1], h->par[h->acur ^ 1]);
     });
     phase(h, kPhDisable, 1, [&] {
         launch_pdl(has_long(parts) ? k_ids_disable<OffT, W, true> : k_ids_disable<OffT, W, false>,
-                   parts.heavy + parts.wide + tiles, kBlock, 0, s, d, parts, h->ids[h->acur], h->ids[h->acur ^ 1],
+                   parts.heavy + parts.wide + scan_blocks(h->n), kBlock, 0, s, d, parts, h->ids[h->acur], h->ids[h->acur ^ 1],
                    h->xt[h->xcur], nt);
     });
     phase(h, kPhCvol, 1, [&] { launch_pdl(k_cvol_scan<OffT>, tiles, kBlock, 0, s, d, nt); });

@@ -28,6 +28,27 @@ constexpr int kBlock = 256;
 #endif
 constexpr int kScanItems = 8;                        // items per thread in look-back kernels
 constexpr int kScanTile = kBlock * kScanItems;
+// Tiles of the kernels over the active vertices: kScanItems items per thread,
+// or kFineItems where whole tiles would be too few to fill the GPU (a few
+// hundred thousand active vertices leave most SMs without a block, and a block's
+// dependent loads one after another bound the kernel).  Decompositions, all
+// coarse / fine up to 2^18 / 2^20 / 3 * 2^20 items: 3D grid 41^3 7.50 / 6.57 /
+// 6.55 / 6.55 ms, 96^3 13.7 / 13.4 / 13.7 / 13.7, 128^3 22.4 / 22.1 / 22.2 /
+// 24.3; 8-regular 0.5 M vertices 8.36 / 8.14 / 8.10 / 8.08; batch of 8 instances
+// 7.40 / 6.30 / 6.28 / 6.28, of 32 32.7 / 31.9 / 31.7 / 32.8.
+constexpr int kFineItems = 2;
+constexpr int kFineTile = kBlock * kFineItems;
+#ifndef PXR_FINE_MAX
+#define PXR_FINE_MAX (1u << 19)
+#endif
+constexpr uint32_t kFineMax = PXR_FINE_MAX;
+// blocks a launch over up to n active vertices needs for either tile
+inline uint32_t scan_blocks(uint32_t n) {
+    const uint32_t coarse = (n + kScanTile - 1) / kScanTile;
+    const uint32_t fine = ((n < kFineMax ? n : kFineMax) + kFineTile - 1) / kFineTile;
+    const uint32_t b = coarse > fine ? coarse : fine;
+    return b ? b : 1u;
+}
 // k_relabel runs over the roots, often far fewer than the vertices: smaller
 // tiles keep more of its latency-bound gathers in flight
 constexpr int kRelabelItems = 2;
@@ -759,17 +780,14 @@ __device__ __forceinline__ float sweep_ratio(uint32_t num, uint32_t den, uint32_
     return __fdiv_rn((float)num, (float)den);
 }
 
-template <typename OffT>
-__global__ void __launch_bounds__(kBlock) k_sweep_scan(Dev<OffT> d, ClusterTables t, const uint64_t* keys0,
-                                                       const uint64_t* keys1, const uint32_t* vals0,
-                                                       const uint32_t* vals1) {
-    pdl_wait();
+template <int ITEMS, typename OffT>
+__device__ __forceinline__ void sweep_scan_tile(const Dev<OffT>& d, const ClusterTables& t, const uint64_t* keys0,
+                                                const uint64_t* keys1, const uint32_t* vals0, const uint32_t* vals1,
+                                                uint32_t count) {
     __shared__ uint64_t warp_tot[kBlock / 32];
     __shared__ uint64_t s_excl;
-    const uint32_t count = d.ctr->n_sweep;
-    const uint32_t ntiles = (count + kScanTile - 1) / kScanTile;
+    if (blockIdx.x >= (count + kBlock * ITEMS - 1) / (kBlock * ITEMS)) return;   // as many tiles as blocks left
     const uint32_t tile = fetch_tile(d.ctr, kSiteScan);
-    if (tile >= ntiles) return;
     const uint32_t sel = sorted_sel(d.sort);
     if (tile == 0 && threadIdx.x == 0) {
         d.ctr->main_sel = sel;
@@ -779,13 +797,13 @@ __global__ void __launch_bounds__(kBlock) k_sweep_scan(Dev<OffT> d, ClusterTable
     const uint64_t* keys = sel ? keys1 : keys0;
     const uint32_t* vals = sel ? vals1 : vals0;
     const uint32_t epoch = d.lb_epoch[kSiteScan];
-    const uint32_t first = tile * kScanTile + threadIdx.x * kScanItems;
+    const uint32_t first = tile * (kBlock * ITEMS) + threadIdx.x * ITEMS;
 
-    uint32_t lab[kScanItems];
-    uint64_t pre[kScanItems];
+    uint32_t lab[ITEMS];
+    uint64_t pre[ITEMS];
     uint64_t run = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const uint32_t i = first + k;
         uint64_t val = 0;
         lab[k] = 0;
@@ -814,7 +832,7 @@ __global__ void __launch_bounds__(kBlock) k_sweep_scan(Dev<OffT> d, ClusterTable
     unsigned long long a_first = ~0ull, a_last = ~0ull;
     ArgminAgg am{reinterpret_cast<unsigned long long*>(t.best)};
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const uint32_t i = first + k;
         if (i >= count) break;
         const uint64_t p = PairAdd::combine(texcl, pre[k]);
@@ -840,6 +858,16 @@ __global__ void __launch_bounds__(kBlock) k_sweep_scan(Dev<OffT> d, ClusterTable
         }
     }
     emit_fragments<ArgminAgg>(has, single, k_first, a_first, k_last, a_last, am);
+}
+
+template <typename OffT>
+__global__ void __launch_bounds__(kBlock) k_sweep_scan(Dev<OffT> d, ClusterTables t, const uint64_t* keys0,
+                                                       const uint64_t* keys1, const uint32_t* vals0,
+                                                       const uint32_t* vals1) {
+    pdl_wait();
+    const uint32_t count = d.ctr->n_sweep;
+    if (count <= kFineMax) sweep_scan_tile<kFineItems>(d, t, keys0, keys1, vals0, vals1, count);
+    else sweep_scan_tile<kScanItems>(d, t, keys0, keys1, vals0, vals1, count);
 }
 
 // per cluster: the best cut, the threshold test (CheckThreshold,
@@ -1195,31 +1223,28 @@ __device__ __forceinline__ void mark_root(const Dev<OffT>& d, uint32_t r) {
 }
 
 // roots, per-cluster data (computeClusterData, cuda/devPartition.h:380-411)
-template <typename OffT>
-__global__ void __launch_bounds__(kBlock) k_components_data(Dev<OffT> d, ClusterTables t, const uint32_t* vals0,
-                                                            const uint32_t* vals1, const uint64_t* keys0,
-                                                            const uint64_t* keys1) {
-    pdl_wait();
+template <int ITEMS, typename OffT>
+__device__ __forceinline__ void components_data_tiles(const Dev<OffT>& d, const ClusterTables& t, const uint32_t* vals0,
+                                                      const uint32_t* vals1, const uint64_t* keys0,
+                                                      const uint64_t* keys1, uint32_t count, uint32_t* t_keys,
+                                                      ClusterAcc* t_vals) {
     // the sorted order: a cluster's items are contiguous, so runs of one root
     // are long and the per-root atomics few
-    const uint32_t count = d.ctr->n_sweep;
     const uint32_t sel = d.ctr->main_sel;
     const uint32_t* vals = sel ? vals1 : vals0;
     const uint64_t* keys = sel ? keys1 : keys0;
     const int e = fixed_exponent(d.ctr->xmax_walk_bits, d.nb_bits);
     const double scale = pow2(e);
-    __shared__ uint32_t t_keys[kTableSlots];
-    __shared__ ClusterAcc t_vals[kTableSlots];
     const TableAgg<DataAgg> agg{{d.acc_max, d.acc_min, d.acc_sum, d.acc_cnt}, t_keys, t_vals};
-    if (blockIdx.x * kScanTile >= count) return;
+    if (blockIdx.x * (kBlock * ITEMS) >= count) return;
     agg.clear();
-    const uint32_t stride = gridDim.x * kScanTile;
-    for (uint32_t base = blockIdx.x * kScanTile; base < count; base += stride) {
-        const uint32_t first = base + threadIdx.x * kScanItems;
+    const uint32_t stride = gridDim.x * (kBlock * ITEMS);
+    for (uint32_t base = blockIdx.x * (kBlock * ITEMS); base < count; base += stride) {
+        const uint32_t first = base + threadIdx.x * ITEMS;
         bool has = false, single = true;
         uint32_t k_first = 0, k_last = 0;
         ClusterAcc a_first = DataAgg::identity(), a_last = DataAgg::identity();
-        for (int k = 0; k < kScanItems; ++k) {
+        for (int k = 0; k < ITEMS; ++k) {
             const uint32_t i = first + k;
             if (i >= count) break;
             const uint32_t c = (uint32_t)(keys[i] >> 32);
@@ -1254,6 +1279,18 @@ __global__ void __launch_bounds__(kBlock) k_components_data(Dev<OffT> d, Cluster
         emit_fragments<TableAgg<DataAgg>>(has, single, k_first, a_first, k_last, a_last, agg);
     }
     agg.flush();
+}
+
+template <typename OffT>
+__global__ void __launch_bounds__(kBlock) k_components_data(Dev<OffT> d, ClusterTables t, const uint32_t* vals0,
+                                                            const uint32_t* vals1, const uint64_t* keys0,
+                                                            const uint64_t* keys1) {
+    pdl_wait();
+    __shared__ uint32_t t_keys[kTableSlots];
+    __shared__ ClusterAcc t_vals[kTableSlots];
+    const uint32_t count = d.ctr->n_sweep;
+    if (count <= kFineMax) components_data_tiles<kFineItems>(d, t, vals0, vals1, keys0, keys1, count, t_keys, t_vals);
+    else components_data_tiles<kScanItems>(d, t, vals0, vals1, keys0, keys1, count, t_keys, t_vals);
 }
 
 // ---------------------------------------------------------------------------
@@ -1441,28 +1478,23 @@ __global__ void __launch_bounds__(kBlock) k_newlab(Dev<OffT> d, ClusterTables t,
 
 // new labels and recentering (learned schedule only), and the stable
 // compaction of the sorted order into the next round's active list.
-template <typename OffT>
-__global__ void __launch_bounds__(kBlock) k_apply(Dev<OffT> d, ClusterTables t, const uint32_t* vals0,
-                                                  const uint32_t* vals1, const uint64_t* keys0,
-                                                  const uint64_t* keys1, uint32_t* act_next, uint32_t* par_next) {
-    pdl_wait();
-    if (d.ctr->walk_only) return;   // nothing due: the round only walks
+template <int ITEMS, typename OffT>
+__device__ __forceinline__ void apply_tile(const Dev<OffT>& d, const ClusterTables& t, const uint32_t* vals0,
+                                           const uint32_t* vals1, const uint64_t* keys0, const uint64_t* keys1,
+                                           uint32_t* act_next, uint32_t* par_next, uint32_t count) {
     __shared__ uint64_t warp_tot[kBlock / 32];
     __shared__ uint64_t s_excl;
-    const uint32_t count = d.ctr->n_sweep;
-    const uint32_t ntiles = (count + kScanTile - 1) / kScanTile;
+    if (blockIdx.x >= (count + kBlock * ITEMS - 1) / (kBlock * ITEMS)) return;   // as many tiles as blocks left
     const uint32_t tile = fetch_tile(d.ctr, kSiteApply);
-    if (tile == 0 && threadIdx.x == 0) d.ctr->xmax_bits = 0;
-    if (tile >= ntiles) return;
     const uint32_t sel = d.ctr->main_sel;
     const uint32_t* vals = sel ? vals1 : vals0;
     const uint64_t* keys = sel ? keys1 : keys0;
     const uint32_t epoch = d.lb_epoch[kSiteApply];
-    const uint32_t first = tile * kScanTile + threadIdx.x * kScanItems;
-    uint32_t vv[kScanItems], cc[kScanItems];
+    const uint32_t first = tile * (kBlock * ITEMS) + threadIdx.x * ITEMS;
+    uint32_t vv[ITEMS], cc[ITEMS];
     uint32_t keepmask = 0, run = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const uint32_t i = first + k;
         vv[k] = 0;
         cc[k] = 0;
@@ -1498,12 +1530,24 @@ __global__ void __launch_bounds__(kBlock) k_apply(Dev<OffT> d, ClusterTables t, 
     __syncthreads();
     uint32_t pos = (uint32_t)(s_excl + incl - run);
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k)
+    for (int k = 0; k < ITEMS; ++k)
         if (keepmask & (1u << k)) {
             act_next[pos] = vv[k];
             par_next[pos] = cc[k];   // the cluster the vertex was swept in: runs of the next list
             ++pos;
         }
+}
+
+template <typename OffT>
+__global__ void __launch_bounds__(kBlock) k_apply(Dev<OffT> d, ClusterTables t, const uint32_t* vals0,
+                                                  const uint32_t* vals1, const uint64_t* keys0,
+                                                  const uint64_t* keys1, uint32_t* act_next, uint32_t* par_next) {
+    pdl_wait();
+    if (d.ctr->walk_only) return;   // nothing due: the round only walks
+    if (blockIdx.x == 0 && threadIdx.x == 0) d.ctr->xmax_bits = 0;
+    const uint32_t count = d.ctr->n_sweep;
+    if (count <= kFineMax) apply_tile<kFineItems>(d, t, vals0, vals1, keys0, keys1, act_next, par_next, count);
+    else apply_tile<kScanItems>(d, t, vals0, vals1, keys0, keys1, act_next, par_next, count);
 }
 
 // Returns max |x| over the rows this thread finished.
@@ -1542,38 +1586,24 @@ __device__ __forceinline__ uint32_t disable_long_rows(const Dev<OffT>& d, float*
     return vmax;
 }
 
-// next round's vertex-order list, edge disabling (disableEdgesKernel_node,
-// cuda/devPartition.h:80-146), internal degrees, x/d, cluster volumes.
-template <typename OffT, int W, bool LONG>
-__global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, RowParts parts, const uint32_t* ids,
-                                                        uint32_t* ids_next, float* xt, ClusterTables nt) {
-    pdl_wait();
-    if (d.ctr->walk_only) return;   // nothing due: the round only walks
-    uint32_t block, blocks;
-    const int part = parts.part<LONG>(&block, &blocks);
-    if (part != 2) {   // disjoint rows; the shared results (volumes, max |x|) are atomics
-        __shared__ uint32_t sh[kBlock / 32];
-        const uint32_t m = part == 0 ? disable_long_rows<OffT, kBlock>(d, xt, nt, block, blocks, sh)
-                                     : disable_long_rows<OffT, 32>(d, xt, nt, block, blocks, sh);
-        block_atomic_max(&d.ctr->xmax_bits, m);
-        return;
-    }
+// A tile of the active list in vertex order; s_list, s_hkey, s_hval: shared, a
+// tile's entries each.
+template <int ITEMS, int W, typename OffT>
+__device__ __forceinline__ void ids_disable_tile(const Dev<OffT>& d, const uint32_t* ids, uint32_t* ids_next, float* xt,
+                                                 const ClusterTables& nt, uint32_t count, uint32_t block,
+                                                 uint32_t* s_list, uint32_t* s_hkey, uint32_t* s_hval) {
     __shared__ uint64_t warp_tot[kBlock / 32];
     __shared__ uint64_t s_excl;
-    __shared__ uint32_t s_list[kScanTile];
-    __shared__ uint32_t s_hkey[kScanTile];
-    __shared__ uint32_t s_hval[kScanTile];
     __shared__ uint32_t s_n;
-    const uint32_t count = d.ctr->n_active;
-    const uint32_t ntiles = (count + kScanTile - 1) / kScanTile;
+    constexpr uint32_t kTile = kBlock * ITEMS;
+    if (block >= (count + kTile - 1) / kTile) return;   // as many tiles as blocks left
     const uint32_t tile = fetch_tile(d.ctr, kSiteIds);
-    if (tile >= ntiles) return;
     const uint32_t epoch = d.lb_epoch[kSiteIds];
-    const uint32_t first = tile * kScanTile + threadIdx.x * kScanItems;
-    uint32_t vv[kScanItems];
+    const uint32_t first = tile * kTile + threadIdx.x * ITEMS;
+    uint32_t vv[ITEMS];
     uint32_t keepmask = 0, run = 0;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k) {
+    for (int k = 0; k < ITEMS; ++k) {
         const uint32_t j = first + k;
         vv[k] = 0;
         if (j >= count) continue;
@@ -1594,7 +1624,7 @@ __global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, RowParts pa
     uint32_t lpos = (uint32_t)(incl - run);
     const uint32_t gpos = (uint32_t)s_excl;
 #pragma unroll
-    for (int k = 0; k < kScanItems; ++k)
+    for (int k = 0; k < ITEMS; ++k)
         if (keepmask & (1u << k)) {
             ids_next[gpos + lpos] = vv[k];
             s_list[lpos] = vv[k];
@@ -1603,7 +1633,7 @@ __global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, RowParts pa
     __syncthreads();
     // row pass over this tile's kept vertices, W lanes per vertex; cluster
     // volumes are summed per tile in a shared hash table keyed by label
-    for (uint32_t q = threadIdx.x; q < kScanTile; q += kBlock) { s_hkey[q] = 0xFFFFFFFFu; s_hval[q] = 0u; }
+    for (uint32_t q = threadIdx.x; q < kTile; q += kBlock) { s_hkey[q] = 0xFFFFFFFFu; s_hval[q] = 0u; }
     __syncthreads();
     const uint32_t nkept = s_n;
     const uint32_t gl = threadIdx.x & (W - 1);
@@ -1650,17 +1680,41 @@ __global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, RowParts pa
             xt[v] = deg ? __double2float_rn(__ddiv_rn((double)xv, (double)deg)) : 0.0f;
             const uint32_t b = __float_as_uint(fabsf(xv));
             vmax = b > vmax ? b : vmax;
-            uint32_t h = ((uint32_t)lv * 2654435761u) & (kScanTile - 1);
+            uint32_t h = ((uint32_t)lv * 2654435761u) & (kTile - 1);
             for (;;) {
                 const uint32_t prev = atomicCAS(&s_hkey[h], 0xFFFFFFFFu, (uint32_t)lv);
                 if (prev == 0xFFFFFFFFu || prev == (uint32_t)lv) { atomicAdd(&s_hval[h], deg); break; }
-                h = (h + 1) & (kScanTile - 1);
+                h = (h + 1) & (kTile - 1);
             }
         }
     }
     block_atomic_max(&d.ctr->xmax_bits, vmax);
-    for (uint32_t q = threadIdx.x; q < kScanTile; q += kBlock)
+    for (uint32_t q = threadIdx.x; q < kTile; q += kBlock)
         if (s_hkey[q] != 0xFFFFFFFFu && s_hval[q]) atomicAdd(&nt.vol[s_hkey[q]], s_hval[q]);
+}
+
+// next round's vertex-order list, edge disabling (disableEdgesKernel_node,
+// cuda/devPartition.h:80-146), internal degrees, x/d, cluster volumes.
+template <typename OffT, int W, bool LONG>
+__global__ void __launch_bounds__(kBlock) k_ids_disable(Dev<OffT> d, RowParts parts, const uint32_t* ids,
+                                                        uint32_t* ids_next, float* xt, ClusterTables nt) {
+    pdl_wait();
+    if (d.ctr->walk_only) return;   // nothing due: the round only walks
+    uint32_t block, blocks;
+    const int part = parts.part<LONG>(&block, &blocks);
+    if (part != 2) {   // disjoint rows; the shared results (volumes, max |x|) are atomics
+        __shared__ uint32_t sh[kBlock / 32];
+        const uint32_t m = part == 0 ? disable_long_rows<OffT, kBlock>(d, xt, nt, block, blocks, sh)
+                                     : disable_long_rows<OffT, 32>(d, xt, nt, block, blocks, sh);
+        block_atomic_max(&d.ctr->xmax_bits, m);
+        return;
+    }
+    __shared__ uint32_t s_list[kScanTile];
+    __shared__ uint32_t s_hkey[kScanTile];
+    __shared__ uint32_t s_hval[kScanTile];
+    const uint32_t count = d.ctr->n_active;
+    if (count <= kFineMax) ids_disable_tile<kFineItems, W>(d, ids, ids_next, xt, nt, count, block, s_list, s_hkey, s_hval);
+    else ids_disable_tile<kScanItems, W>(d, ids, ids_next, xt, nt, count, block, s_list, s_hkey, s_hval);
 }
 
 // exclusive prefix of cluster volumes over labels

@@ -1,5 +1,5 @@
-"""The one-kernel decomposition of small graphs (graph driver, plain form)
-against the CPU oracle: sizes around a warp's, a CTA's and a cluster's share
+"""The one-kernel decomposition of small graphs (graph driver, plain form) and
+the general path's tile sizes against the CPU oracle: sizes around a warp's, a CTA's and a cluster's share
 of vertices, rows in every bin, many clusters from the start, and a run
 stopped at its round cap and continued by the general path."""
 import numpy as np
@@ -18,6 +18,10 @@ def _edges(n, e):
     e = np.asarray(e, dtype=np.int64).reshape(-1, 2)
     return G.csr_from_edges(e[:, 0], e[:, 1], n)
 
+
+# active vertices around the general path's switch of tile sizes (2^19), which the
+# run crosses as clusters are certified
+LARGE = {"grid81": lambda: G.grid3d(81), "grid80": lambda: G.grid3d(80)}
 
 SHAPES = {
     "path": lambda: _edges(5000, [(i, i + 1) for i in range(4999)]),
@@ -61,6 +65,12 @@ def test_sizes_match_the_oracle(n):
 @pytest.mark.parametrize("name", sorted(SHAPES))
 def test_shapes_match_the_oracle(name):
     dm, orc = _loaded(SHAPES[name]())
+    _check(dm, orc, dm.expanderDecomposition())
+
+
+@pytest.mark.parametrize("name", sorted(LARGE))
+def test_tile_sizes_of_the_general_path(name):
+    dm, orc = _loaded(LARGE[name]())
     _check(dm, orc, dm.expanderDecomposition())
 
 
