@@ -731,37 +731,47 @@ void launch_walk(pxr_handle* h, const Dev<OffT>& d, cudaStream_t s, const float*
                xt_out);
 }
 
+// in_round: part of a whole round, whose preparation and end op_round launches
 template <typename OffT, int W>
 cudaError_t op_walk(pxr_handle* h, bool in_round = false) {
     Dev<OffT> d = make_dev<OffT>(h);
     cudaStream_t s = h->stream;
     hold_for_profiling(h);
-    phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, s, d, 0, kNoCond, kNoCond); });
+    if (!in_round)
+        phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, s, d, (int)kPrepWalk, kNoCond, kNoCond); });
     phase(h, kPhWalk, 1, [&] { launch_walk<OffT, W>(h, d, s, h->xt[h->xcur], h->xt[h->xcur ^ 1]); });
     // the next walk's fixed-point scale follows max |x'|; inside a plain round
-    // the cut stage recomputes it over the recentred potentials anyway
-    if (!in_round || h->sched.mode) phase(h, kPhBook, 1, [&] { launch_pdl(k_after_walk<OffT>, 1, 1, 0, s, d); });
+    // the cut stage recomputes it over the recentred potentials anyway, inside a
+    // learned one k_walk_only_check takes it over
+    if (!in_round) phase(h, kPhBook, 1, [&] { launch_pdl(k_after_walk<OffT>, 1, 1, 0, s, d); });
     h->xcur ^= 1;
     return cudaGetLastError();
 }
 
+// The two sorts' IF nodes of a round being captured (plain form): a round
+// launches only the sort it uses.
+struct SortConds {
+    cudaGraphConditionalHandle gsort = 0, chunk = 0;
+};
+cudaError_t make_sort_conds(pxr_handle* h, SortConds* c) {
+    if (h->sched.mode) return cudaSuccess;
+    if (cudaGraph_t g = capture_graph(h)) {
+        PXR_TRY(cudaGraphConditionalHandleCreate(&c->gsort, g, 1u, cudaGraphCondAssignDefault));
+        PXR_TRY(cudaGraphConditionalHandleCreate(&c->chunk, g, 1u, cudaGraphCondAssignDefault));
+        h->sort_regions = true;
+    }
+    return cudaSuccess;
+}
+
 template <typename OffT, int W>
-cudaError_t op_sweep(pxr_handle* h) {
+cudaError_t op_sweep(pxr_handle* h, bool in_round = false, const SortConds& conds = {}) {
     Dev<OffT> d = make_dev<OffT>(h);
     cudaStream_t s = h->stream;
     const ClusterTables& t = h->tab[h->tcur];
     hold_for_profiling(h);
-    // graph driver, plain form: the global sort and the chunked sort become
-    // IF nodes, so a round launches only the sort it uses
-    cudaGraphConditionalHandle c_gsort = 0, c_chunk = 0;
-    if (!h->sched.mode) {
-        if (cudaGraph_t g = capture_graph(h)) {
-            PXR_TRY(cudaGraphConditionalHandleCreate(&c_gsort, g, 1u, cudaGraphCondAssignDefault));
-            PXR_TRY(cudaGraphConditionalHandleCreate(&c_chunk, g, 1u, cudaGraphCondAssignDefault));
-            h->sort_regions = true;
-        }
-    }
-    phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, s, d, 1, c_gsort, c_chunk); });
+    const cudaGraphConditionalHandle c_gsort = conds.gsort, c_chunk = conds.chunk;
+    if (!in_round)
+        phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, s, d, (int)kPrepSweep, kNoCond, kNoCond); });
     const uint32_t tiles = std::max((h->n + kScanTile - 1) / kScanTile, 1u);
     const RowParts parts = row_parts(h);
     const uint32_t row_grid = parts.heavy + parts.wide + grid_for((uint64_t)h->n * W);
@@ -769,7 +779,7 @@ cudaError_t op_sweep(pxr_handle* h) {
         phase(h, kPhSched, 3, [&] {
             launch_pdl(k_cluster_spread<OffT>, std::min(tiles, kMaxGrid), kBlock, 0, s, d, h->ids[h->acur]);
             launch_pdl(k_due_scan<OffT>, tiles, kBlock, 0, s, d, t);
-            launch_pdl(k_walk_only_check<OffT>, 1, 1, 0, s, d);
+            launch_pdl(k_walk_only_check<OffT>, 1, 1, 0, s, d, in_round);
         });
     // learned schedule: the sweep set is compacted first and the edge
     // differences are taken over it alone (carried clusters need none)
@@ -784,9 +794,12 @@ cudaError_t op_sweep(pxr_handle* h) {
         phase(h, kPhNodeDiff, 1, [&] {
             launch_pdl(has_long(parts) ? k_nodediff<OffT, W, true> : k_nodediff<OffT, W, false>, row_grid, kBlock, 0, s, d, parts, h->ids[h->acur], (const uint32_t*)nullptr);
         });
-        phase(h, kPhEmit, 1, [&] {
-            launch_pdl(k_emit<OffT>, grid_for(h->n), kBlock, 0, s, d, h->act[h->acur], h->keys[0], h->vals[0], t.best);
-        });
+        // in a captured round the keys are part of the global sort's IF node
+        // (the tables' argmin words start reset: k_relabel, k_loop_begin)
+        if (!c_gsort)
+            phase(h, kPhEmit, 1, [&] {
+                launch_pdl(k_emit<OffT>, grid_for(h->n), kBlock, 0, s, d, h->act[h->acur], h->keys[0], h->vals[0], t.best);
+            });
     }
     SortBuffers<uint64_t> b{};
     b.keys[0] = h->keys[0]; b.keys[1] = h->keys[1];
@@ -806,9 +819,11 @@ cudaError_t op_sweep(pxr_handle* h) {
         run_gsort = chunk_path == 0;
         run_chunk = chunk_path != 0;
     }
-    phase(h, kPhSort, (run_gsort ? kGsortLaunches : 0) + (run_chunk ? 1 : 0), [&] {
+    phase(h, kPhSort, (run_gsort ? kGsortLaunches + (c_gsort ? 1 : 0) : 0) + (run_chunk ? 1 : 0), [&] {
         if (run_gsort)
             e = if_region(h, c_gsort, [&](cudaStream_t st) {
+                if (c_gsort)
+                    k_emit<OffT><<<grid_for(h->n), kBlock, 0, st>>>(d, h->act[h->acur], h->keys[0], h->vals[0], t.best);
                 return radix_sort<uint64_t>(b, h->sort, &h->ctr->err, st, 64, (int)h->sort_info.plan);
             });
         // the chunked sort writes buffer 0, which round preparation selects
@@ -824,13 +839,18 @@ cudaError_t op_sweep(pxr_handle* h) {
     phase(h, kPhScan, 1, [&] {
         k_sweep_scan<OffT><<<scan_blocks(h->n), kBlock, 0, s>>>(d, t, h->keys[0], h->keys[1], h->vals[0], h->vals[1]);
     });
-    phase(h, kPhClusterCut, 1, [&] { launch_pdl(k_cluster_cut<OffT>, grid_for(h->n), kBlock, 0, s, d, t); });
+    if (in_round)
+        phase(h, kPhClusterCut, 1, [&] {
+            launch_pdl(k_cut<OffT>, grid_for(h->n), kBlock, 0, s, d, t, h->vals[0], h->vals[1], h->keys[0], h->keys[1]);
+        });
+    else
+        phase(h, kPhClusterCut, 1, [&] { launch_pdl(k_cluster_cut<OffT>, grid_for(h->n), kBlock, 0, s, d, t); });
     h->sweep_tab = h->tcur;
     return cudaGetLastError();
 }
 
 template <typename OffT, int W>
-cudaError_t op_cut(pxr_handle* h) {
+cudaError_t op_cut(pxr_handle* h, bool in_round = false) {
     Dev<OffT> d = make_dev<OffT>(h);
     cudaStream_t s = h->stream;
     const ClusterTables& t = h->tab[h->tcur];
@@ -838,14 +858,15 @@ cudaError_t op_cut(pxr_handle* h) {
     const uint32_t tiles = std::max((h->n + kScanTile - 1) / kScanTile, 1u);
     const RowParts parts = row_parts(h);
     hold_for_profiling(h);
-    phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, s, d, 2, kNoCond, kNoCond); });
+    if (!in_round)
+        phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, s, d, (int)kPrepCut, kNoCond, kNoCond); });
     if (h->sched.mode)
         phase(h, kPhSched, 2, [&] {
             launch_pdl(k_carry_all<OffT>, grid_for(h->n), kBlock, 0, s, d, t, nt, h->act[h->acur], h->act[h->acur ^ 1],
                                                                  h->ids[h->acur], h->ids[h->acur ^ 1]);
             launch_pdl(k_carry_roots<OffT>, grid_for(h->n), kBlock, 0, s, d, t);
         });
-    phase(h, kPhCutInit, 1, [&] {
+    if (!in_round) phase(h, kPhCutInit, 1, [&] {
         launch_pdl(k_cut_init<OffT>, grid_for(h->n), kBlock, 0, s, d, t, h->vals[0], h->vals[1], h->keys[0], h->keys[1]);
     });
     phase(h, kPhUnion, 3 + (d.union_sampled ? 3 : 0), [&] {
@@ -886,28 +907,50 @@ cudaError_t op_cut(pxr_handle* h) {
     phase(h, kPhCvol, 1, [&] { launch_pdl(k_cvol_scan<OffT>, tiles, kBlock, 0, s, d, nt); });
     if (h->sched.mode || d.trace)
         phase(h, kPhSched, 1, [&] { launch_pdl(k_schedule<OffT>, std::min(grid_for(h->n), 148u * 8u), kBlock, 0, s, d, t, nt); });
-    phase(h, kPhBook, 1, [&] { launch_pdl(k_round_end<OffT>, 1, 1, 0, s, d); });
+    if (!in_round) phase(h, kPhBook, 1, [&] { launch_pdl(k_round_end<OffT>, 1, 1, 0, s, d); });
     h->tcur ^= 1;
     h->acur ^= 1;
     return cudaGetLastError();
 }
 
 template <typename OffT, int W>
-cudaError_t op_round(pxr_handle* h) {
+cudaError_t op_round_stages(pxr_handle* h, const SortConds& conds) {
     cudaError_t e = op_walk<OffT, W>(h, true);
-    if (e == cudaSuccess) e = op_sweep<OffT, W>(h);
-    if (e == cudaSuccess) e = op_cut<OffT, W>(h);
+    if (e == cudaSuccess) e = op_sweep<OffT, W>(h, true, conds);
+    if (e == cudaSuccess) e = op_cut<OffT, W>(h, true);
     return e;
 }
 
-// two rounds (the parities return to their start) and the loop condition
+template <typename OffT, int W>
+cudaError_t op_round(pxr_handle* h) {
+    Dev<OffT> d = make_dev<OffT>(h);
+    phase(h, kPhBook, 1, [&] { launch_pdl(k_round_prep<OffT>, 1, 32, 0, h->stream, d, (int)kPrepRound, kNoCond, kNoCond); });
+    const cudaError_t e = op_round_stages<OffT, W>(h, {});
+    if (e != cudaSuccess) return e;
+    phase(h, kPhBook, 1, [&] { launch_pdl(k_round_end<OffT>, 1, 1, 0, h->stream, d); });
+    return cudaGetLastError();
+}
+
+// Two rounds (the parities return to their start) and the loop condition.
+// One bookkeeping kernel stands between rounds and one at either end; each is
+// a launch of 2-3 us on the round's chain (nine of them took 1.3 of the 22 ms
+// of the 128^3 grid).
 template <typename OffT, int W>
 cudaError_t op_loop_body(pxr_handle* h, cudaGraphConditionalHandle cond) {
-    cudaError_t e = op_round<OffT, W>(h);
-    if (e == cudaSuccess) e = op_round<OffT, W>(h);
-    if (e != cudaSuccess) return e;
     Dev<OffT> d = make_dev<OffT>(h);
-    phase(h, kPhBook, 1, [&] { launch_pdl(k_loop_cond<OffT>, 1, 1, 0, h->stream, d, cond); });
+    SortConds conds[2];
+    for (SortConds& c : conds) PXR_TRY(make_sort_conds(h, &c));
+    phase(h, kPhBook, 1, [&] {
+        launch_pdl(k_round_prep<OffT>, 1, 32, 0, h->stream, d, (int)kPrepRound, conds[0].gsort, conds[0].chunk);
+    });
+    cudaError_t e = op_round_stages<OffT, W>(h, conds[0]);
+    if (e != cudaSuccess) return e;
+    phase(h, kPhBook, 1, [&] {
+        launch_pdl(k_round_next<OffT>, 1, 32, 0, h->stream, d, conds[1].gsort, conds[1].chunk);
+    });
+    e = op_round_stages<OffT, W>(h, conds[1]);
+    if (e != cudaSuccess) return e;
+    phase(h, kPhBook, 1, [&] { launch_pdl(k_loop_end<OffT>, 1, 1, 0, h->stream, d, cond); });
     return cudaGetLastError();
 }
 
@@ -1005,9 +1048,16 @@ pxr_status build_loop_graph(pxr_handle* h, int key) {
     return PXR_OK;
 }
 
-__global__ void k_loop_begin(RoundCtr* c, uint32_t cap) {
-    c->loop_start = c->rounds;
-    c->loop_cap = cap;
+// The loop's bounds, and the argmin words of the clusters it starts from (a
+// sweep called by itself leaves them set; the rounds' own are reset as they are
+// made).
+__global__ void k_loop_begin(RoundCtr* c, uint32_t cap, uint64_t* best) {
+    const uint32_t k = c->n_clusters;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) best[i] = ~0ull;
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        c->loop_start = c->rounds;
+        c->loop_cap = cap;
+    }
 }
 
 // CTAs of the small-graph kernel for the loaded graph, or 0 when the general
@@ -1105,7 +1155,8 @@ pxr_status decompose_graph(pxr_handle* h) {
         pxr_status st = build_loop_graph(h, key);
         if (st != PXR_OK) return st;
     }
-    k_loop_begin<<<1, 1, 0, h->stream>>>(h->ctr, h->cfg.max_rounds);
+    k_loop_begin<<<std::min(grid_for(std::max(h->h_ctr->n_clusters, 1u)), 148u), kBlock, 0, h->stream>>>(
+        h->ctr, h->cfg.max_rounds, h->tab[h->tcur].best);
     PXR_CUDA(h, cudaGetLastError());
     const uint32_t before = h->h_ctr->rounds;
     const uint64_t g0 = h->h_ctr->stat_gsort_slots, c0 = h->h_ctr->stat_chunk_slots;
@@ -1117,7 +1168,7 @@ pxr_status decompose_graph(pxr_handle* h) {
     const uint64_t iters = std::max<uint64_t>(1, (ran + 1) / 2);
     if (h->body_regions[key]) {
         const uint64_t dg = h->h_ctr->stat_gsort_slots - g0, dc = h->h_ctr->stat_chunk_slots - c0;
-        h->launches += 1 + iters * (h->body_launches[key] - 2 * (kGsortLaunches + 1)) + dg * kGsortLaunches + dc;
+        h->launches += 1 + iters * (h->body_launches[key] - 2 * (kGsortLaunches + 2)) + dg * (kGsortLaunches + 1) + dc;
     } else {
         h->launches += 1 + h->body_launches[key] * iters;
     }

@@ -234,14 +234,16 @@ __device__ __forceinline__ uint32_t stream_col(const uint32_t* p) { return __ldc
 // ---------------------------------------------------------------------------
 // round bookkeeping
 
-// stage: 0 before the walk, 1 before the sweep, 2 before the cut
-// In the graph driver, the global sort and the chunked sort of stage 1 sit
+// Before a stage (kPrepWalk, kPrepSweep, kPrepCut: the stages called one by
+// one) or before a whole round (all three at once: every counter that a stage
+// starts from zero is only touched in that stage and read by the round's end).
+// In the graph driver, the global sort and the chunked sort of the sweep sit
 // under two IF nodes whose conditions (gsort, chunk) are set here.
+enum : int { kPrepWalk = 1, kPrepSweep = 2, kPrepCut = 4, kPrepRound = 7 };
+
 template <typename OffT>
-__global__ void k_round_prep(Dev<OffT> d, int stage, cudaGraphConditionalHandle gsort = 0,
-                             cudaGraphConditionalHandle chunk = 0) {
-    pdl_wait();
-    pdl_launch_next();
+__device__ __forceinline__ void round_prep(const Dev<OffT>& d, int stages, cudaGraphConditionalHandle gsort,
+                                           cudaGraphConditionalHandle chunk) {
     RoundCtr* c = d.ctr;
     // one warp: lane i resets look-back site i, lane 0 does the rest (the
     // sites' dependent read-modify-writes in one thread took ~4 us)
@@ -251,23 +253,23 @@ __global__ void k_round_prep(Dev<OffT> d, int stage, cudaGraphConditionalHandle 
         d.lb_epoch[lane] += 1;
     }
     if (lane != 0) return;
-    if (stage == 2) c->n_cut_swept = c->n_cut;   // the sweep's count, read by the cut stage
+    c->n_cut_swept = stages == kPrepCut ? c->n_cut : 0u;   // the sweep's count, read by the cut stage
     c->n_cut = 0;
     c->n_roots = 0;
-    if (stage == 0) {
+    if (stages & kPrepWalk) {
         c->xmax_walk_bits = 0;
         c->walk_only = 0;
     }
     c->smallest_next = 0;
     c->n_keep = 0;
     c->n_active_next = 0;
-    if (stage == 1) {
+    if (stages & kPrepSweep) {
         c->n_due_items = 0;
         c->any_split = 0;
         if (d.sched) c->n_sweep = 0;   // set by k_due_scan
     }
     if (!d.sched) c->n_sweep = c->n_active;
-    if (stage == 1) {
+    if (stages & kPrepSweep) {
         // every previous cluster fits a chunk: sort in shared memory (pxr_chunk.cuh)
         c->chunk_path = (!d.sched && c->max_parent <= kChunkCapRows && c->n_active > 0) ? 1u : 0u;
         c->n_gsort = c->chunk_path ? 0u : c->n_sweep;
@@ -284,9 +286,17 @@ __global__ void k_round_prep(Dev<OffT> d, int stage, cudaGraphConditionalHandle 
             if (c->chunk_path) c->stat_chunk_slots += 1; else c->stat_gsort_slots += 1;
         }
     }
-    if (stage == 2) c->max_csize_next = 0;
+    if (stages & kPrepCut) c->max_csize_next = 0;
     const uint32_t k = c->n_clusters;
     *d.sort_end_bit = 32u + bitlen(k > 0 ? k - 1 : 0);
+}
+
+template <typename OffT>
+__global__ void k_round_prep(Dev<OffT> d, int stages, cudaGraphConditionalHandle gsort = 0,
+                             cudaGraphConditionalHandle chunk = 0) {
+    pdl_wait();
+    pdl_launch_next();
+    round_prep(d, stages, gsort, chunk);
 }
 
 template <typename OffT>
@@ -297,9 +307,7 @@ __global__ void k_after_walk(Dev<OffT> d) {
 }
 
 template <typename OffT>
-__global__ void k_round_end(Dev<OffT> d) {
-    pdl_wait();
-    pdl_launch_next();
+__device__ __forceinline__ void round_end(const Dev<OffT>& d) {
     RoundCtr* c = d.ctr;
     if (c->n_active > 0) {
         c->rounds += 1;
@@ -313,13 +321,33 @@ __global__ void k_round_end(Dev<OffT> d) {
     c->n_clusters = c->n_keep;
     c->smallest = c->smallest_next;
     c->full_components = 0;
+    c->n_cut = 0;
     c->done = (c->n_active == 0 || c->n_clusters == 0) ? 1u : 0u;
 }
 
-// device-driven round loop: keep looping while clusters remain and the cap allows
 template <typename OffT>
-__global__ void k_loop_cond(Dev<OffT> d, cudaGraphConditionalHandle cond) {
+__global__ void k_round_end(Dev<OffT> d) {
     pdl_wait();
+    pdl_launch_next();
+    round_end(d);
+}
+
+// a round's end and the preparation of the one after it
+template <typename OffT>
+__global__ void k_round_next(Dev<OffT> d, cudaGraphConditionalHandle gsort, cudaGraphConditionalHandle chunk) {
+    pdl_wait();
+    pdl_launch_next();
+    if (threadIdx.x == 0) round_end(d);
+    __syncwarp();
+    round_prep(d, kPrepRound, gsort, chunk);
+}
+
+// A round's end in the device-driven loop: keep looping while clusters remain
+// and the cap allows.
+template <typename OffT>
+__global__ void k_loop_end(Dev<OffT> d, cudaGraphConditionalHandle cond) {
+    pdl_wait();
+    round_end(d);
     const RoundCtr* c = d.ctr;
     const bool more = !c->done && c->err == 0 && (c->rounds - c->loop_start) < c->loop_cap;
     cudaGraphSetConditional(cond, more ? 1u : 0u);
@@ -873,9 +901,7 @@ __global__ void __launch_bounds__(kBlock) k_sweep_scan(Dev<OffT> d, ClusterTable
 // per cluster: the best cut, the threshold test (CheckThreshold,
 // cuda/devSweepCut.h:321-331, 701-709) and the components plan.
 template <typename OffT>
-__global__ void __launch_bounds__(kBlock) k_cluster_cut(Dev<OffT> d, ClusterTables t) {
-    pdl_wait();
-    if (d.ctr->walk_only) return;   // nothing due: the round only walks
+__device__ __forceinline__ void cut_clusters(const Dev<OffT>& d, const ClusterTables& t) {
     const uint32_t k = d.ctr->n_clusters;
     const uint32_t full = d.ctr->full_components;
     pxr_sweep_cut* cuts = reinterpret_cast<pxr_sweep_cut*>(d.allcuts);
@@ -910,6 +936,13 @@ __global__ void __launch_bounds__(kBlock) k_cluster_cut(Dev<OffT> d, ClusterTabl
     }
 }
 
+template <typename OffT>
+__global__ void __launch_bounds__(kBlock) k_cluster_cut(Dev<OffT> d, ClusterTables t) {
+    pdl_wait();
+    if (d.ctr->walk_only) return;   // nothing due: the round only walks
+    cut_clusters(d, t);
+}
+
 // ---------------------------------------------------------------------------
 // cut (PartitionManager::cutClusters, cuda/devPartition.h:545-622): in a cut
 // cluster, positions past the chosen prefix take a fresh label; every vertex
@@ -932,6 +965,31 @@ __global__ void __launch_bounds__(kBlock) k_cut_init(Dev<OffT> d, ClusterTables 
         const uint32_t co = d.cut_off[c];
         const uint32_t pos = i - t.start[c] + 1u;
         d.lab[v] = (co != kNoCut && pos > co) ? (int32_t)(k + c) : (int32_t)c;
+    }
+}
+
+// Both of the above in one launch (whole rounds): an item reads its cluster's
+// decision from the sweep's argmin itself instead of waiting for it in a table.
+template <typename OffT>
+__global__ void __launch_bounds__(kBlock) k_cut(Dev<OffT> d, ClusterTables t, const uint32_t* vals0,
+                                                const uint32_t* vals1, const uint64_t* keys0, const uint64_t* keys1) {
+    pdl_wait();
+    if (d.ctr->walk_only) return;   // nothing due: the round only walks
+    cut_clusters(d, t);
+    const uint32_t count = d.ctr->n_sweep;
+    const uint32_t k = d.ctr->n_clusters;
+    const uint32_t full = d.ctr->full_components;
+    const uint32_t sel = d.ctr->main_sel;
+    const uint32_t* vals = sel ? vals1 : vals0;
+    const uint64_t* keys = sel ? keys1 : keys0;
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+        const uint32_t c = (uint32_t)(keys[i] >> 32);
+        const uint32_t fl = d.sched ? d.sflag[c] : 3u;
+        if (!(fl & 1u)) continue;   // swept for the audit only
+        const uint64_t b = t.best[c];
+        const bool cut = (fl & 2u) && __uint_as_float((uint32_t)(b >> 32)) < d.sc_threshold;
+        // ~position of the chosen prefix's last item
+        if (cut || full) d.lab[vals[i]] = (cut && i > ~(uint32_t)b) ? (int32_t)(k + c) : (int32_t)c;
     }
 }
 

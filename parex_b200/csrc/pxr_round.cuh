@@ -148,11 +148,13 @@ enum : int {
 __device__ __forceinline__ uint32_t bitlen(uint32_t v) { return v ? 32u - __clz(v) : 0u; }
 
 // Learned schedule: this round cut more than cut_gate x its clusters, so the
-// next round sweeps every cluster (read after the cut, before the round ends).
+// next round sweeps every cluster (read after the cut, before the round ends;
+// the count is in n_cut, or in n_cut_swept once a cut stage called by itself
+// has begun).
 template <typename OffT>
 __device__ __forceinline__ bool cut_gate_on(const Dev<OffT>& d) {
     return d.cut_gate > 0.0f &&
-           __uint2float_rn(d.ctr->n_cut_swept) > __fmul_rn(d.cut_gate, __uint2float_rn(d.ctr->n_clusters));
+           __uint2float_rn(d.ctr->n_cut_swept + d.ctr->n_cut) > __fmul_rn(d.cut_gate, __uint2float_rn(d.ctr->n_clusters));
 }
 
 // Learned schedule: the next round's skip sk of a cluster of `size`

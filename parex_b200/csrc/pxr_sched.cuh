@@ -210,8 +210,9 @@ __global__ void __launch_bounds__(kBlock) k_emit_sched(Dev<OffT> d, const uint32
 
 // After the due scan: a round in which no cluster is due only walks.
 template <typename OffT>
-__global__ void k_walk_only_check(Dev<OffT> d) {
+__global__ void k_walk_only_check(Dev<OffT> d, bool after_walk) {
     pdl_wait();
+    if (after_walk) d.ctr->xmax_bits = d.ctr->xmax_walk_bits;   // the next walk's scale, as k_after_walk
     d.ctr->walk_only = (d.ctr->n_sweep == 0 && d.ctr->n_active > 0) ? 1u : 0u;
 }
 
