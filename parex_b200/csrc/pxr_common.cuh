@@ -56,6 +56,7 @@ struct RoundCtr {
     uint32_t sweep_k;         // clusters of the last sweep
     uint32_t loop_start;      // rounds at the start of the device-driven loop
     uint32_t loop_cap;        // round cap of the device-driven loop
+    uint32_t loop_take;       // active vertices at which it hands over to the small-graph kernel
     uint32_t n_sweep;         // vertices in this round's sweep (all active ones in the plain form)
     uint32_t n_due_items;     // vertices of the clusters swept and acted on this round
     uint32_t chunk_path;      // this round's sort runs chunk by chunk in shared memory

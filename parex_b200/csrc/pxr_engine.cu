@@ -1051,32 +1051,54 @@ pxr_status build_loop_graph(pxr_handle* h, int key) {
 // The loop's bounds, and the argmin words of the clusters it starts from (a
 // sweep called by itself leaves them set; the rounds' own are reset as they are
 // made).
-__global__ void k_loop_begin(RoundCtr* c, uint32_t cap, uint64_t* best) {
+__global__ void k_loop_begin(RoundCtr* c, uint32_t cap, uint32_t take, uint64_t* best) {
     const uint32_t k = c->n_clusters;
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < k; i += gridDim.x * blockDim.x) best[i] = ~0ull;
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         c->loop_start = c->rounds;
         c->loop_cap = cap;
+        c->loop_take = take;
     }
 }
 
-// CTAs of the small-graph kernel for the loaded graph, or 0 when the general
-// path takes it (the measurements are at kSmallMaxSlots).
-uint32_t small_cluster(const pxr_handle* h) {
-    if (h->sched.mode || h->sched.trace || h->n == 0 || h->slots > kSmallMaxSlots) return 0;
-    const uint32_t need = (h->n + kSmallTile - 1) / kSmallTile;
-    uint32_t ctas = 1;
-    while (ctas < need || (ctas < h->small_ctas && (h->n > ctas * kSmallVerticesPerCta ||
-                                                    h->slots > (uint64_t)ctas * kSmallSlotsPerCta)))
-        ctas <<= 1;
-    return ctas <= h->small_ctas ? ctas : 0u;
+// Largest active set that k_small_decompose takes on the loaded graph, 0: none
+// (the measurements are at kSmallMaxSlots).  Its stages look through the whole
+// lists of long rows, so those of a graph that is not small itself must be few.
+uint32_t small_take(const pxr_handle* h) {
+    if (h->sched.mode || h->sched.trace || h->n == 0) return 0;
+    const uint64_t by_slots = (uint64_t)kSmallMaxSlots * h->n / std::max<uint64_t>(h->slots, 1);
+    const uint32_t take = (uint32_t)std::min<uint64_t>(by_slots, h->small_ctas * kSmallTile);
+    return h->n <= take || h->n_wide + h->n_heavy <= kSmallLongRows ? take : 0u;
 }
 
+// CTAs for `active` vertices (at most small_take).
+uint32_t small_cluster(const pxr_handle* h, uint32_t active) {
+    const uint64_t slots = h->slots * (uint64_t)active / std::max(h->n, 1u);
+    uint32_t ctas = 1;
+    while (ctas * kSmallTile < active || (ctas < h->small_ctas && (active > ctas * kSmallVerticesPerCta ||
+                                                                  slots > (uint64_t)ctas * kSmallSlotsPerCta)))
+        ctas <<= 1;
+    return ctas;
+}
+
+// Light rows of the small-graph kernel: up to 64 slots, 128 where the mean row
+// is above 32.  The tuner times plans on the whole GPU, where they differ by a
+// hair on a small graph (R-MAT 14, mean 26: 3.6 ms at 64, 4.3 at a tuned 128;
+// planted partition of mean degree 63: 3.4 at 64, 2.9 at 128).
+uint32_t small_light(const pxr_handle* h) { return h->slots > 32ull * h->n ? 128u : 64u; }
+
 template <typename OffT>
-cudaError_t launch_small(pxr_handle* h, uint32_t ctas) {
+cudaError_t launch_small(pxr_handle* h, uint32_t ctas, uint32_t max_rounds) {
     SmallArgs<OffT> a{};
     a.d = make_dev<OffT>(h);
     a.d.union_sampled = 0;
+    // light rows go by the mean degree here whatever the tuned plan.  The list is
+    // ordered by length, so the longer rows are a prefix of it.
+    const uint32_t light = small_light(h);
+    if (!h->plan_forced && h->wide_max >= light && (h->maxdeg <= light || (h->long_built && h->long_above <= light))) {
+        a.d.light_max = light;
+        a.d.n_wide = h->rows_above[light] - h->n_heavy;
+    }
     for (int i = 0; i < 2; ++i) {
         a.tab[i] = h->tab[i];
         a.act[i] = h->act[i];
@@ -1089,7 +1111,7 @@ cudaError_t launch_small(pxr_handle* h, uint32_t ctas) {
     a.xcur = h->xcur;
     a.tcur = h->tcur;
     a.acur = h->acur;
-    a.max_rounds = h->cfg.max_rounds;
+    a.max_rounds = max_rounds;
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = ctas;
     cfg.blockDim = kSmallThreads;
@@ -1135,9 +1157,10 @@ uint32_t prepare_small() {
     return 0;
 }
 
-pxr_status decompose_small(pxr_handle* h, uint32_t ctas) {
+pxr_status decompose_small(pxr_handle* h, uint32_t max_rounds) {
     const uint32_t before = h->h_ctr->rounds;
-    PXR_CUDA(h, h->off64 ? launch_small<uint64_t>(h, ctas) : launch_small<uint32_t>(h, ctas));
+    const uint32_t ctas = small_cluster(h, h->h_ctr->n_active);
+    PXR_CUDA(h, h->off64 ? launch_small<uint64_t>(h, ctas, max_rounds) : launch_small<uint32_t>(h, ctas, max_rounds));
     ++h->launches;
     const pxr_status st = sync_ctr(h);
     const uint32_t ran = h->h_ctr->rounds - before;
@@ -1149,14 +1172,15 @@ pxr_status decompose_small(pxr_handle* h, uint32_t ctas) {
 }
 
 pxr_status decompose_graph(pxr_handle* h) {
-    if (const uint32_t ctas = small_cluster(h)) return decompose_small(h, ctas);
+    const uint32_t take = small_take(h);
+    if (take && h->h_ctr->n_active <= take) return decompose_small(h, h->cfg.max_rounds);
     const int key = h->xcur | (h->tcur << 1) | (h->acur << 2);
     if (!h->graphs[key]) {
         pxr_status st = build_loop_graph(h, key);
         if (st != PXR_OK) return st;
     }
     k_loop_begin<<<std::min(grid_for(std::max(h->h_ctr->n_clusters, 1u)), 148u), kBlock, 0, h->stream>>>(
-        h->ctr, h->cfg.max_rounds, h->tab[h->tcur].best);
+        h->ctr, h->cfg.max_rounds, take, h->tab[h->tcur].best);
     PXR_CUDA(h, cudaGetLastError());
     const uint32_t before = h->h_ctr->rounds;
     const uint64_t g0 = h->h_ctr->stat_gsort_slots, c0 = h->h_ctr->stat_chunk_slots;
@@ -1172,6 +1196,9 @@ pxr_status decompose_graph(pxr_handle* h) {
     } else {
         h->launches += 1 + h->body_launches[key] * iters;
     }
+    // the loop ends early once the small-graph kernel can take the rest over
+    if (st == PXR_OK && !h->h_ctr->done && ran < h->cfg.max_rounds && h->h_ctr->n_active <= take)
+        return decompose_small(h, h->cfg.max_rounds - ran);
     return st;
 }
 
@@ -1518,8 +1545,10 @@ pxr_status choose_row_plan(pxr_handle* h, bool reuse, uint32_t nb_bits) {
             g_plan_cache[key] = plan;
         }
     }
-    if (h->n > 0 && h->maxdeg > plan.light_max) {
-        pxr_status bst = build_long_rows<OffT>(h, plan.light_max);
+    // a small graph's list goes down to the small-graph kernel's own bound
+    const uint32_t listed = h->n <= h->small_ctas * kSmallTile ? std::min(plan.light_max, small_light(h)) : plan.light_max;
+    if (h->n > 0 && h->maxdeg > listed) {
+        pxr_status bst = build_long_rows<OffT>(h, listed);
         if (bst == PXR_OK) bst = count_rows<OffT>(h, plan.light_max, plan.wide_max);
         if (bst != PXR_OK) return bst;
     }

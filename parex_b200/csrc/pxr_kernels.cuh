@@ -342,14 +342,15 @@ __global__ void k_round_next(Dev<OffT> d, cudaGraphConditionalHandle gsort, cuda
     round_prep(d, kPrepRound, gsort, chunk);
 }
 
-// A round's end in the device-driven loop: keep looping while clusters remain
-// and the cap allows.
+// A round's end in the device-driven loop: keep looping while clusters remain,
+// the cap allows, and the active set is too large for the small-graph kernel.
 template <typename OffT>
 __global__ void k_loop_end(Dev<OffT> d, cudaGraphConditionalHandle cond) {
     pdl_wait();
     round_end(d);
     const RoundCtr* c = d.ctr;
-    const bool more = !c->done && c->err == 0 && (c->rounds - c->loop_start) < c->loop_cap;
+    const bool more = !c->done && c->err == 0 && (c->rounds - c->loop_start) < c->loop_cap &&
+                      c->n_active > c->loop_take;
     cudaGraphSetConditional(cond, more ? 1u : 0u);
 }
 

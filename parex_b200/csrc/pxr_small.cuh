@@ -1,4 +1,5 @@
-// A whole plain decomposition of a small graph in one kernel (sm_100a).
+// The plain rounds of a small active set in one kernel (sm_100a): whole
+// decompositions of small graphs, and the last rounds of larger ones.
 //
 // A round of the general path is about 23 launches.  On a graph of a few
 // thousand vertices each of them is one or a few busy blocks walking a chain
@@ -25,11 +26,11 @@ namespace pxr {
 
 constexpr int kSmallThreads = 1024;
 constexpr int kSmallWarps = kSmallThreads / 32;
-constexpr uint32_t kSmallTile = 2 * kSmallThreads;   // sorted items of a CTA, and vertices it owns in the scans
+constexpr uint32_t kSmallTile = 2 * kSmallThreads;   // sorted items of a CTA, and list positions it owns in the scans
 constexpr uint32_t kSmallMaxCtas = 16;               // the largest (opt-in) cluster
-// Which graphs take this kernel: those whose vertices fit the tiles of the
-// largest cluster, up to kSmallMaxSlots edge slots (a cluster is 16 of 148
-// SMs, so long row passes go to the whole GPU).  Measured, whole decomposition
+// Which active sets take this kernel: those whose vertices fit the tiles of the
+// largest cluster, up to kSmallMaxSlots edge slots at the graph's mean degree (a
+// cluster is 16 of 148 SMs, so long row passes go to the whole GPU).  Measured, whole decomposition
 // on a B200, here / general path in a graph: planted partition 2,048 vertices
 // 1.54 / 4.42 ms, 8,192 2.09 / 5.94, 16,384 2.80 / 6.98, 32,000 (0.67 M slots)
 // 3.90 / 6.22; 16,000 vertices and 1.0 M slots 2.87 / 5.64; 3D grid 31^3
@@ -42,6 +43,7 @@ constexpr uint32_t kSmallMaxSlots = 1u << 20;
 // 3.24, 2.42, 2.08 ms).
 constexpr uint32_t kSmallVerticesPerCta = 256;
 constexpr uint32_t kSmallSlotsPerCta = 8192;
+constexpr uint32_t kSmallLongRows = 2048;   // rows above light_max of a larger graph
 constexpr uint32_t kSmallHash = 2 * kSmallTile;      // cluster volumes of a CTA's rescanned rows
 
 struct SmallShared {
@@ -255,7 +257,6 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
     uint32_t max_parent = 0xFFFFFFFFu, max_csize = d.n;   // the list at entry has no known runs
     bool err = ctr->err != 0;
     unsigned long long st_v = 0, st_s = 0, st_g = 0, st_items = 0;
-    const uint32_t own = (d.n + gridDim.x - 1) / gridDim.x;   // <= kSmallTile vertices per CTA in the root scan
     small_sync();   // everyone has read the counters
     if (gid == 0) {
         ctr->xmax_walk_bits = 0;
@@ -586,13 +587,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
                     const uint32_t c = lab[j], v = vtx[j];
                     if (d.split[c]) {
                         r = uf_find_flat(d.parent, v);
-                        if (r == v) {
-                            mark_root(d, r);
-                            d.rootc[r] = (kOriginChild << 30) | c;
-                        }
+                        if (r == v) d.rootc[r] = (kOriginChild << 30) | c;
                     } else {
                         r = t.root[c];
-                        if (ifirst + j == t.start[c]) mark_root(d, r);
                     }
                     const float xv = d.x[v];
                     const uint32_t ob = ordered_bits(xv);
@@ -618,8 +615,9 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
         }
         small_sync();
 
-        // ---- roots in vertex order: index, dense label and start of each (two vertices a thread)
-        const uint32_t v0 = blockIdx.x * own, vend = min(d.n, v0 + own), vfirst = v0 + 2u * threadIdx.x;
+        // ---- the active list in vertex order: every vertex's root, and the roots'
+        // index, dense label and start
+        uint32_t idv[2], idc[2], idr[2];
         uint32_t rcnt[2];   // kept cluster: its size; 0: dropped
         uint32_t rinfo[2], rvol[2];
         double rsum[2];
@@ -627,9 +625,16 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
         uint64_t rrun = 0;  // roots | kept << 20 | kept vertices << 40
 #pragma unroll
         for (uint32_t j = 0; j < 2; ++j) {
-            const uint32_t v = vfirst + j;
-            root[j] = v < vend && ((d.rootmap[v >> 5] >> (v & 31u)) & 1u);
+            root[j] = false;
             rcnt[j] = 0;
+            idv[j] = 0;
+            if (j >= ipt || ifirst + j >= iend) continue;
+            const uint32_t v = ids[ifirst + j];
+            const uint32_t lv = (uint32_t)d.lab[v];
+            idv[j] = v;
+            idc[j] = lv >= k ? lv - k : lv;
+            idr[j] = d.split[idc[j]] ? ld_relaxed(&d.parent[v]) : t.root[idc[j]];
+            root[j] = idr[j] == v;
             if (root[j]) {
                 const uint32_t cnt = d.acc_cnt[v];
                 const float pot = __fsub_rn(from_ordered_bits(d.acc_max[v]), from_ordered_bits(d.acc_min[v]));
@@ -653,8 +658,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
             if (lane == 0 && biggest) atomicMax(&ctr->max_csize_next, biggest);
 #pragma unroll
             for (uint32_t j = 0; j < 2; ++j) {
-                const uint32_t r = vfirst + j;
-                if (r < vend && (r & 31u) == 0) d.rootmap[r >> 5] = 0u;   // zero again for the next round
+                const uint32_t r = idv[j];
                 if (!root[j]) continue;
                 if (rcnt[j]) {
                     const uint32_t nl = (uint32_t)(p >> 20) & 0xFFFFFu;
@@ -681,19 +685,14 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
         small_sync();
 
         // ---- new labels, recentring, certificates (vertex order); both lists' survivors counted
-        uint32_t idv[2], keep_a = 0, keep_b = 0;
+        uint32_t keep_a = 0, keep_b = 0;
 #pragma unroll
         for (uint32_t j = 0; j < 2; ++j) {
-            idv[j] = 0;
             if (j >= ipt || ifirst + j >= iend) continue;
-            const uint32_t c0s = lab[j];
-            const uint32_t rs = d.split[c0s] ? ld_relaxed(&d.parent[vtx[j]]) : t.root[c0s];
+            const uint32_t cs = lab[j];
+            const uint32_t rs = d.split[cs] ? ld_relaxed(&d.parent[vtx[j]]) : t.root[cs];
             if (d.newlab[rs] >= 0) keep_a |= 1u << j;
-            const uint32_t v = ids[ifirst + j];
-            idv[j] = v;
-            const uint32_t lv = (uint32_t)d.lab[v];
-            const uint32_t c = lv >= k ? lv - k : lv;
-            const uint32_t r = d.split[c] ? ld_relaxed(&d.parent[v]) : t.root[c];
+            const uint32_t v = idv[j], c = idc[j], r = idr[j];
             const int32_t nl = d.newlab[r];
             d.lab[v] = nl;
             if (nl >= 0) {
