@@ -4,9 +4,9 @@
 // The active list is in the previous round's sort order with deactivated
 // vertices removed, so the vertices of each previous-round cluster (a
 // "parent") form one contiguous run of it, and every cluster of this round
-// lies inside one parent's run.  When every parent holds at most kChunkCap
-// vertices, CTA k takes the parents whose run starts in
-// [k * kChunk, (k + 1) * kChunk) - at most kChunk + kChunkCap - 1 items -
+// lies inside one parent's run.  When every parent holds at most CAP
+// vertices, chunk k takes the parents whose run starts in
+// [k * ROWS, (k + 1) * ROWS) - at most ROWS + CAP - 1 items -
 // sorts them stably by (label, potential) with an LSD radix sort in shared
 // memory, and writes every cluster to its start position from the cluster
 // tables.  The result is the global stable sort's, item for item: the same
@@ -18,27 +18,36 @@
 
 namespace pxr {
 
-constexpr uint32_t kChunk = 4096;
-constexpr uint32_t kChunkCap = kChunkCapRows;
-constexpr uint32_t kChunkItems = kChunk + kChunkCap;
-constexpr int kChunkThreads = 512;
-constexpr int kChunkIPT = kChunkItems / kChunkThreads;   // 16 items per thread
-constexpr int kChunkWarps = kChunkThreads / 32;
-constexpr uint32_t kChunkSlots = 16384;                  // label hash table (in the second key buffer)
+// A chunk's shape: ROWS list positions whose parents it takes, CAP the longest
+// parent, THREADS a CTA's threads.
+template <uint32_t ROWS, uint32_t CAP, int THREADS>
+struct ChunkShape {
+    static constexpr uint32_t kRows = ROWS;
+    static constexpr uint32_t kItems = ROWS + CAP;
+    static constexpr int kThreads = THREADS;
+    static constexpr int kIpt = (int)kItems / THREADS;      // items per thread
+    static constexpr int kWarps = THREADS / 32;
+    static constexpr uint32_t kSlots = 2 * kItems;          // label hash table (in the second key buffer)
+    static constexpr size_t kSmem = 2 * kItems * sizeof(uint64_t) + 2 * kItems * sizeof(uint32_t) +
+                                    kWarps * 256 * sizeof(uint32_t);
+};
+// One CTA per SM while clusters of thousands of vertices remain; then chunks of
+// a quarter of the size, three CTAs per SM: what bounds a chunk is its own chain
+// of gathers, scans and barriers (36 us whatever the list's length), so several
+// per SM hide it (sorts of the 128^3 grid 5.6 -> 5.0 ms, its decomposition 20.6 ->
+// 19.8; 64^3 7.1 -> 6.8; two or four CTAs per SM within 1 %).
+using LargeChunk = ChunkShape<4096, kChunkCapRows, 512>;
+using SmallChunk = ChunkShape<1024, kChunkCapSmall, 256>;
 // Direct ranking (comparisons within a parent run) is used when no parent
 // run of the chunk is longer than this.
 constexpr uint32_t kCountRun = 512;
 
-constexpr size_t chunk_sort_smem() {
-    return 2 * kChunkItems * sizeof(uint64_t) + 2 * kChunkItems * sizeof(uint32_t) +
-           kChunkWarps * 256 * sizeof(uint32_t);
-}
-
 // first p >= p0 where a parent run starts (p == 0, or the parent changes), else n
+template <class C>
 __device__ __forceinline__ uint32_t chunk_boundary(const uint32_t* par, uint32_t p0, uint32_t n, uint32_t* s_min) {
     if (p0 == 0) return 0;
     if (p0 >= n) return n;
-    for (uint32_t base = p0; base < n; base += kChunkThreads) {
+    for (uint32_t base = p0; base < n; base += C::kThreads) {
         if (threadIdx.x == 0) *s_min = n;
         __syncthreads();
         const uint32_t p = base + threadIdx.x;
@@ -51,36 +60,23 @@ __device__ __forceinline__ uint32_t chunk_boundary(const uint32_t* par, uint32_t
     return n;
 }
 
-// block sum over kChunkThreads threads (valid in every thread)
-__device__ __forceinline__ uint32_t chunk_block_sum(uint32_t v, uint32_t* sh) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xFFFFFFFFu, v, o);
-    __syncthreads();
-    if ((threadIdx.x & 31u) == 0) sh[threadIdx.x >> 5] = v;
-    __syncthreads();
-    uint32_t t = 0;
-    for (int w = 0; w < kChunkWarps; ++w) t += sh[w];
-    __syncthreads();
-    return t;
-}
-
 // One stable LSD pass over cnt items (8-bit digit at `shift`), src -> dst.
+template <class C>
 __device__ __forceinline__ void chunk_pass(const uint64_t* sk, const uint32_t* sv, uint64_t* dk, uint32_t* dv,
-                                           uint32_t cnt, int shift, uint32_t (*whist)[256], uint32_t* tpre,
-                                           uint32_t* sh) {
+                                           uint32_t cnt, int shift, uint32_t (*whist)[256], uint32_t* tpre) {
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
     const uint32_t lt = lanemask_lt();
     for (int i = lane; i < 256; i += 32) whist[warp][i] = 0;
     __syncwarp();
-    const uint32_t base = warp * (32 * kChunkIPT);
-    uint32_t dg[kChunkIPT], rank[kChunkIPT];
+    const uint32_t base = warp * (32 * C::kIpt);
+    uint32_t dg[C::kIpt], rank[C::kIpt];
 #pragma unroll
-    for (int k = 0; k < kChunkIPT; ++k) {
+    for (int k = 0; k < C::kIpt; ++k) {
         const uint32_t j = base + k * 32 + lane;
         dg[k] = j < cnt ? ((uint32_t)(sk[j] >> shift) & 0xFFu) : 0x100u;
     }
 #pragma unroll
-    for (int k = 0; k < kChunkIPT; ++k) {
+    for (int k = 0; k < C::kIpt; ++k) {
         const bool valid = dg[k] < 0x100u;
         const uint32_t peers = __match_any_sync(0xFFFFFFFFu, dg[k]);
         // the lowest lane of each digit reads and advances the warp's count
@@ -100,7 +96,7 @@ __device__ __forceinline__ void chunk_pass(const uint64_t* sk, const uint32_t* s
         const uint32_t d = threadIdx.x;
         uint32_t tot = 0;
 #pragma unroll
-        for (int w = 0; w < kChunkWarps; ++w) {
+        for (int w = 0; w < C::kWarps; ++w) {
             const uint32_t c = whist[w][d];
             whist[w][d] = tot;
             tot += c;
@@ -124,7 +120,7 @@ __device__ __forceinline__ void chunk_pass(const uint64_t* sk, const uint32_t* s
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < kChunkIPT; ++k) {
+    for (int k = 0; k < C::kIpt; ++k) {
         const uint32_t j = base + k * 32 + lane;
         if (dg[k] < 0x100u) {
             const uint32_t pos = tpre[dg[k]] + whist[warp][dg[k]] + rank[k];
@@ -133,10 +129,9 @@ __device__ __forceinline__ void chunk_pass(const uint64_t* sk, const uint32_t* s
         }
     }
     __syncthreads();
-    (void)sh;
 }
 
-template <typename OffT>
+template <class C, typename OffT>
 __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTables& t, const uint32_t* act,
                                           const uint32_t* par, uint64_t* keys_out, uint32_t* vals_out, uint32_t lo,
                                           uint32_t n, uint64_t* ka, uint64_t* kb, uint32_t* va, uint32_t* vb,
@@ -146,26 +141,25 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     uint32_t& s_and = *s_and_p;
     uint32_t& s_or = *s_or_p;
     uint32_t* table = reinterpret_cast<uint32_t*>(kb);   // label hash table until the first pass
-    const uint32_t begin = chunk_boundary(par, lo, n, &s_min);
-    const uint32_t end = chunk_boundary(par, lo + kChunk, n, &s_min);
+    const uint32_t begin = chunk_boundary<C>(par, lo, n, &s_min);
+    const uint32_t end = chunk_boundary<C>(par, lo + C::kRows, n, &s_min);
     if (begin >= end) return;
     const uint32_t cnt = end - begin;
-    if (cnt > kChunkItems) {   // a parent longer than kChunkCap: the path was chosen wrongly
+    if (cnt > C::kItems) {   // a parent longer than the shape's cap: the path was chosen wrongly
         if (threadIdx.x == 0) atomicOr(&d.ctr->err, kErrLabelRange);
         return;
     }
-    for (uint32_t q = threadIdx.x; q < kChunkSlots; q += kChunkThreads) table[q] = 0xFFFFFFFFu;
     if (threadIdx.x == 0) { s_and = 0xFFFFFFFFu; s_or = 0u; }
     // gathers: every load of a thread in flight together
-    uint32_t v[kChunkIPT], L[kChunkIPT], xo[kChunkIPT];
+    uint32_t v[C::kIpt], L[C::kIpt], xo[C::kIpt];
 #pragma unroll
-    for (int r = 0; r < kChunkIPT; ++r) {
-        const uint32_t j = threadIdx.x + r * kChunkThreads;
+    for (int r = 0; r < C::kIpt; ++r) {
+        const uint32_t j = threadIdx.x + r * C::kThreads;
         v[r] = j < cnt ? act[begin + j] : 0u;
     }
 #pragma unroll
-    for (int r = 0; r < kChunkIPT; ++r) {
-        const uint32_t j = threadIdx.x + r * kChunkThreads;
+    for (int r = 0; r < C::kIpt; ++r) {
+        const uint32_t j = threadIdx.x + r * C::kThreads;
         L[r] = j < cnt ? (uint32_t)d.lab[v[r]] : 0u;
         xo[r] = j < cnt ? ordered_bits(d.x[v[r]]) : 0u;
     }
@@ -173,8 +167,8 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     // run with the same label (earlier by potential, ties by list position),
     // which is its place in the stable sort.  Work: sum of squared run lengths.
 #pragma unroll
-    for (int r = 0; r < kChunkIPT; ++r) {
-        const uint32_t j = threadIdx.x + r * kChunkThreads;
+    for (int r = 0; r < C::kIpt; ++r) {
+        const uint32_t j = threadIdx.x + r * C::kThreads;
         if (j < cnt) {
             ka[j] = ((uint64_t)L[r] << 32) | xo[r];
             va[j] = v[r];
@@ -184,18 +178,18 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     __syncthreads();
     // parent runs by block scans over a contiguous layout (16 items per thread):
     // run start = last head at or before i, run end = first head after i
-    const uint32_t c0 = threadIdx.x * kChunkIPT;
-    uint32_t rs[kChunkIPT], re[kChunkIPT];
+    const uint32_t c0 = threadIdx.x * C::kIpt;
+    uint32_t rs[C::kIpt], re[C::kIpt];
     uint32_t last = 0;
 #pragma unroll
-    for (int k = 0; k < kChunkIPT; ++k) {
+    for (int k = 0; k < C::kIpt; ++k) {
         const uint32_t i = c0 + k;
         if (i < cnt && (i == 0 || vb[i] != vb[i - 1])) last = i;
         rs[k] = last;
     }
     uint32_t first = cnt;   // first head after this thread's items, from the right
 #pragma unroll
-    for (int k = kChunkIPT - 1; k >= 0; --k) {
+    for (int k = C::kIpt - 1; k >= 0; --k) {
         const uint32_t i = c0 + k;
         re[k] = first;
         if (i < cnt && (i == 0 || vb[i] != vb[i - 1])) first = i;
@@ -218,10 +212,10 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     uint32_t after_min = __shfl_down_sync(0xFFFFFFFFu, mn, 1);
     if ((threadIdx.x & 31u) == 31u) after_min = cnt;
     for (uint32_t w = 0; w < (threadIdx.x >> 5); ++w) before_max = max(before_max, tpre[w]);
-    for (uint32_t w = (threadIdx.x >> 5) + 1; w < (uint32_t)kChunkWarps; ++w) after_min = min(after_min, tpre[32 + w]);
+    for (uint32_t w = (threadIdx.x >> 5) + 1; w < (uint32_t)C::kWarps; ++w) after_min = min(after_min, tpre[32 + w]);
     uint32_t longest = 0;
 #pragma unroll
-    for (int k = 0; k < kChunkIPT; ++k) {
+    for (int k = 0; k < C::kIpt; ++k) {
         const uint32_t i = c0 + k;
         rs[k] = max(rs[k], before_max);
         if (i >= cnt) continue;
@@ -234,21 +228,21 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     if ((threadIdx.x & 31u) == 0) sh[threadIdx.x >> 5] = longest;
     __syncthreads();
     uint32_t run_max = 0;
-    for (int w = 0; w < kChunkWarps; ++w) run_max = max(run_max, sh[w]);
+    for (int w = 0; w < C::kWarps; ++w) run_max = max(run_max, sh[w]);
     __syncthreads();
     if (run_max <= kCountRun) {
         // run bounds to shared memory (the second key buffer is free on this
         // path), then neighbouring lanes rank neighbouring items: the lanes
         // of a warp read the same run, so the reads are broadcasts
         uint32_t* srs = reinterpret_cast<uint32_t*>(kb);
-        uint32_t* sre = srs + kChunkItems;
+        uint32_t* sre = srs + C::kItems;
 #pragma unroll
-        for (int k = 0; k < kChunkIPT; ++k)
+        for (int k = 0; k < C::kIpt; ++k)
             if (c0 + k < cnt) { srs[c0 + k] = rs[k]; sre[c0 + k] = re[k]; }
         __syncthreads();
 #pragma unroll 1
-        for (int k = 0; k < kChunkIPT; ++k) {
-            const uint32_t i = threadIdx.x + k * kChunkThreads;
+        for (int k = 0; k < C::kIpt; ++k) {
+            const uint32_t i = threadIdx.x + k * C::kThreads;
             if (i >= cnt) break;
             const uint64_t ki = ka[i];
             const uint32_t li = (uint32_t)(ki >> 32), xi = (uint32_t)ki;
@@ -265,15 +259,16 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
         }
         return;
     }
+    for (uint32_t q = threadIdx.x; q < C::kSlots; q += C::kThreads) table[q] = 0xFFFFFFFFu;
     __syncthreads();
     // local cluster slot: the label's place in a hash table (injective; the
     // order of clusters inside a chunk is irrelevant, positions come from
     // the cluster starts)
-    uint32_t slot[kChunkIPT];
+    uint32_t slot[C::kIpt];
     uint32_t a = 0xFFFFFFFFu, o = 0u;
 #pragma unroll
-    for (int r = 0; r < kChunkIPT; ++r) {
-        const uint32_t j = threadIdx.x + r * kChunkThreads;
+    for (int r = 0; r < C::kIpt; ++r) {
+        const uint32_t j = threadIdx.x + r * C::kThreads;
         const bool valid = j < cnt;
         if (valid) {
             a &= xo[r];
@@ -284,12 +279,12 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
         const uint32_t key = valid ? L[r] : 0xFFFFFFFFu;
         const uint32_t peers = __match_any_sync(0xFFFFFFFFu, key);
         const int leader = __ffs(peers) - 1;
-        uint32_t h = (key * 2654435761u) >> 18;   // 14 bits
+        uint32_t h = ((key * 2654435761u) >> 16) & (C::kSlots - 1);
         if (valid && (int)(threadIdx.x & 31u) == leader) {
-            for (uint32_t probe = 0; probe < kChunkSlots; ++probe) {
+            for (uint32_t probe = 0; probe < C::kSlots; ++probe) {
                 const uint32_t prev = atomicCAS(&table[h], 0xFFFFFFFFu, key);
                 if (prev == 0xFFFFFFFFu || prev == key) break;
-                h = (h + 1) & (kChunkSlots - 1);
+                h = (h + 1) & (C::kSlots - 1);
             }
         }
         slot[r] = __shfl_sync(0xFFFFFFFFu, h, leader);
@@ -302,10 +297,10 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     if ((threadIdx.x & 31u) == 0) { atomicAnd(&s_and, a); atomicOr(&s_or, o); }
     __syncthreads();
     // dense local ids: rank of the occupied slots (32 slots per thread)
-    uint32_t occ = 0, mine[kChunkSlots / kChunkThreads];
+    uint32_t occ = 0, mine[C::kSlots / C::kThreads];
 #pragma unroll
-    for (int q = 0; q < (int)(kChunkSlots / kChunkThreads); ++q) {
-        mine[q] = table[threadIdx.x * (kChunkSlots / kChunkThreads) + q] != 0xFFFFFFFFu ? 1u : 0u;
+    for (int q = 0; q < (int)(C::kSlots / C::kThreads); ++q) {
+        mine[q] = table[threadIdx.x * (C::kSlots / C::kThreads) + q] != 0xFFFFFFFFu ? 1u : 0u;
         occ += mine[q];
     }
     uint32_t inc = occ;
@@ -317,23 +312,23 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     if ((threadIdx.x & 31u) == 31u) sh[threadIdx.x >> 5] = inc;
     __syncthreads();
     uint32_t wbase = 0, distinct = 0;
-    for (int w = 0; w < kChunkWarps; ++w) {
+    for (int w = 0; w < C::kWarps; ++w) {
         if (w < (int)(threadIdx.x >> 5)) wbase += sh[w];
         distinct += sh[w];
     }
     __syncthreads();
     uint32_t rk = wbase + inc - occ;
 #pragma unroll
-    for (int q = 0; q < (int)(kChunkSlots / kChunkThreads); ++q) {
+    for (int q = 0; q < (int)(C::kSlots / C::kThreads); ++q) {
         // the slot's dense id replaces its label (each thread rewrites only its own slots)
-        const uint32_t idx = threadIdx.x * (kChunkSlots / kChunkThreads) + q;
+        const uint32_t idx = threadIdx.x * (C::kSlots / C::kThreads) + q;
         table[idx] = mine[q] ? rk : 0u;
         rk += mine[q];
     }
     __syncthreads();
 #pragma unroll
-    for (int r = 0; r < kChunkIPT; ++r) {
-        const uint32_t j = threadIdx.x + r * kChunkThreads;
+    for (int r = 0; r < C::kIpt; ++r) {
+        const uint32_t j = threadIdx.x + r * C::kThreads;
         if (j < cnt) {
             ka[j] = ((uint64_t)table[slot[r]] << 32) | xo[r];
             va[j] = v[r];
@@ -347,15 +342,15 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     uint32_t *sv = va, *dv = vb;
     for (int shift = 0; shift < 32 + id_bits; shift += 8) {
         if (shift < 32 && ((varying >> shift) & 0xFFu) == 0u) continue;
-        chunk_pass(sk, sv, dk, dv, cnt, shift, whist, tpre, sh);
+        chunk_pass<C>(sk, sv, dk, dv, cnt, shift, whist, tpre);
         uint64_t* tk = sk; sk = dk; dk = tk;
         uint32_t* tv = sv; sv = dv; dv = tv;
     }
     // write out: position = cluster start + index inside the cluster's run
-    const uint32_t q0 = threadIdx.x * kChunkIPT;
+    const uint32_t q0 = threadIdx.x * C::kIpt;
     uint32_t head = 0;   // last run start at or before this thread's items
 #pragma unroll
-    for (int k = 0; k < kChunkIPT; ++k) {
+    for (int k = 0; k < C::kIpt; ++k) {
         const uint32_t q = q0 + k;
         if (q < cnt && (q == 0 || (sk[q] >> 32) != (sk[q - 1] >> 32))) head = q;
     }
@@ -372,16 +367,16 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     uint32_t prev = __shfl_up_sync(0xFFFFFFFFu, hinc, 1);
     if ((threadIdx.x & 31u) == 0) prev = 0;
     uint32_t run = max(carry, prev);
-    uint32_t vv[kChunkIPT], LL[kChunkIPT];
+    uint32_t vv[C::kIpt], LL[C::kIpt];
 #pragma unroll
-    for (int k = 0; k < kChunkIPT; ++k) {
+    for (int k = 0; k < C::kIpt; ++k) {
         const uint32_t q = q0 + k;
         vv[k] = q < cnt ? sv[q] : 0u;
     }
 #pragma unroll
-    for (int k = 0; k < kChunkIPT; ++k) LL[k] = q0 + k < cnt ? (uint32_t)d.lab[vv[k]] : 0u;
+    for (int k = 0; k < C::kIpt; ++k) LL[k] = q0 + k < cnt ? (uint32_t)d.lab[vv[k]] : 0u;
 #pragma unroll
-    for (int k = 0; k < kChunkIPT; ++k) {
+    for (int k = 0; k < C::kIpt; ++k) {
         const uint32_t q = q0 + k;
         if (q >= cnt) break;
         const uint64_t key = sk[q];
@@ -392,25 +387,26 @@ __device__ __forceinline__ void chunk_one(const Dev<OffT>& d, const ClusterTable
     }
 }
 
-template <typename OffT>
-__global__ void __launch_bounds__(kChunkThreads, 1) k_chunk_sort(Dev<OffT> d, ClusterTables t, const uint32_t* act,
-                                                                 const uint32_t* par, uint64_t* keys_out,
-                                                                 uint32_t* vals_out) {
+// path: the value of RoundCtr::chunk_path this shape serves
+template <class C, int CTAS, typename OffT>
+__global__ void __launch_bounds__(C::kThreads, CTAS) k_chunk_sort(Dev<OffT> d, ClusterTables t, const uint32_t* act,
+                                                                  const uint32_t* par, uint64_t* keys_out,
+                                                                  uint32_t* vals_out, uint32_t path) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     uint64_t* ka = reinterpret_cast<uint64_t*>(smem_raw);
-    uint64_t* kb = ka + kChunkItems;
-    uint32_t* va = reinterpret_cast<uint32_t*>(kb + kChunkItems);
-    uint32_t* vb = va + kChunkItems;
-    uint32_t (*whist)[256] = reinterpret_cast<uint32_t (*)[256]>(vb + kChunkItems);
+    uint64_t* kb = ka + C::kItems;
+    uint32_t* va = reinterpret_cast<uint32_t*>(kb + C::kItems);
+    uint32_t* vb = va + C::kItems;
+    uint32_t (*whist)[256] = reinterpret_cast<uint32_t (*)[256]>(vb + C::kItems);
     __shared__ uint32_t tpre[256];
-    __shared__ uint32_t sh[kChunkWarps];
+    __shared__ uint32_t sh[C::kWarps];
     __shared__ uint32_t s_min, s_and, s_or;
 
-    if (!d.ctr->chunk_path) return;
+    if (d.ctr->chunk_path != path) return;
     const uint32_t n = d.ctr->n_active;
-    for (uint32_t chunk = blockIdx.x; chunk * kChunk < n; chunk += gridDim.x) {
-        chunk_one(d, t, act, par, keys_out, vals_out, chunk * kChunk, n, ka, kb, va, vb, whist, tpre, sh, &s_min,
-                  &s_and, &s_or);
+    for (uint32_t chunk = blockIdx.x; chunk * C::kRows < n; chunk += gridDim.x) {
+        chunk_one<C>(d, t, act, par, keys_out, vals_out, chunk * C::kRows, n, ka, kb, va, vb, whist, tpre, sh, &s_min,
+                     &s_and, &s_or);
         __syncthreads();
     }
 }

@@ -59,7 +59,7 @@ struct RoundCtr {
     uint32_t loop_take;       // active vertices at which it hands over to the small-graph kernel
     uint32_t n_sweep;         // vertices in this round's sweep (all active ones in the plain form)
     uint32_t n_due_items;     // vertices of the clusters swept and acted on this round
-    uint32_t chunk_path;      // this round's sort runs chunk by chunk in shared memory
+    uint32_t chunk_path;      // this round's sort runs chunk by chunk in shared memory: 1 large, 2 small chunks
     uint32_t n_gsort;         // items of the global sort (0 on the chunk path)
     uint32_t max_parent;      // largest cluster of the previous round (bounds the active list's runs)
     uint32_t max_csize;       // largest cluster of this round

@@ -681,6 +681,9 @@ constexpr cudaGraphConditionalHandle kNoCond = 0;   // round preparation outside
 
 // kernels of the global sort (histogram, plan, 8 digit passes)
 constexpr uint64_t kGsortLaunches = 2 + kMaxPasses;
+// kernels of the chunked sort (one per chunk shape)
+constexpr uint64_t kChunkLaunches = 2;
+constexpr uint32_t kSmallChunkCtas = 3;
 
 // The graph being captured on h->stream, or null outside capture.
 cudaGraph_t capture_graph(pxr_handle* h) {
@@ -819,7 +822,7 @@ cudaError_t op_sweep(pxr_handle* h, bool in_round = false, const SortConds& cond
         run_gsort = chunk_path == 0;
         run_chunk = chunk_path != 0;
     }
-    phase(h, kPhSort, (run_gsort ? kGsortLaunches + (c_gsort ? 1 : 0) : 0) + (run_chunk ? 1 : 0), [&] {
+    phase(h, kPhSort, (run_gsort ? kGsortLaunches + (c_gsort ? 1 : 0) : 0) + (run_chunk ? kChunkLaunches : 0), [&] {
         if (run_gsort)
             e = if_region(h, c_gsort, [&](cudaStream_t st) {
                 if (c_gsort)
@@ -829,9 +832,13 @@ cudaError_t op_sweep(pxr_handle* h, bool in_round = false, const SortConds& cond
         // the chunked sort writes buffer 0, which round preparation selects
         if (e == cudaSuccess && run_chunk)
             e = if_region(h, c_chunk, [&](cudaStream_t st) {
-                k_chunk_sort<OffT><<<std::min(std::max((h->n + kChunk - 1) / kChunk, 1u), 148u), kChunkThreads,
-                                     chunk_sort_smem(), st>>>(d, t, h->act[h->acur], h->par[h->acur], h->keys[0],
-                                                              h->vals[0]);
+                k_chunk_sort<LargeChunk, 1, OffT>
+                    <<<std::min((h->n + LargeChunk::kRows - 1) / LargeChunk::kRows, 148u), LargeChunk::kThreads,
+                       LargeChunk::kSmem, st>>>(d, t, h->act[h->acur], h->par[h->acur], h->keys[0], h->vals[0], 1u);
+                k_chunk_sort<SmallChunk, kSmallChunkCtas, OffT>
+                    <<<std::min((h->n + SmallChunk::kRows - 1) / SmallChunk::kRows, 148u * kSmallChunkCtas),
+                       SmallChunk::kThreads, SmallChunk::kSmem, st>>>(d, t, h->act[h->acur], h->par[h->acur],
+                                                                      h->keys[0], h->vals[0], 2u);
                 return cudaGetLastError();
             });
     });
@@ -1157,6 +1164,14 @@ uint32_t prepare_small() {
     return 0;
 }
 
+template <typename OffT>
+void prepare_chunk_sort() {
+    cudaFuncSetAttribute(k_chunk_sort<LargeChunk, 1, OffT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)LargeChunk::kSmem);
+    cudaFuncSetAttribute(k_chunk_sort<SmallChunk, kSmallChunkCtas, OffT>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                         (int)SmallChunk::kSmem);
+}
+
 pxr_status decompose_small(pxr_handle* h, uint32_t max_rounds) {
     const uint32_t before = h->h_ctr->rounds;
     const uint32_t ctas = small_cluster(h, h->h_ctr->n_active);
@@ -1192,7 +1207,8 @@ pxr_status decompose_graph(pxr_handle* h) {
     const uint64_t iters = std::max<uint64_t>(1, (ran + 1) / 2);
     if (h->body_regions[key]) {
         const uint64_t dg = h->h_ctr->stat_gsort_slots - g0, dc = h->h_ctr->stat_chunk_slots - c0;
-        h->launches += 1 + iters * (h->body_launches[key] - 2 * (kGsortLaunches + 2)) + dg * (kGsortLaunches + 1) + dc;
+        h->launches += 1 + iters * (h->body_launches[key] - 2 * (kGsortLaunches + 1 + kChunkLaunches)) +
+                       dg * (kGsortLaunches + 1) + dc * kChunkLaunches;
     } else {
         h->launches += 1 + h->body_launches[key] * iters;
     }
@@ -1843,10 +1859,8 @@ pxr_status pxr_create(const pxr_config* cfg, pxr_handle** out) {
         if (!attrs_set[h->device]) {
             radix_sort_prepare<uint64_t>();
             radix_sort_prepare<uint32_t>();
-            cudaFuncSetAttribute(k_chunk_sort<uint32_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)chunk_sort_smem());
-            cudaFuncSetAttribute(k_chunk_sort<uint64_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)chunk_sort_smem());
+            prepare_chunk_sort<uint32_t>();
+            prepare_chunk_sort<uint64_t>();
             small_ctas[h->device] = std::min(prepare_small<uint32_t>(), prepare_small<uint64_t>());
             attrs_set[h->device] = true;
         }

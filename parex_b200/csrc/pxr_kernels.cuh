@@ -271,7 +271,9 @@ __device__ __forceinline__ void round_prep(const Dev<OffT>& d, int stages, cudaG
     if (!d.sched) c->n_sweep = c->n_active;
     if (stages & kPrepSweep) {
         // every previous cluster fits a chunk: sort in shared memory (pxr_chunk.cuh)
-        c->chunk_path = (!d.sched && c->max_parent <= kChunkCapRows && c->n_active > 0) ? 1u : 0u;
+        c->chunk_path = d.sched || c->n_active == 0 || c->max_parent > kChunkCapRows ? 0u
+                        : c->max_parent > kChunkCapSmall                              ? 1u
+                                                                                      : 2u;
         c->n_gsort = c->chunk_path ? 0u : c->n_sweep;
         if (c->chunk_path) {   // the chunked sort reads and writes every item once
             c->stat_sort_items += c->n_sweep;

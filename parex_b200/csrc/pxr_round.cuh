@@ -138,6 +138,7 @@ constexpr uint32_t kWideRow = 4096;
 // Largest previous-round cluster for which a round's sort runs chunk by
 // chunk in shared memory (pxr_chunk.cuh).
 constexpr uint32_t kChunkCapRows = 4096;
+constexpr uint32_t kChunkCapSmall = 1024;   // the same with the smaller chunks
 
 // look-back sites (index into Dev::lb_epoch and RoundCtr::tile_counter)
 enum : int {

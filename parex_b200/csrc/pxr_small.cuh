@@ -30,12 +30,14 @@ constexpr uint32_t kSmallTile = 2 * kSmallThreads;   // sorted items of a CTA, a
 constexpr uint32_t kSmallMaxCtas = 16;               // the largest (opt-in) cluster
 // Which active sets take this kernel: those whose vertices fit the tiles of the
 // largest cluster, up to kSmallMaxSlots edge slots at the graph's mean degree (a
-// cluster is 16 of 148 SMs, so long row passes go to the whole GPU).  Measured, whole decomposition
-// on a B200, here / general path in a graph: planted partition 2,048 vertices
-// 1.54 / 4.42 ms, 8,192 2.09 / 5.94, 16,384 2.80 / 6.98, 32,000 (0.67 M slots)
-// 3.90 / 6.22; 16,000 vertices and 1.0 M slots 2.87 / 5.64; 3D grid 31^3
-// 3.89 / 6.87; R-MAT 14 4.40 / 6.96, R-MAT 15 (0.88 M slots, long rows)
-// 7.13 / 8.69; 2,000 vertices and 0.84 M slots 2.03 / 4.58.
+// cluster is 16 of 148 SMs, so long row passes go to the whole GPU).  Measured,
+// whole decomposition on a B200, here / general path in a graph: planted
+// partition 2,048 vertices 1.50 / 4.42 ms, 8,192 2.10 / 5.94, 16,384 2.77 / 6.98,
+// 32,000 (0.67 M slots) 3.87 / 6.22; 16,000 vertices and 1.0 M slots 2.88 / 5.64;
+// 3D grid 25^3 2.92 / 6.39; R-MAT 14 3.53 / 6.96, R-MAT 15 (0.88 M slots, long
+// rows) 6.47 / 8.69; 2,000 vertices and 0.84 M slots 1.46 / 4.58.  Handing the
+// last rounds over: 3D grid 41^3 6.2 -> 5.6 ms, 8-regular 100,000 vertices 4.8 ->
+// 4.3, batch of 8 instances 6.0 -> 4.4, of 64 instances 85.9 -> 83.5.
 constexpr uint32_t kSmallMaxSlots = 1u << 20;
 // CTAs are added while each has more vertices or edge slots than this
 // (2,048-vertex planted partition: 1, 2, 4, 8 CTAs take 2.20, 2.22, 1.97,

@@ -135,3 +135,27 @@ def test_schedule_switched_on_after_plain_graphs():
         out.append((dm.getFinalPartition().clusterIds, dm.downloadCertificates()))
     np.testing.assert_array_equal(out[0][0], out[1][0])
     np.testing.assert_array_equal(out[0][1], out[1][1])
+
+
+@pytest.mark.parametrize("size", [1023, 1024, 1025, 4095, 4096, 4097])
+def test_sort_paths_at_their_largest_clusters(size):
+    """Batches whose clusters sit at the bounds of the chunked sort's two shapes and of the global sort."""
+    count = 40000 // size + 1
+    starts = np.arange(count + 1, dtype=np.int64) * size
+    e = []
+    for i in range(count):
+        p = G.random_regular(size + size % 2, 8, seed=i + 1)   # an even number of stubs; the odd vertex is left out
+        src = np.repeat(np.arange(p.n), np.diff(p.offsets.astype(np.int64)))
+        keep = (src < p.cols) & (p.cols < size)
+        e.append(np.stack([src[keep], p.cols[keep].astype(np.int64)], axis=1) + starts[i])
+    g = _edges(int(starts[-1]), np.concatenate(e))
+    dm = P.CudaDeviceManager()
+    dm.initialize_batched(g, starts)
+    act = np.zeros(g.n, dtype=O.LNODE)
+    labels = np.repeat(np.arange(count, dtype=np.int32), size)
+    act["nix"], act["label"] = np.arange(g.n, dtype=np.uint32), labels
+    orc = O.Oracle(g.offsets, g.cols, O.MODE_PXR)
+    orc.set_state(labels, act, dm.readRandomWalkValues().astype(np.float64),
+                  np.diff(g.offsets.astype(np.int64)).astype(np.uint32), g.cols, count, 0)
+    dm.expanderDecomposition()
+    _check(dm, orc)
