@@ -148,6 +148,15 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
     return r.load(cuda::memory_order_relaxed);
 }
 
+// A word that other blocks change while this one reads it, where an older value
+// (no older than the kernel's start) serves as well: the load may be answered
+// by the SM's own L1.
+__device__ __forceinline__ uint32_t ld_near(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.relaxed.cta.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+}
+
 // ---------------------------------------------------------------------------
 // Decoupled look-back over tiles for an associative operator on uint64 values.
 // flags[t] holds (epoch << 2) | f with f = 1 (aggregate ready) or 2

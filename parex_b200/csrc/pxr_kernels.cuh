@@ -1008,10 +1008,17 @@ __device__ __forceinline__ bool in_split(const Dev<OffT>& d, uint32_t k, int32_t
 // roots), so a component's root is its minimum vertex and atomicMin can only
 // move a pointer closer to the root.  find() splits the path as it walks
 // with atomicMin, so a stored root is never replaced by a non-root ancestor.
+//
+// The reads may come from L1.  A parent read earlier in the kernel is still an
+// ancestor: the walk ends at the root, or while sets are being joined at a
+// vertex that was the root, which the join's compare-and-swap finds out.  In
+// the kernels that join nothing the roots stand still, and find() is exact.
+// Once a giant set has formed nearly every walk ends at its root, whose one
+// word all blocks then asked of one L2 slice.
 __device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t v) {
-    uint32_t p = ld_relaxed(&parent[v]);
+    uint32_t p = ld_near(&parent[v]);
     while (p != v) {
-        const uint32_t gp = ld_relaxed(&parent[p]);
+        const uint32_t gp = ld_near(&parent[p]);
         if (gp < p) atomicMin(&parent[v], gp);
         v = p;
         p = gp;
@@ -1021,7 +1028,7 @@ __device__ __forceinline__ uint32_t uf_find(uint32_t* parent, uint32_t v) {
 
 // Root of v, left in parent[v] (the atomic only where v's parent is not the root).
 __device__ __forceinline__ uint32_t uf_find_flat(uint32_t* parent, uint32_t v) {
-    const uint32_t p0 = ld_relaxed(&parent[v]);
+    const uint32_t p0 = ld_near(&parent[v]);
     const uint32_t r = p0 == v ? v : uf_find(parent, p0);
     if (r != p0) atomicMin(&parent[v], r);
     return r;
@@ -1097,18 +1104,24 @@ __global__ void __launch_bounds__(kBlock) k_compress(Dev<OffT> d, const uint32_t
     }
 }
 
-// Join the sets of v and nb (both in a split cluster, same label).  hint is
-// a word of v's set: when nb's parent is it, the two are joined already.
-__device__ __forceinline__ void uf_join(uint32_t* parent, uint32_t* err, uint32_t v, uint32_t nb, uint32_t& hint) {
-    if (ld_relaxed(&parent[nb]) == hint) return;
-    uint32_t a = v, b = nb;
+// Join the sets of v and nb (same label, both in a split cluster), given as a
+// vertex of each: hint, which is left at v's set's latest known root, and q,
+// nb's parent.  The walks start there and not at v and nb, whose own pointers
+// the component data flattens later.  A failed swap brings the fresh parent of
+// a vertex that is no root any more: each turn one of the two moves to a smaller vertex.
+// With walks from the parents through L1 the union phase of the 8-regular
+// graph on 2^22 vertices (learned) went from 10.5 to 4.6 ms, the 64-instance
+// batch's from 21.3 to 16.1, the 128^3 grid's from 3.1 to 2.5.
+__device__ __forceinline__ void uf_join(uint32_t* parent, uint32_t* err, uint32_t& hint, uint32_t q) {
+    if (q == hint) return;
+    uint32_t a = hint, b = q;
     for (uint32_t tries = 0;; ++tries) {
         if (tries > kSpinLimit) { atomicOr(err, kErrUnionFind); return; }
         const uint32_t ra = uf_find(parent, a), rb = uf_find(parent, b);
         if (ra == rb) { hint = ra; return; }
         const uint32_t hi = ra > rb ? ra : rb, lo = ra > rb ? rb : ra;
-        if (atomicCAS(&parent[hi], hi, lo) == hi) { hint = lo; return; }
-        a = hi;
+        a = atomicCAS(&parent[hi], hi, lo);
+        if (a == hi) { hint = lo; return; }
         b = lo;
     }
 }
@@ -1136,8 +1149,8 @@ __global__ void __launch_bounds__(kBlock) k_union_sample(Dev<OffT> d, const uint
         if (end == beg) continue;
         const uint32_t nb = d.cols[beg + (OffT)(mix32(v) % (uint64_t)(end - beg))];
         if (!slot_valid(nb) || d.lab[nb] != lv) continue;
-        uint32_t hint = ld_relaxed(&d.parent[v]);
-        uf_join(d.parent, &d.ctr->err, v, nb, hint);
+        uint32_t hint = ld_near(&d.parent[v]);
+        uf_join(d.parent, &d.ctr->err, hint, ld_near(&d.parent[nb]));
     }
 }
 
@@ -1170,7 +1183,7 @@ template <typename OffT>
 __device__ __forceinline__ bool union_skip_row(const Dev<OffT>& d, uint32_t k, uint32_t v, int32_t lv,
                                                uint32_t& hint) {
     if (!d.union_sampled) {
-        hint = ld_relaxed(&d.parent[v]);
+        hint = ld_near(&d.parent[v]);
         return false;
     }
     const uint32_t c = (uint32_t)lv >= k ? (uint32_t)lv - k : (uint32_t)lv;
@@ -1179,14 +1192,10 @@ __device__ __forceinline__ bool union_skip_row(const Dev<OffT>& d, uint32_t k, u
     return hint == rep;
 }
 
-// One light row of the union pass: lane gl of W joins its share of the slots.
-// BATCHED: labels and parents of kSlotUnroll slots loaded together, for rows
-// whose slots mostly need no join (sampled linking: the 64-instance batch's
-// union phase 25.6 -> 20.4 ms; the small-graph kernel, after its hooking
-// pass).  Where joins are common the parents loaded ahead go stale and cost
-// second looks: the 8-regular graph of 4.2 M vertices 10.1 -> 12.1 ms, so the
-// plain schedule takes slot by slot.
-template <bool BATCHED, typename OffT>
+// One light row of the union pass: lane gl of W joins its share of the slots,
+// labels and parents of kSlotUnroll slots loaded together (64-instance batch,
+// sampled linking: union phase 25.6 -> 20.4 ms).
+template <typename OffT>
 __device__ __forceinline__ void union_light_row(const Dev<OffT>& d, uint32_t k, uint32_t v, uint32_t gl, uint32_t W) {
     const int32_t lv = d.lab[v];
     if (!in_split(d, k, lv)) return;
@@ -1194,15 +1203,6 @@ __device__ __forceinline__ void union_light_row(const Dev<OffT>& d, uint32_t k, 
     if ((uint64_t)(end - beg) > d.light_max) return;   // union_long_rows
     uint32_t hint;
     if (union_skip_row(d, k, v, lv, hint)) return;
-    if (!BATCHED) {
-        for (OffT s = beg + gl; s < end; s += W) {
-            const uint32_t nb = d.cols[s];
-            if (!slot_valid(nb) || nb == v) continue;
-            if (!d.union_sampled && nb > v) break;   // each edge once, from its larger end
-            if (d.lab[nb] == lv) uf_join(d.parent, &d.ctr->err, v, nb, hint);
-        }
-        return;
-    }
     // each edge once, from its larger end; with sampled linking from this end whatever the order
     const uint32_t below = d.union_sampled ? kDisabledBit : v;
     for (OffT s = beg + gl; s < end; s += kSlotUnroll * W) {
@@ -1214,12 +1214,12 @@ __device__ __forceinline__ void union_light_row(const Dev<OffT>& d, uint32_t k, 
         for (int u = 0; u < kSlotUnroll; ++u) {
             const bool ok = nb[u] < below;
             ln[u] = ok ? d.lab[nb[u]] : -1;
-            pr[u] = ok ? ld_relaxed(&d.parent[nb[u]]) : 0u;
+            pr[u] = ok ? ld_near(&d.parent[nb[u]]) : 0u;
         }
         bool past = false;
 #pragma unroll
         for (int u = 0; u < kSlotUnroll; ++u) {
-            if (ln[u] == lv && pr[u] != hint && nb[u] != v) uf_join(d.parent, &d.ctr->err, v, nb[u], hint);
+            if (ln[u] == lv && nb[u] != v) uf_join(d.parent, &d.ctr->err, hint, pr[u]);
             past |= slot_valid(nb[u]) && nb[u] >= below;
         }
         if (past) break;
@@ -1246,7 +1246,7 @@ __device__ __forceinline__ void union_long_rows(const Dev<OffT>& d, uint32_t k, 
             const uint32_t nb = d.cols[s];
             if (!slot_valid(nb) || nb == v) continue;
             if (!d.union_sampled && nb > v) break;
-            if (d.lab[nb] == lv) uf_join(d.parent, &d.ctr->err, v, nb, hint);
+            if (d.lab[nb] == lv) uf_join(d.parent, &d.ctr->err, hint, ld_near(&d.parent[nb]));
         }
     });
 }
@@ -1270,11 +1270,7 @@ __global__ void __launch_bounds__(kBlock) k_union(Dev<OffT> d, RowParts parts, c
     const uint32_t gl = threadIdx.x & (W - 1);
     const uint32_t groups = (blocks * blockDim.x) / W;
     const uint32_t first = (block * blockDim.x + threadIdx.x) / W;
-    if (d.union_sampled) {
-        for (uint32_t j = first; j < count; j += groups) union_light_row<true>(d, k, ids[j], gl, (uint32_t)W);
-    } else {
-        for (uint32_t j = first; j < count; j += groups) union_light_row<false>(d, k, ids[j], gl, (uint32_t)W);
-    }
+    for (uint32_t j = first; j < count; j += groups) union_light_row(d, k, ids[j], gl, (uint32_t)W);
 }
 
 // root registry: one bit per vertex id

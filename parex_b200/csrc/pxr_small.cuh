@@ -565,7 +565,7 @@ __global__ void __launch_bounds__(kSmallThreads, 1) k_small_decompose(SmallArgs<
             }
             small_sync();
             // ---- union
-            for (uint32_t j = gid / W; j < na; j += nt / W) union_light_row<true>(d, k, ids[j], gid & (W - 1u), W);
+            for (uint32_t j = gid / W; j < na; j += nt / W) union_light_row(d, k, ids[j], gid & (W - 1u), W);
             union_long_rows<OffT, 32>(d, k, blockIdx.x, gridDim.x);
             union_long_rows<OffT, kSmallThreads>(d, k, blockIdx.x, gridDim.x);
             small_sync();
