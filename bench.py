@@ -553,7 +553,7 @@ def product_arm(args, rank, world, local_rank):
     d2h = n * 4 + 4
 
     # roofline: the walk step, the kernel the metric names (one launch = one
-    # walk step: the light-row kernel and the warp / CTA long-row kernels)
+    # walk step: light, warp-per-row and CTA-per-row bins together)
     pst = hr["prof_stats"]
     walk = hr["phases"]["walk"]
     steps_walked = max(1, pst["rounds"])
@@ -563,7 +563,7 @@ def product_arm(args, rank, world, local_rank):
     traffic, tsrc = measured_traffic(args.workload)
     roofline = {
         "bound": "hbm", "achieved": ach, "peak": peak, "unit": "GB/s", "frac": ach / peak, "traffic": traffic,
-        "kernel": "walk step: k_walk (light rows) + k_walk_long (warp / CTA per long row), one step per round",
+        "kernel": "walk step: k_walk (light rows, warp-per-row and CTA-per-row bins in one launch), one step per round",
         "algorithmic_bytes_per_launch": alg_walk, "launches": steps_walked, "device_us_per_launch": us_walk,
         "traffic_source": tsrc, "peak_source": f"{peak_kind} HBM copy peak", "form": head,
     }

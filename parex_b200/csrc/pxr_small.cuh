@@ -14,10 +14,10 @@
 // above).  What bounds it is the chain of dependent L2 loads inside a stage
 // and the barriers between stages (0.5-0.8 us each, about 18 a round), so a
 // stage keeps several loads in flight per thread and does in one pass what
-// the general path spreads over kernels.  Every result - labels, potentials, certificates, disabled slots,
-// tables of the last sweep - is the general path's bit for bit: sums are exact
-// fixed point, the sort is the same stable sort, roots and ties follow the
-// same rules.
+// the general path spreads over kernels.  Every result (labels, potentials,
+// certificates, disabled slots, tables of the last sweep) is the general
+// path's bit for bit: sums are exact fixed point, the sort is the same stable
+// sort, roots and ties follow the same rules.
 #pragma once
 
 #include "pxr_kernels.cuh"
@@ -35,8 +35,9 @@ constexpr uint32_t kSmallMaxCtas = 16;               // the largest (opt-in) clu
 // partition 2,048 vertices 1.50 / 4.42 ms, 8,192 2.10 / 5.94, 16,384 2.77 / 6.98,
 // 32,000 (0.67 M slots) 3.87 / 6.22; 16,000 vertices and 1.0 M slots 2.88 / 5.64;
 // 3D grid 25^3 2.92 / 6.39; R-MAT 14 3.53 / 6.96, R-MAT 15 (0.88 M slots, long
-// rows) 6.47 / 8.69; 2,000 vertices and 0.84 M slots 1.46 / 4.58.  Handing the
-// last rounds over: 3D grid 41^3 6.2 -> 5.6 ms, 8-regular 100,000 vertices 4.8 ->
+// rows) 6.47 / 8.69; 2,000 vertices and 0.84 M slots 1.46 / 4.58 (the
+// union-find walks through L1 came after: here 1.45, 2.56, 3.70, 2.85 ms at
+// 2,048, 16,384, 32,000 and 16,000 vertices).  Handing the last rounds over: 3D grid 41^3 6.2 -> 5.6 ms, 8-regular 100,000 vertices 4.8 ->
 // 4.3, batch of 8 instances 6.0 -> 4.4, of 64 instances 85.9 -> 83.5.
 constexpr uint32_t kSmallMaxSlots = 1u << 20;
 // CTAs are added while each has more vertices or edge slots than this

@@ -1,7 +1,8 @@
-"""The one-kernel decomposition of small graphs (graph driver, plain form) and
-the general path's tile sizes against the CPU oracle: sizes around a warp's, a CTA's and a cluster's share
-of vertices, rows in every bin, many clusters from the start, and a run
-stopped at its round cap and continued by the general path."""
+"""The one-kernel decomposition of small graphs (graph driver, plain form),
+the general path's tile sizes and the sweep order's download against the CPU
+oracle: sizes around a warp's, a CTA's and a cluster's share of vertices, rows
+in every bin, many clusters from the start, and a run stopped at its round cap
+and continued by the general path."""
 import numpy as np
 import pytest
 
