@@ -37,8 +37,9 @@ constexpr uint32_t kSmallMaxCtas = 16;               // the largest (opt-in) clu
 // 3D grid 25^3 2.92 / 6.39; R-MAT 14 3.53 / 6.96, R-MAT 15 (0.88 M slots, long
 // rows) 6.47 / 8.69; 2,000 vertices and 0.84 M slots 1.46 / 4.58 (the
 // union-find walks through L1 came after: here 1.45, 2.56, 3.70, 2.85 ms at
-// 2,048, 16,384, 32,000 and 16,000 vertices).  Handing the last rounds over: 3D grid 41^3 6.2 -> 5.6 ms, 8-regular 100,000 vertices 4.8 ->
-// 4.3, batch of 8 instances 6.0 -> 4.4, of 64 instances 85.9 -> 83.5.
+// 2,048, 16,384, 32,000 and 16,000 vertices).  Handing the last rounds over:
+// 3D grid 41^3 6.2 -> 5.6 ms, 8-regular 100,000 vertices 4.8 -> 4.3, batch of 8
+// instances 6.0 -> 4.4, of 64 instances 85.9 -> 83.5.
 constexpr uint32_t kSmallMaxSlots = 1u << 20;
 // CTAs are added while each has more vertices or edge slots than this
 // (2,048-vertex planted partition: 1, 2, 4, 8 CTAs take 2.20, 2.22, 1.97,
