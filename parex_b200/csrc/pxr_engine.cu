@@ -719,6 +719,11 @@ constexpr uint64_t kGsortLaunches = 2 + kMaxPasses;
 // kernels of the chunked sort (one per chunk shape)
 constexpr uint64_t kChunkLaunches = 2;
 constexpr uint32_t kSmallChunkCtas = 3;
+// one block at least, as every launch: a graph of no vertices runs the same stages
+template <class C, uint32_t CTAS>
+uint32_t chunk_blocks(uint32_t n) {
+    return std::max(std::min((n + C::kRows - 1) / C::kRows, 148u * CTAS), 1u);
+}
 
 // The graph being captured on h->stream, or null outside capture.
 cudaGraph_t capture_graph(pxr_handle* h) {
@@ -868,12 +873,11 @@ cudaError_t op_sweep(pxr_handle* h, bool in_round = false, const SortConds& cond
         if (e == cudaSuccess && run_chunk)
             e = if_region(h, c_chunk, [&](cudaStream_t st) {
                 k_chunk_sort<LargeChunk, 1, OffT>
-                    <<<std::min((h->n + LargeChunk::kRows - 1) / LargeChunk::kRows, 148u), LargeChunk::kThreads,
-                       LargeChunk::kSmem, st>>>(d, t, h->act[h->acur], h->par[h->acur], h->keys[0], h->vals[0], 1u);
+                    <<<chunk_blocks<LargeChunk, 1>(h->n), LargeChunk::kThreads, LargeChunk::kSmem, st>>>(
+                        d, t, h->act[h->acur], h->par[h->acur], h->keys[0], h->vals[0], 1u);
                 k_chunk_sort<SmallChunk, kSmallChunkCtas, OffT>
-                    <<<std::min((h->n + SmallChunk::kRows - 1) / SmallChunk::kRows, 148u * kSmallChunkCtas),
-                       SmallChunk::kThreads, SmallChunk::kSmem, st>>>(d, t, h->act[h->acur], h->par[h->acur],
-                                                                      h->keys[0], h->vals[0], 2u);
+                    <<<chunk_blocks<SmallChunk, kSmallChunkCtas>(h->n), SmallChunk::kThreads, SmallChunk::kSmem, st>>>(
+                        d, t, h->act[h->acur], h->par[h->acur], h->keys[0], h->vals[0], 2u);
                 return cudaGetLastError();
             });
     });
