@@ -44,9 +44,14 @@ struct DeviceGuard {
 };
 
 // cnt entries of the sweep order from entry first on, as the caller's records.
+// A cluster's first position comes from the order itself, by binary search over
+// the sorted labels: the cluster tables of the round that was swept are rewritten
+// by later rounds, and which of the two held them is not known to the host after
+// a captured loop.  18 loads an item on 274,625 vertices; the copy out of the
+// device bounds the call.
 __global__ void __launch_bounds__(kBlock) k_pack_nodes(const uint64_t* keys, const uint32_t* vals, const int32_t* pdif,
-                                                       const uint32_t* pvol, const uint32_t* starts, uint32_t n,
-                                                       uint32_t first, uint32_t cnt, pxr_node_data* out) {
+                                                       const uint32_t* pvol, uint32_t first, uint32_t cnt,
+                                                       pxr_node_data* out) {
     for (uint32_t q = blockIdx.x * blockDim.x + threadIdx.x; q < cnt; q += gridDim.x * blockDim.x) {
         const uint32_t i = first + q;
         pxr_node_data e;
@@ -54,7 +59,12 @@ __global__ void __launch_bounds__(kBlock) k_pack_nodes(const uint64_t* keys, con
         e.prefix_volume = pvol[i];
         e.prefix_edge_diff = pdif[i];
         const uint32_t c = (uint32_t)(keys[i] >> 32);
-        e.offset_in_cluster = i - (c < n ? starts[c] : 0u) + 1u;
+        uint32_t lo = 0, hi = i;   // the run of c starts in [lo, hi]
+        while (lo < hi) {
+            const uint32_t mid = lo + (hi - lo) / 2;
+            if ((uint32_t)(keys[mid] >> 32) < c) lo = mid + 1; else hi = mid;
+        }
+        e.offset_in_cluster = i - lo + 1u;
         out[q] = e;
     }
 }
@@ -488,7 +498,6 @@ struct pxr_handle {
     pxr_cluster_record* records = nullptr;   // n entries, allocated when trace is first enabled
     uint32_t records_n = 0;
     int xcur = 0, tcur = 0, acur = 0;
-    int sweep_tab = 0;
     uint32_t small_ctas = 0;         // largest cluster k_small_decompose can launch on this device
     cudaGraphExec_t graphs[8] = {};  // device-driven loop, one per parity combination
     cudaGraphConditionalHandle conds[8] = {};
@@ -891,7 +900,6 @@ cudaError_t op_sweep(pxr_handle* h, bool in_round = false, const SortConds& cond
         });
     else
         phase(h, kPhClusterCut, 1, [&] { launch_pdl(k_cluster_cut<OffT>, grid_for(h->n), kBlock, 0, s, d, t); });
-    h->sweep_tab = h->tcur;
     return cudaGetLastError();
 }
 
@@ -1218,7 +1226,6 @@ pxr_status decompose_small(pxr_handle* h, uint32_t max_rounds) {
     ++h->launches;
     const pxr_status st = sync_ctr(h);
     const uint32_t ran = h->h_ctr->rounds - before;
-    if (ran > 0) h->sweep_tab = h->tcur ^ (int)((ran - 1) & 1u);
     h->xcur ^= (int)(ran & 1u);
     h->tcur ^= (int)(ran & 1u);
     h->acur ^= (int)(ran & 1u);
@@ -2066,8 +2073,8 @@ pxr_status pxr_download_partition(pxr_handle* h, pxr_node_data* out, uint32_t ca
     const uint32_t room = (uint32_t)(slice_bytes(std::max<size_t>(h->n, 1) * sizeof(*h->dv)) / sizeof(pxr_node_data));
     for (uint32_t i = 0; i < c; i += room) {
         const uint32_t cnt = std::min(room, c - i);
-        k_pack_nodes<<<grid_for(cnt), kBlock, 0, h->stream>>>(h->keys[sel], h->vals[sel], h->pdif, h->pvol,
-                                                              h->tab[h->sweep_tab].start, h->n, i, cnt, packed);
+        k_pack_nodes<<<grid_for(cnt), kBlock, 0, h->stream>>>(h->keys[sel], h->vals[sel], h->pdif, h->pvol, i,
+                                                              cnt, packed);
         h->launches += 1;
         PXR_CUDA(h, cudaGetLastError());
         PXR_CUDA(h, cudaMemcpyAsync(out + i, packed, (size_t)cnt * sizeof(pxr_node_data), cudaMemcpyDeviceToHost,

@@ -34,3 +34,68 @@ def test_graph_without_vertices(driver, form):
     assert dm.getNumClusters() == 0
     assert dm.getFinalPartition().numClusters == 0
     assert dm.getNumCutEdges() == 0
+
+
+def _paths(count):
+    """A batch of paths of 1 to 7 vertices and its instance starts."""
+    sizes = 1 + np.arange(count) % 7
+    starts = np.concatenate([[0], np.cumsum(sizes)]).astype(np.int64)
+    inner = np.ones(int(starts[-1]), dtype=bool)
+    inner[starts[1:] - 1] = False
+    at = np.nonzero(inner)[0]
+    return _edges(int(starts[-1]), np.stack([at, at + 1], axis=1)), starts, sizes
+
+
+def _batch_oracle(dm, g, sizes):
+    count = sizes.shape[0]
+    act = np.zeros(g.n, dtype=O.LNODE)
+    labels = np.repeat(np.arange(count, dtype=np.int32), sizes)
+    act["nix"], act["label"] = np.arange(g.n, dtype=np.uint32), labels
+    orc = O.Oracle(g.offsets, g.cols, O.MODE_PXR)
+    orc.set_state(labels, act, dm.readRandomWalkValues().astype(np.float64),
+                  np.diff(g.offsets.astype(np.int64)).astype(np.uint32), g.cols, count, 0)
+    return orc
+
+
+def _run_rounds(orc, rounds=None):
+    """The oracle's rounds one by one: how many ran, and the last one's sweep order."""
+    done, srt = 0, None
+    while orc.n_active and orc.n_clusters and done != rounds:
+        orc.walk()
+        orc.sweep()
+        srt = orc.sorted()
+        orc.cut_clusters()
+        done += 1
+    return done, srt
+
+
+def _check_sweep_order(dm, srt):
+    part = dm.downloadPartition()
+    for ours, theirs in (("nix", "nix"), ("prefix_edge_diff", "prefix_edge_diff"),
+                         ("prefix_volume", "prefix_volume"), ("offset_in_cluster", "offset")):
+        np.testing.assert_array_equal(part[ours], srt[theirs])
+
+
+@pytest.mark.parametrize("cap", [200000, 2, 4])
+def test_sweep_order_after_a_decomposition(cap):
+    """Of the last round that ran: after a run handed over or stopped at its cap, then
+    after one that ends in its first round and replays the first one's captured loop."""
+    g, starts, sizes = _paths(12000)
+    dm = P.CudaDeviceManager(max_rounds=cap)
+    dm.initialize_batched(g, starts)
+    orc = _batch_oracle(dm, g, sizes)
+    try:
+        rounds = dm.expanderDecomposition()
+    except P.PxrError:
+        rounds = cap
+    done, srt = _run_rounds(orc, cap)
+    assert done == rounds
+    _check_sweep_order(dm, srt)
+
+    dm.initialize_batched(g, starts)
+    dm.set_potentials(np.zeros(g.n))      # no spread anywhere: every cluster is certified at once
+    orc = _batch_oracle(dm, g, sizes)
+    assert dm.expanderDecomposition() == 1
+    done, srt = _run_rounds(orc)
+    assert done == 1
+    _check_sweep_order(dm, srt)
