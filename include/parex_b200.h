@@ -380,7 +380,9 @@ pxr_status pxr_final_partition_static(const int32_t* labels, uint32_t n, int32_t
 /* Test hooks with no counterpart in the reference: overwrite the potentials
  * (n doubles, rounded to the product's float storage), or the whole round
  * state.  act holds the n_act active vertex ids in the order their keys are
- * emitted; labels of active vertices must be dense in [0, n_clusters). */
+ * emitted; labels of active vertices must be dense in [0, n_clusters), with
+ * n_clusters <= n.  Labels that no active vertex carries are accepted with
+ * full_components only (the first round drops them). */
 pxr_status pxr_set_potentials(pxr_handle* h, const double* x);
 pxr_status pxr_set_state(pxr_handle* h, const int32_t* labels, const uint32_t* act, uint32_t n_act,
                          const double* x, const uint32_t* internal_degrees, const uint32_t* cols,

@@ -2340,6 +2340,8 @@ pxr_status pxr_set_state(pxr_handle* h, const int32_t* labels, const uint32_t* a
     if (!h->initialized) return fail(h, PXR_NOT_INITIALIZED, "no graph uploaded");
     const uint32_t n = h->n;
     if (n_act > n) return fail(h, PXR_INVALID_ARG, "n_act exceeds n");
+    // the cluster tables hold n entries, slices of one allocation
+    if (n_clusters > n) return fail(h, PXR_INVALID_ARG, "n_clusters exceeds n");
     std::vector<uint32_t> size(std::max<uint32_t>(n_clusters, 1), 0), vol(std::max<uint32_t>(n_clusters, 1), 0),
         root(std::max<uint32_t>(n_clusters, 1), 0xFFFFFFFFu);
     for (uint32_t i = 0; i < n_act; ++i) {
@@ -2351,6 +2353,9 @@ pxr_status pxr_set_state(pxr_handle* h, const int32_t* labels, const uint32_t* a
         vol[l] += ideg[v];
         root[l] = std::min(root[l], v);
     }
+    // a cluster without vertices has no root: only a round that recomputes every component drops it unread
+    if (!full_components && std::find(size.begin(), size.begin() + n_clusters, 0u) != size.begin() + n_clusters)
+        return fail(h, PXR_INVALID_ARG, "a cluster without vertices needs full_components");
     std::vector<uint32_t> start(size.size(), 0), vol_start(size.size(), 0);
     for (uint32_t c = 1; c < n_clusters; ++c) {
         start[c] = start[c - 1] + size[c - 1];

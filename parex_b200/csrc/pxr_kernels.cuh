@@ -1164,10 +1164,10 @@ __global__ void __launch_bounds__(kBlock) k_union_reps(Dev<OffT> d, ClusterTable
     const uint32_t k = d.ctr->n_clusters;
     const uint32_t* vals = d.ctr->main_sel ? vals1 : vals0;
     for (uint32_t c = blockIdx.x * blockDim.x + threadIdx.x; c < k; c += gridDim.x * blockDim.x) {
-        if (!d.split[c]) continue;
         const uint32_t st = t.start[c], sz = t.size[c];
+        if (!d.split[c] || sz == 0) continue;   // a loaded state may name clusters without vertices
         d.rep[0][c] = uf_find(d.parent, vals[st]);
-        if (d.cut_off[c] != kNoCut && sz > 0) d.rep[1][c] = uf_find(d.parent, vals[st + sz - 1]);
+        if (d.cut_off[c] != kNoCut) d.rep[1][c] = uf_find(d.parent, vals[st + sz - 1]);
     }
 }
 

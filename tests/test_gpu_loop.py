@@ -99,3 +99,52 @@ def test_sweep_order_after_a_decomposition(cap):
     done, srt = _run_rounds(orc)
     assert done == 1
     _check_sweep_order(dm, srt)
+
+
+def _state(g, active, count, n_clusters):
+    """Labels that spread the `count` paths of the first `active` vertices over
+    [0, n_clusters) at an even step, the rest inactive."""
+    sizes = 1 + np.arange(count) % 7
+    labels = np.full(g.n, -1, dtype=np.int32)
+    labels[:active] = np.repeat(np.arange(count) * (n_clusters // count), sizes)
+    return labels
+
+
+def _loaded_state(g, active, count, n_clusters, full=True, **kw):
+    dm = P.CudaDeviceManager(**kw)
+    dm.initialize(g)
+    x = np.sin(np.arange(g.n) * 0.37)
+    dm.set_state(_state(g, active, count, n_clusters), np.arange(active, dtype=np.uint32), x,
+                 np.diff(g.offsets.astype(np.int64)).astype(np.uint32), g.cols, n_clusters, -1, full)
+    return dm
+
+
+def test_state_with_more_clusters_than_tables_is_refused():
+    """The cluster tables hold a cluster per vertex; a cluster without vertices has no
+    root to go on with unless the first round recomputes every component."""
+    g, starts, _ = _paths(700)
+    active = int(starts[300])
+    for n_clusters in (g.n + 1, 0xFFFFFFFF):
+        with pytest.raises(P.PxrError):
+            _loaded_state(g, active, 300, n_clusters)
+    with pytest.raises(P.PxrError):
+        _loaded_state(g, active, 300, 301, full=False)
+    _loaded_state(g, active, 300, g.n)
+    dm = _loaded_state(g, active, 300, 300, full=False)
+    assert dm.getNumClusters() == 300
+
+
+# sampled linking looks a representative up for every cluster
+@pytest.mark.parametrize("driver,components", [(P.DRIVER_STREAM, P.COMPONENTS_PLAIN),
+                                               (P.DRIVER_STREAM, P.COMPONENTS_SAMPLED)])
+@pytest.mark.parametrize("count,n_clusters", [(300, 5000), (5000, 17000), (5000, 47000)])
+def test_labels_without_vertices(count, n_clusters, driver, components):
+    """A state with gaps between its labels and past the last one gives the dense one's decomposition."""
+    g, starts, _ = _paths(12000)
+    out = []
+    for k in (count, n_clusters):
+        dm = _loaded_state(g, int(starts[count]), count, k, driver=driver, components=components)
+        dm.expanderDecomposition()
+        out.append((dm.downloadLabels(), dm.downloadCertificates(), dm.readRandomWalkValues().view(np.uint32)))
+    for a, b in zip(*out):
+        np.testing.assert_array_equal(a, b)
