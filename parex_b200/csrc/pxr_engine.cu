@@ -1125,12 +1125,15 @@ uint32_t small_take(const pxr_handle* h) {
     return h->n <= take || h->n_wide + h->n_heavy <= kSmallLongRows ? take : 0u;
 }
 
-// CTAs for `active` vertices (at most small_take).
-uint32_t small_cluster(const pxr_handle* h, uint32_t active) {
+// CTAs for `active` vertices in `clusters` clusters (at most small_take, and
+// small_ctas * kSmallTile): kSmallTile of either a CTA.  A loaded state can name
+// more clusters than it has vertices; every later round has two vertices a cluster.
+uint32_t small_cluster(const pxr_handle* h, uint32_t active, uint32_t clusters) {
     const uint64_t slots = h->slots * (uint64_t)active / std::max(h->n, 1u);
+    const uint32_t held = std::max(active, clusters);
     uint32_t ctas = 1;
-    while (ctas * kSmallTile < active || (ctas < h->small_ctas && (active > ctas * kSmallVerticesPerCta ||
-                                                                  slots > (uint64_t)ctas * kSmallSlotsPerCta)))
+    while (ctas * kSmallTile < held || (ctas < h->small_ctas && (active > ctas * kSmallVerticesPerCta ||
+                                                                slots > (uint64_t)ctas * kSmallSlotsPerCta)))
         ctas <<= 1;
     return ctas;
 }
@@ -1221,7 +1224,7 @@ void prepare_chunk_sort() {
 
 pxr_status decompose_small(pxr_handle* h, uint32_t max_rounds) {
     const uint32_t before = h->h_ctr->rounds;
-    const uint32_t ctas = small_cluster(h, h->h_ctr->n_active);
+    const uint32_t ctas = small_cluster(h, h->h_ctr->n_active, h->h_ctr->n_clusters);
     PXR_CUDA(h, h->off64 ? launch_small<uint64_t>(h, ctas, max_rounds) : launch_small<uint32_t>(h, ctas, max_rounds));
     ++h->launches;
     const pxr_status st = sync_ctr(h);
@@ -1234,7 +1237,8 @@ pxr_status decompose_small(pxr_handle* h, uint32_t max_rounds) {
 
 pxr_status decompose_graph(pxr_handle* h) {
     const uint32_t take = small_take(h);
-    if (take && h->h_ctr->n_active <= take) return decompose_small(h, h->cfg.max_rounds);
+    if (take && h->h_ctr->n_active <= take && h->h_ctr->n_clusters <= h->small_ctas * kSmallTile)
+        return decompose_small(h, h->cfg.max_rounds);
     const int key = h->xcur | (h->tcur << 1) | (h->acur << 2);
     if (!h->graphs[key]) {
         pxr_status st = build_loop_graph(h, key);

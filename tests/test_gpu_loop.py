@@ -136,10 +136,13 @@ def test_state_with_more_clusters_than_tables_is_refused():
 
 # sampled linking looks a representative up for every cluster
 @pytest.mark.parametrize("driver,components", [(P.DRIVER_STREAM, P.COMPONENTS_PLAIN),
-                                               (P.DRIVER_STREAM, P.COMPONENTS_SAMPLED)])
+                                               (P.DRIVER_STREAM, P.COMPONENTS_SAMPLED),
+                                               (P.DRIVER_GRAPH, P.COMPONENTS_PLAIN)])
 @pytest.mark.parametrize("count,n_clusters", [(300, 5000), (5000, 17000), (5000, 47000)])
 def test_labels_without_vertices(count, n_clusters, driver, components):
-    """A state with gaps between its labels and past the last one gives the dense one's decomposition."""
+    """A state with gaps between its labels and past the last one gives the dense
+    one's decomposition, also where the one-kernel form has more clusters than
+    vertices to lay its CTAs out for, or more than its largest cluster holds."""
     g, starts, _ = _paths(12000)
     out = []
     for k in (count, n_clusters):
