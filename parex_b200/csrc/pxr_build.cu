@@ -433,7 +433,7 @@ __global__ void k_contract_slots(uint32_t n, const uint32_t* off, const uint32_t
         if (c < 0 || (uint32_t)c >= k) { if (lane == 0) atomicOr(bad, 1u); continue; }
         const uint32_t beg = off[v], end = off[v + 1];
         uint32_t cut = 0;
-        for (uint32_t s = beg + lane; s < end; s += 32) {
+        for (uint64_t s = (uint64_t)beg + lane; s < end; s += 32) {   // end may lie within 32 of 2^32
             const uint32_t u = cols[s];
             if (u >= n) { atomicOr(bad, 1u); continue; }
             const int32_t cu = ids[u];

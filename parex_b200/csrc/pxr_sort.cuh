@@ -29,6 +29,15 @@ constexpr int kSortTile = kSortThreads * kSortItems;
 constexpr int kRadix = 256;
 constexpr int kMaxPasses = 8;
 
+// Tiles of `tile` items over count items.  Counts go up to 2^32 - 1 (both
+// directions of 2^31 - 1 edges), where count + tile - 1 does not fit 32 bits.
+__host__ __device__ constexpr uint32_t sort_tiles(uint32_t count, uint32_t tile) {
+    return count / tile + (count % tile ? 1u : 0u);
+}
+static_assert(sort_tiles(0xFFFFFFFFu, 4096) == 1u << 20 && sort_tiles(0, 4096) == 0 && sort_tiles(4096, 4096) == 1 &&
+                  sort_tiles(4097, 4096) == 2,
+              "every item has a tile");
+
 struct SortState {
     uint32_t* hist;       // [kMaxPasses][kRadix] digit counts (kept zero between sorts)
     uint32_t* bases;      // [kMaxPasses][kRadix] exclusive digit bases
@@ -60,7 +69,8 @@ __global__ void __launch_bounds__(kSortThreads) sort_histogram_kernel(SortBuffer
     const uint32_t end_bit = *b.end_bit;
     const int npasses = (int)((end_bit + 7u) / 8u);
     const K* keys = b.keys[0];
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
+    // 64-bit: within a stride of 2^32 a 32-bit index would start over and never end
+    for (uint64_t i = blockIdx.x * blockDim.x + threadIdx.x; i < count; i += gridDim.x * blockDim.x) {
         const K k = keys[i];
         for (int p = 0; p < npasses; ++p) atomicAdd(&sh[p][(uint32_t)(k >> (8 * p)) & 0xFFu], 1u);
     }
@@ -166,7 +176,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
     uint32_t* vout = in ? b.vals[0] : b.vals[1];
     const bool has_vals = vin != nullptr;
     const uint32_t count = *b.count;
-    const uint32_t num_tiles = (count + kSortTile - 1) / kSortTile;
+    const uint32_t num_tiles = sort_tiles(count, kSortTile);
     const uint32_t epoch = *s.epoch + (uint32_t)pass;
     const int shift = 8 * pass;
 
@@ -177,7 +187,8 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
     if (tile >= num_tiles) return;
 
     const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
-    const uint32_t base = tile * kSortTile + warp * (32 * kSortItems);
+    const uint32_t in_warp = warp * (32 * kSortItems);   // the warp's first place in the tile
+    const uint32_t base = tile * kSortTile + in_warp;
     const uint32_t tile_items = min((uint32_t)kSortTile, count - tile * kSortTile);
     const bool full = tile_items == (uint32_t)kSortTile;   // all but the last tile skip the bounds tests
     K key[kSortItems];
@@ -191,8 +202,9 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
 #pragma unroll
         for (int k = 0; k < kSortItems; ++k) {
             const uint32_t idx = base + k * 32 + lane;
-            key[k] = idx < count ? kin[idx] : (K)0;
-            val[k] = (idx < count && has_vals) ? vin[idx] : 0u;
+            const bool valid = in_warp + k * 32 + lane < tile_items;
+            key[k] = valid ? kin[idx] : (K)0;
+            val[k] = (valid && has_vals) ? vin[idx] : 0u;
         }
     }
     // Lanes of the same digit, for every item at once: the ballots of
@@ -213,7 +225,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
         const uint32_t d = sort_digit(key[k], shift);
         uint32_t peers = 0xFFFFFFFFu;
         if (!full) {
-            const bool valid = base + k * 32 + lane < count;
+            const bool valid = in_warp + k * 32 + lane < tile_items;
             const uint32_t in_range = __ballot_sync(0xFFFFFFFFu, valid);
             peers = valid ? in_range : ~in_range;
         }
@@ -226,7 +238,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
     }
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
-        const bool valid = full || base + k * 32 + lane < count;
+        const bool valid = full || in_warp + k * 32 + lane < tile_items;
         const uint32_t d = sort_digit(key[k], shift);
         const uint32_t peers = rank[k];
         // every lane reads its digit's count (peers read one word), the first peer advances it
@@ -267,7 +279,7 @@ __global__ void __launch_bounds__(kSortThreads, MINB) sort_pass_kernel(SortBuffe
 
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
-        if (full || base + k * 32 + lane < count) {
+        if (full || in_warp + k * 32 + lane < tile_items) {
             const uint32_t pos = whist[warp][sort_digit(key[k], shift)] + rank[k];
             skeys[pos] = key[k];
             svals[pos] = val[k];
@@ -302,7 +314,7 @@ constexpr int kSortMinTile = kSortThreads * 8;
 template <typename K, int ITEMS, int MINB>
 inline void launch_sort_passes(const SortBuffers<K>& b, const SortState& s, uint32_t* err, cudaStream_t stream,
                                int npasses) {
-    const uint32_t tiles = (b.capacity + kSortThreads * ITEMS - 1) / (kSortThreads * ITEMS);
+    const uint32_t tiles = sort_tiles(b.capacity, kSortThreads * ITEMS);
     for (int p = 0; p < npasses; ++p)
         sort_pass_kernel<K, ITEMS, MINB><<<tiles, kSortThreads, sort_pass_smem<K, ITEMS>(), stream>>>(b, s, p, err);
 }
@@ -314,7 +326,7 @@ template <typename K>
 inline cudaError_t radix_sort(const SortBuffers<K>& b, const SortState& s, uint32_t* err, cudaStream_t stream,
                               int max_end_bit, int plan = 0) {
     if (b.capacity == 0) return cudaSuccess;
-    const uint32_t tiles = (b.capacity + kSortTile - 1) / kSortTile;
+    const uint32_t tiles = sort_tiles(b.capacity, kSortTile);
     const uint32_t hgrid = min(tiles * 4u, 148u * 8u);
     sort_histogram_kernel<K><<<hgrid, kSortThreads, 0, stream>>>(b, s);
     sort_plan_kernel<K><<<1, kRadix, 0, stream>>>(b, s);

@@ -167,3 +167,27 @@ def test_build_at_tile_edges_and_with_gaps(n, edges, distinct):
     host = G.csr_from_edges(pick[:, 0], pick[:, 1], n)
     assert m == host.m
     _same(B.to_host(off, cols), host)
+
+
+@pytest.mark.parametrize("form", ["merged", "finalize"])
+def test_largest_edge_list(form):
+    """2^31 - 1 edges, as many as are accepted: both directions are two short of
+    2^32 items, within one grid stride and one tile of the 32-bit range's end."""
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 125e9:
+        pytest.skip("needs 125 GB of device memory")
+    e = 2**31 - 1
+    u = torch.zeros(e, dtype=torch.int32, device="cuda")
+    v = torch.ones(e, dtype=torch.int32, device="cuda")
+    u[-1], v[-1] = 1, 2
+    off, cols, m = (B.build_csr if form == "merged" else B.build_csr_finalize)(3, u, v)
+    off = off.cpu().numpy().view(np.uint32).tolist()
+    if form == "merged":
+        assert m == 2 and off == [0, 1, 3, 4]
+        assert cols.tolist() == [1, 0, 2, 1]
+    else:
+        assert m == e and off == [0, e - 1, 2 * e - 1, 2 * e]
+        assert bool((cols[: e - 1] == 1).all()) and bool((cols[e - 1: 2 * e - 2] == 0).all())
+        assert cols[2 * e - 2:].tolist() == [2, 1]
+    del u, v, cols
+    torch.cuda.empty_cache()
