@@ -1295,7 +1295,10 @@ pxr_status reset_schedule_state(pxr_handle* h) {
     return PXR_OK;
 }
 
-constexpr size_t kArenaKeep = 64u << 20;
+// Device memory a handle may hold beyond its graph's need: enough that the small
+// graphs of a hierarchy or a server come and go in one allocation, and little
+// enough that loading a smaller graph gives a large one's memory back.
+constexpr size_t kArenaSpare = 64u << 20;
 
 template <typename OffT>
 pxr_status allocate(pxr_handle* h, uint32_t n, uint64_t m) {
@@ -1346,8 +1349,8 @@ pxr_status allocate(pxr_handle* h, uint32_t n, uint64_t m) {
     size_t total = 0;
     for (const Slice& q : slices) total += slice_bytes(q.bytes);
     // a graph that fits takes over the last one's arena, unless that would hold
-    // more than twice what it needs (or kArenaKeep)
-    const bool keep = h->arena_bytes >= total && h->arena_bytes <= std::max(2 * total, kArenaKeep) && !h->records &&
+    // more than kArenaSpare above what it needs
+    const bool keep = h->arena_bytes >= total && h->arena_bytes - total <= kArenaSpare && !h->records &&
                       !h->sched.trace && h->allocs.size() == 1;
     unsigned char* arena = keep ? static_cast<unsigned char*>(h->allocs[0]) : nullptr;
     cudaError_t e = cudaSuccess;

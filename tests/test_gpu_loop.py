@@ -151,3 +151,13 @@ def test_labels_without_vertices(count, n_clusters, driver, components):
         out.append((dm.downloadLabels(), dm.downloadCertificates(), dm.readRandomWalkValues().view(np.uint32)))
     for a, b in zip(*out):
         np.testing.assert_array_equal(a, b)
+
+
+def test_memory_of_a_larger_graph_is_given_back():
+    """A handle keeps at most 64 MiB more than the graph it holds needs."""
+    used, fresh = P.CudaDeviceManager(), P.CudaDeviceManager()
+    small = G.grid3d(85)
+    used.initialize(G.grid3d(100))
+    used.initialize(small)
+    fresh.initialize(small)
+    assert used.stats()["device_bytes"] <= fresh.stats()["device_bytes"] + (64 << 20)
