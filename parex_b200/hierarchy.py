@@ -25,6 +25,11 @@ from . import _lib
 from .manager import CudaDeviceManager
 
 
+# Device memory of a handle that stays open between two levels (opening one costs
+# a millisecond or two, little beside a level that needs more than this).
+KEEP_BYTES = 64 << 20
+
+
 @dataclass
 class Level:
     n: int                  # vertices of the level graph
@@ -73,27 +78,35 @@ def build(offsets, cols, seed: int = 6582, sc_threshold: float = 0.3, rw_thresho
     off, col = offsets.to(dev), cols.to(dev)
     vol_below = None
     sc = sc_threshold
-    dm, dm_sc = None, None     # one handle for all levels: only a lowered threshold needs another
-    while int(off.shape[0]) - 1 > 1 and len(levels) < max_levels:
-        n = int(off.shape[0]) - 1
-        m = int(col.shape[0]) // 2
-        if dm_sc != sc:
-            if dm is not None:
+    # one handle for all levels: a lowered threshold needs another, and a large
+    # one is closed before the contraction, which needs the memory itself
+    dm, dm_sc = None, None
+    try:
+        while int(off.shape[0]) - 1 > 1 and len(levels) < max_levels:
+            n = int(off.shape[0]) - 1
+            m = int(col.shape[0]) // 2
+            if dm is None or dm_sc != sc:
+                if dm is not None:
+                    dm.close()
+                dm, dm_sc = CudaDeviceManager(seed=seed, sc_threshold=sc, rw_threshold=rw_threshold, device=device), sc
+            dm.initialize_device(n, m, off.data_ptr(), False, col.data_ptr())
+            dm.expanderDecomposition()
+            fp = dm.getFinalPartition()
+            cut = dm.countCutEdges()
+            if m > 0 and cut > 0.95 * m:
+                sc *= 0.8      # the reference's adjustment (expander_hierarchy.h:116-121)
+                continue
+            if dm.stats()["device_bytes"] > KEEP_BYTES:
                 dm.close()
-            dm, dm_sc = CudaDeviceManager(seed=seed, sc_threshold=sc, rw_threshold=rw_threshold, device=device), sc
-        dm.initialize_device(n, m, off.data_ptr(), False, col.data_ptr())
-        dm.expanderDecomposition()
-        fp = dm.getFinalPartition()
-        cut = dm.countCutEdges()
-        if m > 0 and cut > 0.95 * m:
-            sc *= 0.8          # the reference's adjustment (expander_hierarchy.h:116-121)
-            continue
-        ids = torch.from_numpy(fp.clusterIds).to(dev)
-        noff, ncol, nm, cut_sizes, vol = contract(off, col, ids, fp.numClusters, vol_below, device)
-        levels.append(Level(n, m, fp.numClusters, nm, sc, fp.clusterIds, vol.cpu().numpy(), cut_sizes.cpu().numpy()))
-        if fp.numClusters == n:
-            break              # nothing merged (no edges left): the remaining vertices are roots
-        off, col, vol_below = noff, ncol, vol
-    if dm is not None:
-        dm.close()
+                dm = None
+            ids = torch.from_numpy(fp.clusterIds).to(dev)
+            noff, ncol, nm, cut_sizes, vol = contract(off, col, ids, fp.numClusters, vol_below, device)
+            levels.append(Level(n, m, fp.numClusters, nm, sc, fp.clusterIds, vol.cpu().numpy(),
+                                cut_sizes.cpu().numpy()))
+            if fp.numClusters == n:
+                break          # nothing merged (no edges left): the remaining vertices are roots
+            off, col, vol_below = noff, ncol, vol
+    finally:
+        if dm is not None:
+            dm.close()
     return levels

@@ -161,3 +161,34 @@ def test_memory_of_a_larger_graph_is_given_back():
     used.initialize(small)
     fresh.initialize(small)
     assert used.stats()["device_bytes"] <= fresh.stats()["device_bytes"] + (64 << 20)
+
+
+def test_contraction_runs_without_the_decomposition_s_memory(monkeypatch):
+    """A level's contraction has the device to itself but for a small handle kept open for the next level."""
+    import torch
+    from parex_b200 import hierarchy as H
+    open_handles, held = [], []
+
+    class Handle(H.CudaDeviceManager):
+        def __init__(self, **kw):
+            super().__init__(**kw)
+            open_handles.append(self)
+
+        def close(self):
+            if self in open_handles:
+                open_handles.remove(self)
+            super().close()
+
+    contract = H.contract
+
+    def contract_noting(*a, **kw):
+        held.append(sum(h.stats()["device_bytes"] for h in open_handles))
+        return contract(*a, **kw)
+
+    monkeypatch.setattr(H, "CudaDeviceManager", Handle)
+    monkeypatch.setattr(H, "contract", contract_noting)
+    g = G.grid3d(80)
+    levels = H.build(torch.from_numpy(g.offsets.view(np.int32)), torch.from_numpy(g.cols.view(np.int32)))
+    assert len(held) == len(levels) > 1
+    assert max(held) <= 64 << 20
+    assert not open_handles
