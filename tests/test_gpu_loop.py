@@ -192,3 +192,135 @@ def test_contraction_runs_without_the_decomposition_s_memory(monkeypatch):
     assert len(held) == len(levels) > 1
     assert max(held) <= 64 << 20
     assert not open_handles
+
+
+HUBS = {30007: 5000, 41000: 1500, 49999: 300}      # long rows among short ones, by vertex
+LASTING = (30007, 49999)                           # active when the rounds are handed over
+
+
+def _with_hubs():
+    """8-regular beside a planted partition with hubs."""
+    a, b = G.random_regular(30000, 8, seed=1), G.sbm_graph(20000, 40, 9.0, 1.0, 5)
+    rng = np.random.default_rng(3)
+    src, dst = [], []
+    for g, first in ((a, 0), (b, 30000)):
+        src.append(np.repeat(np.arange(g.n), np.diff(g.offsets.astype(np.int64))) + first)
+        dst.append(g.cols.astype(np.int64) + first)
+    for hub, degree in HUBS.items():
+        src.append(np.full(degree, hub))
+        dst.append(30000 + rng.choice(20000, degree, replace=False))
+    src, dst = np.concatenate(src), np.concatenate(dst)
+    keep = src != dst
+    return G.csr_from_edges(src[keep], dst[keep], 50000)
+
+
+# beyond the one-kernel decomposition (32,768 vertices); with each a row plan
+# under which most rows are long, so that the last rounds are not handed over either
+GRAPHS = {
+    "sbm40k": (lambda: G.sbm_graph(40000, 40, 9.0, 1.0, 4), (4, 9, 16)),
+    "grid35": (lambda: G.grid3d(35), (1, 5, 5)),
+    "rmat16": (lambda: G.rmat(16, 8, seed=2), (8, 32, 256)),
+}
+
+
+def _start(g, dm):
+    orc = O.Oracle(g.offsets, g.cols, O.MODE_PXR)
+    orc.set_potentials(dm.readRandomWalkValues().astype(np.float64))
+    return orc
+
+
+def _check_state(dm, orc, srt):
+    np.testing.assert_array_equal(dm.downloadLabels(), orc.labels())
+    np.testing.assert_array_equal(dm.readRandomWalkValues().view(np.uint32),
+                                  np.asarray(orc.potentials(), dtype=np.float32).view(np.uint32))
+    np.testing.assert_array_equal(dm.downloadDegrees(), orc.internal_degrees())
+    np.testing.assert_array_equal(dm.downloadGraph()[1], orc.cols())
+    np.testing.assert_array_equal(dm.downloadCertificates(), orc.certificates())
+    _check_sweep_order(dm, srt)
+    ids, k = orc.final_partition()
+    fp = dm.getFinalPartition()
+    assert fp.numClusters == k
+    np.testing.assert_array_equal(fp.clusterIds, ids)
+
+
+@pytest.mark.parametrize("name", sorted(GRAPHS))
+@pytest.mark.parametrize("components,sort_plan",
+                         [(P.COMPONENTS_PLAIN, 0), (P.COMPONENTS_PLAIN, 1), (P.COMPONENTS_SAMPLED, 2)])
+def test_options_inside_the_captured_loop(name, components, sort_plan):
+    """Both component schedules and every sort plan with all rounds in the captured loop."""
+    make, plan = GRAPHS[name]
+    g = make()
+    dm = P.CudaDeviceManager(components=components)
+    dm.set_row_plan(*plan)
+    dm.set_sort_plan(sort_plan)
+    dm.initialize(g)
+    assert dm.row_plan()["wide_rows"] + dm.row_plan()["heavy_rows"] > 2048
+    orc = _start(g, dm)
+    before = dm.stats()["kernel_launches"]
+    rounds = dm.expanderDecomposition()
+    assert dm.stats()["kernel_launches"] - before > 15 * rounds      # one kernel takes one launch
+    done, srt = _run_rounds(orc)
+    assert rounds == done
+    _check_state(dm, orc, srt)
+
+
+@pytest.mark.parametrize("name", sorted(GRAPHS))
+@pytest.mark.parametrize("offsets", [np.uint32, np.uint64])
+def test_loop_and_hand_over(name, offsets):
+    """The tuned plan: the loop, then the one-kernel form where few rows are long."""
+    g = GRAPHS[name][0]()
+    g = G.CSRGraph(g.offsets.astype(offsets), g.cols, name)
+    dm = P.CudaDeviceManager()
+    dm.initialize(g)
+    orc = _start(g, dm)
+    before = dm.stats()["kernel_launches"]
+    rounds = dm.expanderDecomposition()
+    assert dm.stats()["kernel_launches"] - before > 15 * 2           # at least one body of two rounds
+    done, srt = _run_rounds(orc)
+    assert rounds == done
+    _check_state(dm, orc, srt)
+
+
+@pytest.mark.parametrize("plan", [None, (8, 64, 1024), (1, 64, 128)])
+@pytest.mark.parametrize("offsets", [np.uint32, np.uint64])
+def test_long_rows_are_handed_over(plan, offsets):
+    g = _with_hubs()
+    g = G.CSRGraph(g.offsets.astype(offsets), g.cols, "hubs")
+    dm = P.CudaDeviceManager()
+    if plan:
+        dm.set_row_plan(*plan)
+    dm.initialize(g)
+    orc = _start(g, dm)
+    handed, srt = 0, None
+    while orc.n_active > 32768:          # the loop hands over after an even round
+        done, srt = _run_rounds(orc, 2)
+        handed += done
+    assert orc.n_active and all(orc.labels()[hub] >= 0 for hub in LASTING)
+    rounds = dm.expanderDecomposition()
+    more, srt = _run_rounds(orc)
+    assert rounds == handed + more
+    _check_state(dm, orc, srt)
+
+
+def test_round_cap_inside_the_handed_over_rounds():
+    """A cap three rounds past the hand-over: the state it leaves, and the rest stage by stage."""
+    g = _with_hubs()
+    first = P.CudaDeviceManager()
+    first.initialize(g)
+    orc = _start(g, first)
+    handed = 0
+    while orc.n_active > 32768:
+        handed += _run_rounds(orc, 2)[0]
+    dm = P.CudaDeviceManager(max_rounds=handed + 3)
+    dm.initialize(g)
+    with pytest.raises(P.PxrError):
+        dm.expanderDecomposition()
+    done, srt = _run_rounds(orc, 4)      # the cap is looked at after every second round
+    assert done == 4 and orc.labels()[LASTING[0]] >= 0
+    _check_state(dm, orc, srt)
+    while dm.getNumClusters():
+        dm.iterateRandomWalk()
+        dm.computeSweepCuts()
+        dm.cutClusters()
+    _, srt = _run_rounds(orc)
+    _check_state(dm, orc, srt)
