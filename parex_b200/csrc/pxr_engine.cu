@@ -9,6 +9,7 @@
 #include <new>
 #include <numeric>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "pxr_sched.cuh"
@@ -423,6 +424,7 @@ struct pxr_handle {
     cudaStream_t stream = nullptr;
     bool initialized = false;
     bool off64 = false;
+    bool fits32 = false;             // the graph's offsets fit 32 bits and may be downloaded so
     uint32_t n = 0;
     uint64_t m = 0, slots = 0;
     uint32_t maxdeg = 0;
@@ -1740,6 +1742,7 @@ pxr_status initialize_impl(pxr_handle* h, uint32_t n, uint64_t m, const OffT* of
         return fail(h, PXR_INVALID_ARG, "the volume 2m of the starting cluster must be below 2^32");
     PXR_CUDA(h, cudaSetDevice(h->device));
     h->initialized = false;
+    h->fits32 = sizeof(OffT) == 4;
     const bool reuse = !h->allocs.empty() && h->n == n && h->m == m && h->off64 == (sizeof(OffT) == 8);
     if (!reuse) {
         pxr_status st = allocate<OffT>(h, n, m);
@@ -1794,6 +1797,41 @@ pxr_status initialize_impl(pxr_handle* h, uint32_t n, uint64_t m, const OffT* of
     return sync_ctr(h);
 }
 
+// Slots up to which the row kernels may index with 32 bits: a row is walked in
+// strides of up to kSlotUnroll * kSmallThreads slots, and an index that passes
+// 2^32 behind the last row starts over below its end.
+constexpr uint64_t kMaxSlots32 = (1ull << 32) - (1u << 16);
+static_assert(2 * kSlotUnroll * kSmallThreads <= 1 << 16 && kSmallThreads >= kBlock, "room for a stride and its unroll");
+
+// A graph whose 2m fits 32 bits, from host or device arrays (kind): 32-bit
+// offsets on the device (half the offset traffic) up to kMaxSlots32, and 64-bit
+// ones for the few sizes above it.
+template <typename OffT>
+pxr_status initialize_fitting(pxr_handle* h, uint32_t n, uint64_t m, const OffT* offsets, const uint32_t* cols,
+                              cudaMemcpyKind kind, bool batched = false) {
+    if (!h) return PXR_INVALID_ARG;
+    const bool wide = 2 * m > kMaxSlots32;
+    pxr_status st;
+    if (!offsets || wide == (sizeof(OffT) == 8)) {
+        st = initialize_impl<OffT>(h, n, m, offsets, cols, kind, batched);
+    } else {
+        std::vector<OffT> given;
+        if (kind == cudaMemcpyDeviceToDevice) {
+            given.resize((size_t)n + 1);
+            PXR_CUDA(h, cudaSetDevice(h->device));
+            PXR_CUDA(h, cudaMemcpyAsync(given.data(), offsets, given.size() * sizeof(OffT), cudaMemcpyDeviceToHost, h->stream));
+            PXR_CUDA(h, cudaStreamSynchronize(h->stream));
+            offsets = given.data();
+            kind = cudaMemcpyDefault;   // the columns stay where they are
+        }
+        using Other = std::conditional_t<sizeof(OffT) == 8, uint32_t, uint64_t>;
+        const std::vector<Other> other(offsets, offsets + n + 1);
+        st = initialize_impl<Other>(h, n, m, other.data(), cols, kind, batched);
+    }
+    if (st == PXR_OK) h->fits32 = true;
+    return st;
+}
+
 // Every instance becomes its own cluster: labels, cluster tables and the
 // round counters replace the one-cluster state that initialize_impl left.
 template <typename OffT>
@@ -1841,6 +1879,10 @@ pxr_status batch_setup(pxr_handle* h, uint32_t n_inst, const uint32_t* starts) {
     PXR_CUDA(h, cudaMemcpyAsync(&h->ctr->n_clusters, &n_inst, 4, cudaMemcpyHostToDevice, s));
     h->initialized = true;
     return sync_ctr(h);
+}
+
+pxr_status batch_setup(pxr_handle* h, uint32_t n_inst, const uint32_t* starts) {
+    return h->off64 ? batch_setup<uint64_t>(h, n_inst, starts) : batch_setup<uint32_t>(h, n_inst, starts);
 }
 
 }  // namespace
@@ -1943,16 +1985,11 @@ pxr_status pxr_set_stream(pxr_handle* h, void* stream) {
 
 pxr_status pxr_initialize(pxr_handle* h, uint32_t n, uint64_t m, const uint32_t* offsets, const uint32_t* cols) {
     if (2 * m >= (1ull << 32)) return fail(h, PXR_INVALID_ARG, "32-bit offsets need 2m < 2^32");
-    return initialize_impl<uint32_t>(h, n, m, offsets, cols, cudaMemcpyHostToDevice);
+    return initialize_fitting(h, n, m, offsets, cols, cudaMemcpyHostToDevice);
 }
 
 pxr_status pxr_initialize64(pxr_handle* h, uint32_t n, uint64_t m, const uint64_t* offsets, const uint32_t* cols) {
-    if (offsets && 2 * m < (1ull << 32)) {
-        // keep 32-bit offsets on the device when they fit: half the offset traffic
-        std::vector<uint32_t> o32((size_t)n + 1);
-        for (size_t i = 0; i <= n; ++i) o32[i] = (uint32_t)offsets[i];
-        return initialize_impl<uint32_t>(h, n, m, o32.data(), cols, cudaMemcpyHostToDevice);
-    }
+    if (offsets && 2 * m < (1ull << 32)) return initialize_fitting(h, n, m, offsets, cols, cudaMemcpyHostToDevice);
     return initialize_impl<uint64_t>(h, n, m, offsets, cols, cudaMemcpyHostToDevice);
 }
 
@@ -1961,7 +1998,7 @@ pxr_status pxr_initialize_device(pxr_handle* h, uint32_t n, uint64_t m, const vo
     if (offsets_are_64bit)
         return initialize_impl<uint64_t>(h, n, m, static_cast<const uint64_t*>(offsets), cols, cudaMemcpyDeviceToDevice);
     if (2 * m >= (1ull << 32)) return fail(h, PXR_INVALID_ARG, "32-bit offsets need 2m < 2^32");
-    return initialize_impl<uint32_t>(h, n, m, static_cast<const uint32_t*>(offsets), cols, cudaMemcpyDeviceToDevice);
+    return initialize_fitting(h, n, m, static_cast<const uint32_t*>(offsets), cols, cudaMemcpyDeviceToDevice);
 }
 
 pxr_status pxr_initialize_batched(pxr_handle* h, uint32_t n, uint64_t m, const uint64_t* offsets, const uint32_t* cols,
@@ -1973,17 +2010,10 @@ pxr_status pxr_initialize_batched(pxr_handle* h, uint32_t n, uint64_t m, const u
     for (uint32_t i = 0; i < n_instances; ++i)
         if (instance_start[i + 1] <= instance_start[i])
             return fail(h, PXR_INVALID_ARG, "every instance needs at least one vertex");
-    pxr_status st;
-    if (offsets && 2 * m < (1ull << 32)) {
-        std::vector<uint32_t> o32((size_t)n + 1);
-        for (size_t i = 0; i <= n; ++i) o32[i] = (uint32_t)offsets[i];
-        st = initialize_impl<uint32_t>(h, n, m, o32.data(), cols, cudaMemcpyHostToDevice, true);
-        if (st != PXR_OK) return st;
-        return batch_setup<uint32_t>(h, n_instances, instance_start);
-    }
-    st = initialize_impl<uint64_t>(h, n, m, offsets, cols, cudaMemcpyHostToDevice, true);
-    if (st != PXR_OK) return st;
-    return batch_setup<uint64_t>(h, n_instances, instance_start);
+    const bool fits = offsets && 2 * m < (1ull << 32);
+    const pxr_status st = fits ? initialize_fitting(h, n, m, offsets, cols, cudaMemcpyHostToDevice, true)
+                               : initialize_impl<uint64_t>(h, n, m, offsets, cols, cudaMemcpyHostToDevice, true);
+    return st == PXR_OK ? batch_setup(h, n_instances, instance_start) : st;
 }
 
 pxr_status pxr_initialize_batched_device(pxr_handle* h, uint32_t n, uint64_t m, const void* offsets,
@@ -1996,17 +2026,13 @@ pxr_status pxr_initialize_batched_device(pxr_handle* h, uint32_t n, uint64_t m, 
     for (uint32_t i = 0; i < n_instances; ++i)
         if (instance_start[i + 1] <= instance_start[i])
             return fail(h, PXR_INVALID_ARG, "every instance needs at least one vertex");
-    pxr_status st;
-    if (offsets_are_64bit) {
-        st = initialize_impl<uint64_t>(h, n, m, static_cast<const uint64_t*>(offsets), cols, cudaMemcpyDeviceToDevice,
-                                       true);
-        if (st != PXR_OK) return st;
-        return batch_setup<uint64_t>(h, n_instances, instance_start);
-    }
-    if (2 * m >= (1ull << 32)) return fail(h, PXR_INVALID_ARG, "32-bit offsets need 2m < 2^32");
-    st = initialize_impl<uint32_t>(h, n, m, static_cast<const uint32_t*>(offsets), cols, cudaMemcpyDeviceToDevice, true);
-    if (st != PXR_OK) return st;
-    return batch_setup<uint32_t>(h, n_instances, instance_start);
+    if (!offsets_are_64bit && 2 * m >= (1ull << 32)) return fail(h, PXR_INVALID_ARG, "32-bit offsets need 2m < 2^32");
+    const pxr_status st =
+        offsets_are_64bit ? initialize_impl<uint64_t>(h, n, m, static_cast<const uint64_t*>(offsets), cols,
+                                                      cudaMemcpyDeviceToDevice, true)
+                          : initialize_fitting(h, n, m, static_cast<const uint32_t*>(offsets), cols,
+                                               cudaMemcpyDeviceToDevice, true);
+    return st == PXR_OK ? batch_setup(h, n_instances, instance_start) : st;
 }
 
 pxr_status pxr_walk_step(pxr_handle* h) { return run_op(h, kOpWalk); }
@@ -2169,10 +2195,17 @@ pxr_status pxr_download_graph64(pxr_handle* h, uint64_t* offsets, uint32_t* cols
 
 pxr_status pxr_download_graph(pxr_handle* h, uint32_t* offsets, uint32_t* cols) {
     if (!h || !offsets) return PXR_INVALID_ARG;
-    if (h->off64) return fail(h, PXR_INVALID_ARG, "graph has 64-bit offsets");
+    if (h->off64 && !h->fits32) return fail(h, PXR_INVALID_ARG, "graph has 64-bit offsets");
     if (!h->initialized) return fail(h, PXR_NOT_INITIALIZED, "no graph uploaded");
-    PXR_CUDA(h, cudaMemcpyAsync(offsets, h->off, ((size_t)h->n + 1) * 4, cudaMemcpyDeviceToHost, h->stream));
-    PXR_CUDA(h, cudaStreamSynchronize(h->stream));
+    if (h->off64) {
+        std::vector<uint64_t> o((size_t)h->n + 1);
+        PXR_CUDA(h, cudaMemcpyAsync(o.data(), h->off, o.size() * 8, cudaMemcpyDeviceToHost, h->stream));
+        PXR_CUDA(h, cudaStreamSynchronize(h->stream));
+        std::copy(o.begin(), o.end(), offsets);
+    } else {
+        PXR_CUDA(h, cudaMemcpyAsync(offsets, h->off, ((size_t)h->n + 1) * 4, cudaMemcpyDeviceToHost, h->stream));
+        PXR_CUDA(h, cudaStreamSynchronize(h->stream));
+    }
     return download_cols(h, cols);
 }
 

@@ -324,3 +324,57 @@ def test_round_cap_inside_the_handed_over_rounds():
         dm.cutClusters()
     _, srt = _run_rounds(orc)
     _check_state(dm, orc, srt)
+
+
+def test_slots_up_to_the_end_of_32_bits():
+    """2^32 - 2 slots under 32-bit offsets: rows end within a walk's stride of 2^32.
+    Cliques of 4,096 vertices in pairs joined by a perfect matching, less one edge."""
+    import torch
+    torch.cuda.empty_cache()
+    if torch.cuda.mem_get_info()[0] < 60e9:
+        pytest.skip("needs 60 GB of device memory")
+    n, deg, chunk = 1 << 20, 4096, 1 << 15
+    cols = torch.empty(n * deg - 2, dtype=torch.int32, device="cuda")
+    at = 0
+    for v0 in range(0, n, chunk):
+        v = torch.arange(v0, v0 + chunk, dtype=torch.int32, device="cuda")
+        rows = torch.sort(v[:, None] ^ torch.arange(1, deg + 1, dtype=torch.int32, device="cuda")[None, :], dim=1)[0]
+        rows = rows.reshape(-1)
+        if v0 == 0:       # without the edge 0 - 4,096: the last slot of the one row, the first of the other
+            rows = torch.cat([rows[: deg - 1], rows[deg: deg * deg], rows[deg * deg + 1:]])
+        cols[at: at + rows.shape[0]] = rows
+        at += rows.shape[0]
+    assert at == cols.shape[0]
+    ix = np.arange(n + 1, dtype=np.int64)
+    off = (ix * deg - (ix > 0) - (ix > deg)).astype(np.uint32)
+    off_d = torch.from_numpy(off.view(np.int32)).cuda()
+    dm = P.CudaDeviceManager(tune=P.TUNE_HEURISTIC)
+    dm.initialize_device(n, (n * deg - 2) // 2, off_d.data_ptr(), False, cols.data_ptr())
+
+    x = dm.readRandomWalkValues().astype(np.float64)
+    dm.iterateRandomWalk()
+    degree = np.diff(off.astype(np.int64))
+    share = x / degree
+    total = share.reshape(-1, deg).sum(axis=1).repeat(deg) - share + share[np.arange(n) ^ deg]
+    total[0] -= share[deg]
+    total[deg] -= share[0]
+    # rounding of 4,096 terms x / degree to 24 bits, of their sum and of the result: 2^-24 max|x| each at most
+    np.testing.assert_allclose(dm.readRandomWalkValues(), 0.9 * total + 0.1 * x, rtol=0,
+                               atol=2.0**-22 * np.abs(x).max())
+    dm.computeSweepCuts()
+    dm.cutClusters()
+    dm.expanderDecomposition()
+    ids = torch.from_numpy(dm.getFinalPartition().clusterIds).cuda()
+    pair = torch.arange(n, device="cuda") // (2 * deg)
+    one = torch.full((int(ids.max()) + 1,), -1, dtype=torch.int64, device="cuda")
+    one[ids.long()] = pair
+    assert bool((one[ids.long()] == pair).all())          # no cluster in two components
+    cut = 0
+    for v0 in range(0, n, chunk):
+        b, e = int(off[v0]), int(off[v0 + chunk])
+        d = torch.from_numpy(degree[v0: v0 + chunk]).cuda()
+        cut += int((ids[v0: v0 + chunk].repeat_interleave(d) != ids[cols[b:e].long()]).sum())
+    assert dm.countCutEdges() == cut // 2
+    dm.close()
+    del cols
+    torch.cuda.empty_cache()
