@@ -149,8 +149,11 @@ __device__ __forceinline__ uint32_t ld_relaxed(const uint32_t* p) {
 }
 
 // A word that other blocks change while this one reads it, where an older value
-// (no older than the kernel's start) serves as well: the load may be answered
-// by the SM's own L1.
+// serves as well: the load may be answered by the SM's own L1.  How old that may
+// be is the caller's ordering: no older than what the kernel's start makes
+// visible, or, where a kernel rewrites the word in one pass and reads it in the
+// next, than the barrier between the two, which must then be an acquire over
+// every block that writes (small_sync in pxr_small.cuh).
 __device__ __forceinline__ uint32_t ld_near(const uint32_t* p) {
     uint32_t v;
     asm volatile("ld.relaxed.cta.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");

@@ -83,7 +83,10 @@ struct SmallArgs {
     uint32_t max_rounds;
 };
 
-// Barrier over the cluster; writes before it are visible to every thread after it.
+// Barrier over the cluster; writes before it are visible to every thread after it,
+// CTA-scope reads through L1 (ld_near) included: parent is rewritten every round
+// inside one launch, and it is this acquire before each union-find pass, not the
+// kernel's start, that bounds how old a parent read there can be.
 __device__ __forceinline__ void small_sync() {
     if (gridDim.x == 1) {
         __syncthreads();
