@@ -20,10 +20,7 @@ using namespace pxr;
 
 namespace pxr {
 constexpr uint32_t kMaxGrid = 148u * 32u;
-#ifndef PXR_UNION_LANES
-#define PXR_UNION_LANES 1
-#endif
-constexpr int kUnionLanes = PXR_UNION_LANES;   // lanes per light row in k_union
+constexpr int kUnionLanes = 1;                 // lanes per light row in k_union
 constexpr uint32_t kSampledDegree = 16;        // mean degree from which k_union uses sampled linking
 
 constexpr size_t kSliceAlign = 256;   // as cudaMalloc aligns

@@ -9,23 +9,16 @@
 namespace pxr {
 
 constexpr int kBlock = 256;
-// Walk kernels: CTAs per SM their register budget is sized for, and whether
-// the long-row kernels load the next row's head while gathering this row.
-// The walk is latency-bound (its gathers wait on L2); eight 256-thread CTAs
-// per SM (32 registers, a few bytes spilled) beat five (44 registers): on
-// R-MAT 24 one walk step took 2.11 instead of 2.32 ms, and the prefetch made
-// it slower at either bound (measured on a B200).
-#ifndef PXR_WALK_PREFETCH
-#define PXR_WALK_PREFETCH 0
-#endif
-#ifndef PXR_WALK_MIN_BLOCKS
-#define PXR_WALK_MIN_BLOCKS 8
-#endif
-#if PXR_WALK_MIN_BLOCKS > 0
-#define PXR_WALK_BOUNDS __launch_bounds__(kBlock, PXR_WALK_MIN_BLOCKS)
-#else
-#define PXR_WALK_BOUNDS __launch_bounds__(kBlock)
-#endif
+// Walk kernel: CTAs per SM its register budget is sized for.  The walk is
+// latency-bound (its gathers wait on L2): eight 256-thread CTAs per SM (32
+// registers) beat five (44 registers) when the three bins of rows were kernels of
+// their own, 2.11 against 2.32 ms a step on R-MAT 24, although they spill.  As one
+// kernel (k_walk, RowParts) it spills more, 108 bytes stored and 68 loaded with
+// 32-bit offsets, W = 1 (200 and 140 with 64-bit offsets, W = 8) against 44 / 32
+// before; with the long rows' lists ordered by length it is faster all the same:
+// R-MAT 22 580 -> 492 us a step, R-MAT 20 137 -> 131, with 64-bit offsets 605 ->
+// 523 and 180 -> 141.
+constexpr int kWalkCtas = 8;
 constexpr int kScanItems = 8;                        // items per thread in look-back kernels
 constexpr int kScanTile = kBlock * kScanItems;
 // Tiles of the kernels over the active vertices: kScanItems items per thread,
@@ -38,10 +31,7 @@ constexpr int kScanTile = kBlock * kScanItems;
 // 7.40 / 6.30 / 6.28 / 6.28, of 32 32.7 / 31.9 / 31.7 / 32.8.
 constexpr int kFineItems = 2;
 constexpr int kFineTile = kBlock * kFineItems;
-#ifndef PXR_FINE_MAX
-#define PXR_FINE_MAX (1u << 19)
-#endif
-constexpr uint32_t kFineMax = PXR_FINE_MAX;
+constexpr uint32_t kFineMax = 1u << 19;
 // blocks a launch over up to n active vertices needs for either tile
 inline uint32_t scan_blocks(uint32_t n) {
     const uint32_t coarse = (n + kScanTile - 1) / kScanTile;
@@ -480,7 +470,7 @@ __device__ __forceinline__ const uint32_t* row_list(const Dev<OffT>& d, int G, u
     return G == 32 ? d.wide : d.heavy;
 }
 
-// A long row's head: vertex, label and slot bounds (label -1 past the list).
+// A long row's head: vertex, label and slot bounds.
 template <typename OffT>
 struct RowHead {
     uint32_t v;
@@ -489,15 +479,9 @@ struct RowHead {
 };
 
 template <typename OffT>
-__device__ __forceinline__ RowHead<OffT> row_head(const Dev<OffT>& d, const uint32_t* list, uint32_t h, uint32_t cnt) {
-    RowHead<OffT> r{0u, -1, 0, 0};
-    if (h < cnt) {
-        r.v = list[h];
-        r.lab = d.lab[r.v];
-        r.beg = d.off[r.v];
-        r.end = d.off[r.v + 1];
-    }
-    return r;
+__device__ __forceinline__ RowHead<OffT> row_head(const Dev<OffT>& d, const uint32_t* list, uint32_t h) {
+    const uint32_t v = list[h];
+    return RowHead<OffT>{v, d.lab[v], d.off[v], d.off[v + 1]};
 }
 
 // ---------------------------------------------------------------------------
@@ -621,18 +605,9 @@ __device__ __forceinline__ void walk_long_rows(const Dev<OffT>& d, const float* 
     uint32_t cnt;
     const uint32_t* list = row_list(d, G, &cnt);
     const RowGroups<G> rg(block, blocks);
-    // With PXR_WALK_PREFETCH the next row's id, label and bounds are loaded
-    // before this row's slots are gathered, so a row's setup loads overlap
-    // the previous row's gathers.
-    RowHead<OffT> nx = row_head(d, list, rg.first, cnt);
+    // (loading the next row's head before this row's gathers made the step slower)
     for (uint32_t h = rg.first; h < cnt; h += rg.step) {
-        RowHead<OffT> cur;
-        if (PXR_WALK_PREFETCH) {
-            cur = nx;
-            nx = row_head(d, list, h + rg.step, cnt);
-        } else {
-            cur = row_head(d, list, h, cnt);
-        }
+        const RowHead<OffT> cur = row_head(d, list, h);
         if (cur.lab < 0) continue;
         const uint32_t v = cur.v;
         const OffT beg = cur.beg, end = cur.end;
@@ -661,7 +636,7 @@ __device__ __forceinline__ void walk_long_rows(const Dev<OffT>& d, const float* 
 }
 
 template <typename OffT, int W, bool LONG>
-__global__ void PXR_WALK_BOUNDS k_walk(Dev<OffT> d, RowParts parts, const uint32_t* ids, const float* xt_in,
+__global__ void __launch_bounds__(kBlock, kWalkCtas) k_walk(Dev<OffT> d, RowParts parts, const uint32_t* ids, const float* xt_in,
                                        float* xt_out) {
     pdl_wait();
     __shared__ int64_t sh[kBlock / 32];
